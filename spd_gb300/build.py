@@ -21,14 +21,16 @@ import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
-VARIANTS = {"ieee": ("libspd_gb300.so", "--fmad=false"), "fma": ("libspd_gb300_fma.so", "--fmad=true")}
+VARIANTS = {"ieee": ("libspd_gb300.so", "--fmad=false"), "fma": ("libspd_gb300_fma.so", "--fmad=true", "-DSPD_FUSED")}
 OUT = os.path.join(HERE, VARIANTS["ieee"][0])
 BUILD_DIR = os.path.join(HERE, "_build")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-rdc=false", "-Wno-deprecated-gpu-targets"]
-SOURCES = ["spd_core.cu", "spd_step_d1.cu", "spd_step_d2.cu", "spd_step_d3.cu", "spd_noalloc.cu", "spd_ensemble.cu",
-           "spd_adjoint.cu", "spd_adj_d1.cu", "spd_adj_d2.cu", "spd_adj_d3.cu"]
-
+# translation units: (source, defines); the step is one unit per dimension and
+# degree, the longest ones first
+SOURCES = [("spd_step.cu", f"-DSPD_D={d}", f"-DSPD_P={p}") for d in (3, 2, 1) for p in (4, 3, 2, 1)]
+SOURCES += [(name,) for name in ("spd_adj_d3.cu", "spd_adj_d2.cu", "spd_adj_d1.cu", "spd_core.cu", "spd_noalloc.cu",
+                                 "spd_ensemble.cu", "spd_adjoint.cu")]
 
 
 def nvcc() -> str:
@@ -39,10 +41,11 @@ def nvcc() -> str:
 
 
 def _compile(job) -> str:
-    variant, src = job
+    variant, (src, *defines) = job
     out_dir = os.path.join(BUILD_DIR, variant)
-    obj = os.path.join(out_dir, os.path.splitext(src)[0] + ".o")
-    cmd = [nvcc(), *ARCH, *FLAGS, VARIANTS[variant][1], "-c", os.path.join(CSRC, src), "-o", obj]
+    tag = "".join("_" + d.split("_")[-1].replace("=", "").lower() for d in defines)
+    obj = os.path.join(out_dir, os.path.splitext(src)[0] + tag + ".o")
+    cmd = [nvcc(), *ARCH, *FLAGS, *VARIANTS[variant][1:], *defines, "-c", os.path.join(CSRC, src), "-o", obj]
     subprocess.run(cmd, check=True)
     return obj
 
@@ -70,7 +73,7 @@ def build(force: bool = False, variants=("ieee", "fma")) -> str:
     if todo:
         for v in todo:
             os.makedirs(os.path.join(BUILD_DIR, v), exist_ok=True)
-        jobs = [(v, src) for v in todo for src in SOURCES]
+        jobs = [(v, src) for src in SOURCES for v in todo]
         workers = max(1, min(len(jobs), os.cpu_count() or 1))
         with concurrent.futures.ThreadPoolExecutor(max_workers=workers) as ex:
             objs = list(ex.map(_compile, jobs))

@@ -476,12 +476,12 @@ __global__ void k_adj_faces(Geo g, FvGeo fg, int d, const double* __restrict__ d
     if (f[d] >= 1) {  // right face of subcell f-1
       q[d] = f[d] - 1;
       const long long qi = q[0] + (long long)g.X[0] * (q[1] + (long long)g.X[1] * q[2]);
-      Fa += div_rcp(-dti * Unew_a[(long long)v * g.Nq + qi], fg.dx[d][q[d]], fg.rdx[d][q[d]]);
+      Fa += div_by(-dti * Unew_a[(long long)v * g.Nq + qi], fg.dx[d][q[d]], fg.rdx[d][q[d]]);
     }
     if (f[d] < Xd) {  // left face of subcell f
       q[d] = f[d];
       const long long qi = q[0] + (long long)g.X[0] * (q[1] + (long long)g.X[1] * q[2]);
-      Fa += div_rcp(dti * Unew_a[(long long)v * g.Nq + qi], fg.dx[d][q[d]], fg.rdx[d][q[d]]);
+      Fa += div_by(dti * Unew_a[(long long)v * g.Nq + qi], fg.dx[d][q[d]], fg.rdx[d][q[d]]);
     }
     double ho = Fa, fbv = 0.0;
     if (use_fb) {
@@ -545,11 +545,11 @@ __device__ __forceinline__ void muscl_cell_forward(const Geo& g, const FvGeo& fg
     const long long st = ext_stride(g, dd);
     const int cdd = ec[dd];
     const double hl = fg.hcv[dd][cdd - 1], hr = fg.hcv[dd][cdd], hm = fg.hfp[dd][cdd];
-    const double rhl = fg.rhcv[dd][cdd - 1], rhr = fg.rhcv[dd][cdd];
+    const Rcp rhl = fg.rhcv[dd][cdd - 1], rhr = fg.rhcv[dd][cdd];
     for (int v = 0; v < V; ++v) {
       const double* M = W_ext + (long long)v * g.Nqe;
-      const double SL = div_rcp(M[e] - M[e - st], hl, rhl);
-      const double SR = div_rcp(M[e + st] - M[e], hr, rhr);
+      const double SL = div_by(M[e] - M[e - st], hl, rhl);
+      const double SR = div_by(M[e + st] - M[e], hr, rhr);
       SLs[dd][v] = SL;
       SRs[dd][v] = SR;
       dMh[dd][v] = (limiter == LIM_MINMOD) ? minmod(SL, SR) : moncen(SL, SR, hl, hr, hm);
@@ -759,7 +759,7 @@ __device__ __forceinline__ void adj_muscl_cell(const Geo& g, const FvGeo& fg, in
     for (int v = 0; v < V; ++v) {
       double SLa, SRa;
       limiter_vjp(limiter, SLs[dd][v], SRs[dd][v], hl, hr, hm, in_a[V + dd * V + v], SLa, SRa);
-      const double l = SLa * fg.rhcv[dd][cdd - 1], rr = SRa * fg.rhcv[dd][cdd];
+      const double l = SLa * fg.ihcv[dd][cdd - 1], rr = SRa * fg.ihcv[dd][cdd];
       // SL = (W(e) - W(e-st)) / hl ; SR = (W(e+st) - W(e)) / hr
       own[v] = own[v] + l - rr;
       LA[((long long)(dd * 2 + 0) * V + v) * g.Nqe + e] = l;

@@ -51,11 +51,21 @@ __global__ void k_clip_dt(const double* t, double* dt) {
   if (t[0] + d >= t[1]) *dt = t[1] - t[0];
 }
 
+template <int D>
+StepperBase* make_stepper_for(int P) {
+  switch (P) {
+    case 1: return make_stepper_of<D, 1>();
+    case 2: return make_stepper_of<D, 2>();
+    case 3: return make_stepper_of<D, 3>();
+    case 4: return make_stepper_of<D, 4>();
+    default: return nullptr;
+  }
+}
 StepperBase* make_stepper(int D, int P) {
   switch (D) {
-    case 1: return make_stepper_d1(P);
-    case 2: return make_stepper_d2(P);
-    case 3: return make_stepper_d3(P);
+    case 1: return make_stepper_for<1>(P);
+    case 2: return make_stepper_for<2>(P);
+    case 3: return make_stepper_for<3>(P);
     default: return nullptr;
   }
 }
@@ -175,8 +185,9 @@ int spd_create(const spd_config* cfg, const spd_operators* ops, spd_ctx** out) {
       {
         int ex = 0;
         const double mant = std::frexp(g.h[d], &ex);
-        g.h_pow2[d] = (mant == 0.5) ? 1 : 0;
+        g.h_pow2[d] = (mant == 0.5 && std::abs(ex) <= 64) ? 1 : 0;
         g.inv_h[d] = 1.0 / g.h[d];
+        g.rh[d] = recip_of(g.h[d]);
       }
       h_min = std::min(h_min, g.h[d]);
       g.bc[d][0] = cfg->BC[d][0];
@@ -187,6 +198,7 @@ int spd_create(const spd_config* cfg, const spd_operators* ops, spd_ctx** out) {
       g.Xe[d] = 1;
       g.h[d] = 1.0;
       g.inv_h[d] = 1.0;
+      g.rh[d] = recip_of(1.0);
       g.h_pow2[d] = 1;
       g.bc[d][0] = g.bc[d][1] = SPD_BC_PERIODIC;
     }
@@ -195,6 +207,7 @@ int spd_create(const spd_config* cfg, const spd_operators* ops, spd_ctx** out) {
     g.Nqe *= g.Xe[d];
   }
   g.gamma = cfg->gamma;
+  g.rgm1 = recip_of(cfg->gamma - 1.0);
   g.min_c2 = cfg->min_c2;
   g.iso = cfg->isothermal ? 1 : 0;
   C->h_dt = h_min / (double)(P + 1);
@@ -208,8 +221,25 @@ int spd_create(const spd_config* cfg, const spd_operators* ops, spd_ctx** out) {
   std::memcpy(C->ops.sp_to_cv, ops->sp_to_cv, sizeof(double) * n * n);
   std::memcpy(C->ops.invader, ops->invader, sizeof(double) * T * T);
   std::memcpy(C->ops.w_tp, ops->w_tp, sizeof(double) * T);
-  for (int d = 0; d < 3; ++d)
-    for (int i = 0; i < n * nf; ++i) C->ops.dfp_h[d][i] = C->ops.dfp_to_sp[i] * g.inv_h[d];
+  // the operators as operands of the integer-pipe products
+  {
+    bool in = true;
+    auto prepare = [&in](const double* a, int count, Coef* c) {
+      for (int i = 0; i < count; ++i) {
+        in = in && coef_in_range(a[i]);
+        c[i] = coef_of(a[i]);
+      }
+    };
+    prepare(C->ops.sp_to_fp, nf * n, C->ops.c_sp_to_fp);
+    prepare(C->ops.dfp_to_sp, n * nf, C->ops.c_dfp);
+    prepare(C->ops.sp_to_cv, n * n, C->ops.c_sp_to_cv);
+    prepare(C->ops.invader, T * T, C->ops.c_invader);
+    prepare(C->ops.w_tp, T, C->ops.c_w_tp);
+    C->ops.soft = in ? 1 : 0;
+    // an operator out of their range is also not scaled by 1/h
+    for (int d = 0; d < 3; ++d) g.h_pow2[d] = in ? g.h_pow2[d] : 0;
+    for (int d = 0; d < 3; ++d) C->ops.dfp_eoff[d] = g.h_pow2[d] ? (unsigned)-std::ilogb(g.h[d]) << 20 : 0u;
+  }
 
   CK(cudaStreamCreateWithFlags(&C->own_stream, cudaStreamNonBlocking));
   C->stream = C->own_stream;
@@ -237,11 +267,25 @@ int spd_create(const spd_config* cfg, const spd_operators* ops, spd_ctx** out) {
     if (int r = dalloc(C, &C->K_cv_to_sp, K2.size())) return r;
     CK(cudaMemcpy(C->K_sp_to_cv, K1.data(), K1.size() * sizeof(double), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(C->K_cv_to_sp, K2.data(), K2.size() * sizeof(double), cudaMemcpyHostToDevice));
+    C->K_soft = 1;
+    Coef** kt[2] = {&C->Kt_sp_to_cv, &C->Kt_cv_to_sp};
+    for (int w = 0; w < 2; ++w) {
+      std::vector<Coef> T2((size_t)NS * NS);
+      for (int o = 0; o < NS; ++o)
+        for (int in = 0; in < NS; ++in) {
+          const double a = (*(w ? &K2 : &K1))[(size_t)o * NS + in];
+          if (!coef_in_range(a)) C->K_soft = 0;
+          T2[(size_t)in * NS + o] = coef_of(a);
+        }
+      if (int r = dalloc(C, kt[w], T2.size())) return r;
+      CK(cudaMemcpy(*kt[w], T2.data(), T2.size() * sizeof(Coef), cudaMemcpyHostToDevice));
+    }
   }
   // subcell geometry (src/sdader_simulator.py:61-92, src/fv_simulator.py:195)
   {
     std::vector<double> buf;
-    size_t off[3][8];
+    std::vector<Rcp> rcp;
+    size_t off[3][6], roff[3][3];
     for (int d = 0; d < D; ++d) {
       const int Xd = g.X[d], Xe = g.Xe[d];
       const double* fp = ops->faces[d];
@@ -256,25 +300,30 @@ int spd_create(const spd_config* cfg, const spd_operators* ops, spd_ctx** out) {
       off[d][3] = buf.size();
       for (int e = 0; e + 1 < Xe; ++e) buf.push_back(cen[e + 1] - cen[e]);
       off[d][4] = buf.size();
-      for (int k2 = 0; k2 < Xd; ++k2) buf.push_back(1.0 / buf[off[d][0] + k2]);
+      for (int e = 0; e < Xe; ++e) buf.push_back((e >= 1 && e + 1 < Xe) ? cen[e + 1] - cen[e - 1] : 1.0);
       off[d][5] = buf.size();
       for (int e = 0; e + 1 < Xe; ++e) buf.push_back(1.0 / buf[off[d][3] + e]);
-      off[d][6] = buf.size();
-      for (int e = 0; e < Xe; ++e) buf.push_back((e >= 1 && e + 1 < Xe) ? cen[e + 1] - cen[e - 1] : 1.0);
-      off[d][7] = buf.size();
-      for (int e = 0; e < Xe; ++e) buf.push_back(1.0 / buf[off[d][6] + e]);
+      roff[d][0] = rcp.size();
+      for (int k2 = 0; k2 < Xd; ++k2) rcp.push_back(recip_of(buf[off[d][0] + k2]));
+      roff[d][1] = rcp.size();
+      for (int e = 0; e + 1 < Xe; ++e) rcp.push_back(recip_of(buf[off[d][3] + e]));
+      roff[d][2] = rcp.size();
+      for (int e = 0; e < Xe; ++e) rcp.push_back(recip_of(buf[off[d][4] + e]));
     }
     if (int r = dalloc(C, &C->geo_arrays, buf.size())) return r;
     CK(cudaMemcpy(C->geo_arrays, buf.data(), buf.size() * sizeof(double), cudaMemcpyHostToDevice));
+    if (int r = dalloc(C, &C->geo_rcp, rcp.size())) return r;
+    CK(cudaMemcpy(C->geo_rcp, rcp.data(), rcp.size() * sizeof(Rcp), cudaMemcpyHostToDevice));
     for (int d = 0; d < D; ++d) {
       C->fvg.dx[d] = C->geo_arrays + off[d][0];
       C->fvg.centers[d] = C->geo_arrays + off[d][1];
       C->fvg.hfp[d] = C->geo_arrays + off[d][2];
       C->fvg.hcv[d] = C->geo_arrays + off[d][3];
-      C->fvg.rdx[d] = C->geo_arrays + off[d][4];
-      C->fvg.rhcv[d] = C->geo_arrays + off[d][5];
-      C->fvg.c2[d] = C->geo_arrays + off[d][6];
-      C->fvg.rc2[d] = C->geo_arrays + off[d][7];
+      C->fvg.c2[d] = C->geo_arrays + off[d][4];
+      C->fvg.ihcv[d] = C->geo_arrays + off[d][5];
+      C->fvg.rdx[d] = C->geo_rcp + roff[d][0];
+      C->fvg.rhcv[d] = C->geo_rcp + roff[d][1];
+      C->fvg.rc2[d] = C->geo_rcp + roff[d][2];
     }
   }
   // state and scratch

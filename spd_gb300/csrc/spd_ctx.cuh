@@ -123,8 +123,13 @@ struct spd_ctx {
   double* aff[3] = {nullptr, nullptr, nullptr};
   double* F_FB[3] = {nullptr, nullptr, nullptr};
   double *Mpred = nullptr, *S = nullptr;
-  double *K_sp_to_cv = nullptr, *K_cv_to_sp = nullptr;
+  double *K_sp_to_cv = nullptr, *K_cv_to_sp = nullptr;  // [o][i] (adjoint)
+  // the same, [i][o], as operands of the integer-pipe products; K_soft: all in
+  // their range
+  spd::Coef *Kt_sp_to_cv = nullptr, *Kt_cv_to_sp = nullptr;
+  int K_soft = 0;
   double* geo_arrays = nullptr;
+  spd::Rcp* geo_rcp = nullptr;
   double* staging = nullptr;
   size_t staging_len = 0;
   spd_host::StepperBase* stepper = nullptr;
@@ -247,15 +252,16 @@ struct StepperBase {
   virtual int vjp(spd_ctx* C) = 0;       // Usp_a <- (d U_sp_new / d U_sp)^T Usp_a of the recorded step
   virtual int eq_prims(spd_ctx* C) = 0;  // Weq_cv = prim(Ueq_cv) (well-balanced mode)
   int cpb = 32;       // cells per block of k_interior (a power of two <= max_cpb)
+  bool auto_cpb = true;  // no spd_set_cells_per_block call yet
   int max_cpb = 32;   // largest cpb whose shared-memory tile fits
-  size_t smem = 0;
 };
 
 constexpr int BS = 256;
-constexpr int PERSIST_BLOCKS = 152 * 8;
+constexpr int SMS = 152;
+constexpr int PERSIST_BLOCKS = SMS * 8;
 
-StepperBase* make_stepper_d1(int P);
-StepperBase* make_stepper_d2(int P);
-StepperBase* make_stepper_d3(int P);
+// D = 1..3, P = 1..4 (spd_step.cu)
+template <int D, int P>
+StepperBase* make_stepper_of();
 
 }  // namespace spd_host

@@ -9,10 +9,7 @@
 #include <cmath>
 #include <cstring>
 
-// device code; also host-callable so the scalar maps can be checked on a CPU
-#ifndef SPD_FN
-#define SPD_FN __host__ __device__ __forceinline__
-#endif
+#include "spd_soft.cuh"
 
 namespace spd {
 
@@ -125,47 +122,6 @@ template <int N> SPD_FN bool operator>(const Dual<N>& a, double b) { return a.v 
 // (subnormal or huge b, a or q near underflow or overflow) is divided by
 // IEEE division.  Three FP64 operations instead of a full division where
 // one divisor serves several quotients.
-#ifdef __CUDA_ARCH__
-__device__ __noinline__ double div_ieee_slow(double a, double b) { return a / b; }
-#else
-inline double div_ieee_slow(double a, double b) { return a / b; }
-#endif
-// Predicates on a double's bit pattern evaluated on its two 32-bit words
-// (integer pipes).  The same tests written on the 64-bit pattern (for
-// instance (bits & ~sign) > bits(inf) for NaN) were compiled to FP64-pipe
-// instructions, measured with ncu (one per test), on the pipe that bounds
-// the step's kernels.
-SPD_FN unsigned hi_word(double x) {
-#ifdef __CUDA_ARCH__
-  return (unsigned)__double2hiint(x);
-#else
-  unsigned long long b;
-  memcpy(&b, &x, sizeof(b));
-  return (unsigned)(b >> 32);
-#endif
-}
-SPD_FN unsigned lo_word(double x) {
-#ifdef __CUDA_ARCH__
-  return (unsigned)__double2loint(x);
-#else
-  unsigned long long b;
-  memcpy(&b, &x, sizeof(b));
-  return (unsigned)b;
-#endif
-}
-// x is a NaN
-SPD_FN bool nan_w(double x) {
-  const unsigned h = hi_word(x) & 0x7fffffffu;
-  return h > 0x7ff00000u || (h == 0x7ff00000u && lo_word(x) != 0u);
-}
-// x != 0 (true for NaN, false for both zeros)
-SPD_FN bool nonzero_w(double x) { return ((hi_word(x) & 0x7fffffffu) | lo_word(x)) != 0u; }
-// x > 0 (false for zeros, negatives and NaN)
-SPD_FN bool gt0_w(double x) {
-  const unsigned h = hi_word(x), l = lo_word(x);
-  return (h >> 31) == 0u && (h | l) != 0u && (h < 0x7ff00000u || (h == 0x7ff00000u && l == 0u));
-}
-
 SPD_FN double div_rcp(double a, double b, double rb) {
   const double q = a * rb;
   const double r = fma(-q, b, a);
@@ -188,7 +144,11 @@ SPD_FN double div_rcp(double a, double b, double rb) {
 
 SPD_FN double sval(double x) { return x; }
 template <int N> SPD_FN double sval(const Dual<N>& x) { return x.v; }
+#ifdef SPD_FUSED
 SPD_FN double ad_sqrt(double x) { return sqrt(x); }
+#else
+SPD_FN double ad_sqrt(double x) { return sqrt_soft(x); }
+#endif
 template <int N>
 SPD_FN Dual<N> ad_sqrt(const Dual<N>& x) {
   Dual<N> r; r.v = sqrt(x.v);
@@ -213,14 +173,32 @@ SPD_FN Dual<N> ad_abs(const Dual<N>& x) {
   return Dual<N>(fabs(x.v));
 }
 
-// a / b with b's reciprocal rb precomputed (double: Markstein; dual numbers:
-// plain division, rb unused)
+// a / b with b's reciprocal prepared by recip_of (double: div_soft, or in the
+// build with fused multiply-adds Markstein's correction; dual numbers: plain
+// division, the reciprocal unused)
+template <class S>
+struct RecipOf {
+  using T = S;
+};
+#ifdef SPD_FUSED
 SPD_FN double div_by(double a, double b, double rb) { return div_rcp(a, b, rb); }
+SPD_FN double recip_of(double b) { return 1.0 / b; }
+#else
+template <>
+struct RecipOf<double> {
+  using T = Recip;
+};
+SPD_FN double div_by(double a, double b, const Recip& rb) { return div_soft(a, b, rb); }
+SPD_FN Recip recip_of(double b) { return recip_soft(b); }
+#endif
+// a prepared reciprocal of a double
+using Rcp = typename RecipOf<double>::T;
+// a / b
+SPD_FN double quot(double a, double b) { return div_by(a, b, recip_of(b)); }
 template <int N>
 SPD_FN Dual<N> div_by(const Dual<N>& a, const Dual<N>& b, const Dual<N>&) { return a / b; }
-template <int N>
-SPD_FN Dual<N> div_by(const Dual<N>& a, double b, double) { return a / b; }
-SPD_FN double recip_of(double b) { return 1.0 / b; }
+template <int N, class R>
+SPD_FN Dual<N> div_by(const Dual<N>& a, double b, const R&) { return a / b; }
 template <int N>
 SPD_FN Dual<N> recip_of(const Dual<N>&) { return Dual<N>(0.0); }
 
@@ -342,16 +320,17 @@ SPD_FN int rvel(int idim, int k) { return 1 + (idim + k) % D; }
 // ``iso``: the isothermal system (src/hydro.py:84,123,169): the kinetic term
 // of the energy is multiplied by 0 and the energy flux by 0.
 template <int D, class S>
-SPD_FN void prim(const S* U, S* W, double gamma, int idim_order, S* r0_out = nullptr, bool iso = false) {
+SPD_FN void prim(const S* U, S* W, double gamma, int idim_order, typename RecipOf<S>::T* r0_out = nullptr,
+                 bool iso = false) {
   constexpr int P_ = D + 1;
   W[0] = U[0];
   S K = 0.0;
-  const S r0 = recip_of(U[0]);
+  const auto r0 = recip_of(U[0]);
   if (r0_out) *r0_out = r0;
 #pragma unroll
   for (int k = 0; k < D; ++k) {
     const int v = rvel<D>(idim_order, k);
-    W[v] = (D == 1 && !r0_out) ? U[v] / U[0] : div_by(U[v], U[0], r0);
+    W[v] = div_by(U[v], U[0], r0);
     const S w2 = W[v] * W[v];
     K = (k == 0) ? w2 : K + w2;
   }
@@ -362,7 +341,7 @@ SPD_FN void prim(const S* U, S* W, double gamma, int idim_order, S* r0_out = nul
 
 // W -> U (src/hydro.py:88-125).
 template <int D, class S>
-SPD_FN void cons(const S* W, S* U, double gamma, int idim_order, bool iso = false) {
+SPD_FN void cons(const S* W, S* U, double gamma, int idim_order, bool iso = false, const Rcp* rg = nullptr) {
   constexpr int P_ = D + 1;
   U[0] = W[0];
   S K = 0.0;
@@ -375,12 +354,12 @@ SPD_FN void cons(const S* W, S* U, double gamma, int idim_order, bool iso = fals
   }
   K = K * (0.5 * W[0]);
   if (iso) K = K * 0.0;
-  U[P_] = div_by(W[P_], gamma - 1.0, 1.0 / (gamma - 1.0)) + K;
+  U[P_] = div_by(W[P_], gamma - 1.0, rg ? *rg : recip_of(gamma - 1.0)) + K;
 }
 
 // Euler flux in the rotated frame of direction idim (src/hydro.py:127-170).
 template <int D, class S>
-SPD_FN void flux(const S* W, S* F, double gamma, int idim, bool iso = false) {
+SPD_FN void flux(const S* W, S* F, double gamma, int idim, bool iso = false, const Rcp* rg = nullptr) {
   constexpr int P_ = D + 1;
   const int v1 = rvel<D>(idim, 0);
   S K = 0.0, m = 0.0;
@@ -392,7 +371,7 @@ SPD_FN void flux(const S* W, S* F, double gamma, int idim, bool iso = false) {
     K = (k == D - 1) ? mv : K + mv;
     F[v] = m * W[v1];
   }
-  const S E = div_by(W[P_], gamma - 1.0, 1.0 / (gamma - 1.0)) + 0.5 * K;
+  const S E = div_by(W[P_], gamma - 1.0, rg ? *rg : recip_of(gamma - 1.0)) + 0.5 * K;
   F[0] = m;
   F[v1] = m * W[v1] + W[P_];
   F[P_] = W[v1] * (E + W[P_]);
@@ -402,8 +381,9 @@ SPD_FN void flux(const S* W, S* F, double gamma, int idim, bool iso = false) {
 // Sound speed with floor (src/hydro.py:3-46).
 template <class S, int BM = 0>
 SPD_FN S sound_speed(const S& P, const S& rho, double gamma, double min_c2,
-                                         Br<BM>* br = nullptr, const S* rrho = nullptr) {
-  S c2 = rrho ? div_by(gamma * P, rho, *rrho) : gamma * P / rho;
+                                         Br<BM>* br = nullptr,
+                                         const typename RecipOf<S>::T* rrho = nullptr) {
+  S c2 = div_by(gamma * P, rho, rrho ? *rrho : recip_of(rho));
   c2 = pick(br, fgt(c2, min_c2)) ? c2 : S(min_c2);
   return ad_sqrt(c2);
 }
@@ -411,13 +391,14 @@ SPD_FN S sound_speed(const S& P, const S& rho, double gamma, double min_c2,
 // LLF (src/riemann_solver.py:31-65).
 template <int D, class S, int BM = 0>
 SPD_FN void llf(const S* WL, const S* WR, const S* UL, const S* UR, S* F, double gamma,
-                                    double min_c2, int idim, Br<BM>* br = nullptr, const S* rL = nullptr,
-                                    const S* rR = nullptr, bool iso = false) {
+                                    double min_c2, int idim, Br<BM>* br = nullptr, const typename RecipOf<S>::T* rL = nullptr,
+                                    const typename RecipOf<S>::T* rR = nullptr, bool iso = false,
+                                    const Rcp* rg = nullptr) {
   constexpr int V = D + 2, P_ = D + 1;
   const int v1 = rvel<D>(idim, 0);
   S FL[V], FR[V];
-  flux<D>(WL, FL, gamma, idim, iso);
-  flux<D>(WR, FR, gamma, idim, iso);
+  flux<D>(WL, FL, gamma, idim, iso, rg);
+  flux<D>(WR, FR, gamma, idim, iso, rg);
   const S cL = sound_speed(WL[P_], WL[0], gamma, min_c2, br, rL) + abs_br(WL[v1], br);
   const S cR = sound_speed(WR[P_], WR[0], gamma, min_c2, br, rR) + abs_br(WR[v1], br);
   const S cmax = pick(br, fgt(cL, cR)) ? cL : cR;
@@ -431,7 +412,7 @@ SPD_FN void llf(const S* WL, const S* WR, const S* UL, const S* UR, S* F, double
 template <int D, class S, int BM = 0>
 SPD_FN void hllc(const S* WL, const S* WR, const S* UL, const S* UR, S* F, double gamma,
                                      double min_c2, int idim, bool low_mach, Br<BM>* br = nullptr,
-                                     const S* rL = nullptr, const S* rR = nullptr, bool iso = false) {
+                                     const typename RecipOf<S>::T* rL = nullptr, const typename RecipOf<S>::T* rR = nullptr, bool iso = false) {
   constexpr int P_ = D + 1;
   const int v1 = rvel<D>(idim, 0);
   const S cL = sound_speed(WL[P_], WL[0], gamma, min_c2, br, rL) + abs_br(WL[v1], br);
@@ -443,7 +424,7 @@ SPD_FN void hllc(const S* WL, const S* WR, const S* UL, const S* UR, S* F, doubl
   const S rcL = WL[0] * (vL - sL);
   const S rcR = WR[0] * (sR - vR);
   const S den = rcR + rcL;
-  const S rden = recip_of(den);
+  const auto rden = recip_of(den);
   const S vstar = div_by(rcR * vR + rcL * vL + (WL[P_] - WR[P_]), den, rden);
   S Pstar;
   if (low_mach) {
@@ -474,7 +455,7 @@ SPD_FN void hllc(const S* WL, const S* WR, const S* UL, const S* UR, S* F, doubl
       const S s = lft ? sL : sR, v = lft ? vL : vR;
       const S w0 = lft ? WL[0] : WR[0], wP = lft ? WL[P_] : WR[P_], uP = lft ? UL[P_] : UR[P_];
       const S d = s - vstar;
-      const S rd = recip_of(d);
+      const auto rd = recip_of(d);
       r = div_by(w0 * (s - v), d, rd);
       e = div_by((s - v) * uP - wP * v + Pstar * vstar, d, rd);
       vg = vstar; Pg = Pstar;
@@ -485,13 +466,13 @@ SPD_FN void hllc(const S* WL, const S* WR, const S* UL, const S* UR, S* F, doubl
     r = WL[0]; vg = vL; Pg = WL[P_]; e = UL[P_];
   } else if (pick(br, fgt(vstar, 0.0))) {
     const S d = sL - vstar;
-    const S rd = recip_of(d);
+    const auto rd = recip_of(d);
     r = div_by(WL[0] * (sL - vL), d, rd);
     e = div_by((sL - vL) * UL[P_] - WL[P_] * vL + Pstar * vstar, d, rd);
     vg = vstar; Pg = Pstar;
   } else if (pick(br, fgt(sR, 0.0))) {
     const S d = sR - vstar;
-    const S rd = recip_of(d);
+    const auto rd = recip_of(d);
     r = div_by(WR[0] * (sR - vR), d, rd);
     e = div_by((sR - vR) * UR[P_] - WR[P_] * vR + Pstar * vstar, d, rd);
     vg = vstar; Pg = Pstar;
@@ -516,17 +497,18 @@ SPD_FN void hllc(const S* WL, const S* WR, const S* UL, const S* UR, S* F, doubl
 // (prims=false) or primitive (prims=true); rotated velocity order.
 template <int D, class S, int BM = 0>
 SPD_FN void riemann(int solver, const S* ML, const S* MR, S* F, double gamma, double min_c2,
-                                        int idim, bool prims, Br<BM>* br = nullptr, bool iso = false) {
+                                        int idim, bool prims, Br<BM>* br = nullptr, bool iso = false,
+                                        const Rcp* rg = nullptr) {
   constexpr int V = D + 2;
   S WL[V], WR[V], UL[V], UR[V];
-  S rL, rR;  // 1/rho of the two states when the conversion computed it
-  const S* prL = nullptr;
-  const S* prR = nullptr;
+  typename RecipOf<S>::T rL, rR;  // 1/rho of the two states when the conversion computed it
+  const typename RecipOf<S>::T* prL = nullptr;
+  const typename RecipOf<S>::T* prR = nullptr;
   if (prims) {
 #pragma unroll
     for (int v = 0; v < V; ++v) { WL[v] = ML[v]; WR[v] = MR[v]; }
-    cons<D>(WL, UL, gamma, idim, iso);
-    cons<D>(WR, UR, gamma, idim, iso);
+    cons<D>(WL, UL, gamma, idim, iso, rg);
+    cons<D>(WR, UR, gamma, idim, iso, rg);
   } else {
 #pragma unroll
     for (int v = 0; v < V; ++v) { UL[v] = ML[v]; UR[v] = MR[v]; }
@@ -535,7 +517,7 @@ SPD_FN void riemann(int solver, const S* ML, const S* MR, S* F, double gamma, do
     prL = &rL;
     prR = &rR;
   }
-  if (solver == RS_LLF) llf<D, S, BM>(WL, WR, UL, UR, F, gamma, min_c2, idim, br, prL, prR, iso);
+  if (solver == RS_LLF) llf<D, S, BM>(WL, WR, UL, UR, F, gamma, min_c2, idim, br, prL, prR, iso, rg);
   else hllc<D, S, BM>(WL, WR, UL, UR, F, gamma, min_c2, idim, solver == RS_LHLLC, br, prL, prR, iso);
 }
 
@@ -570,7 +552,7 @@ SPD_FN double dot_dir(const double* A, const double* x, int idim) {
 // Limiters (src/muscl.py:12-59); NaN semantics follow the np.where forms.
 // (comparisons through fgt / fge: integer keys on the device)
 SPD_FN double minmod(double SL, double SR) {
-  double r = SR / SL;
+  double r = quot(SR, SL);
   r = fgt(1.0, r) ? r : 1.0;
   return (fgt(r, 0.0) ? r : 0.0) * SL;
 }
@@ -578,8 +560,9 @@ SPD_FN double np_sign(double x) {
   return fgt(x, 0.0) ? 1.0 : (fgt(0.0, x) ? -1.0 : ((fge(x, 0.0) && fge(0.0, x)) ? 0.0 : x));
 }
 SPD_FN double moncen(double dUL, double dUR, double dxL, double dxR, double dxM) {
-  const double dUC = (dxL * dUL + dxR * dUR) / (dxL + dxR);
-  double slope = np_min(abs_bits(2.0 * dUL * dxL / dxM), abs_bits(2.0 * dUR * dxR / dxM));
+  const double dUC = quot(dxL * dUL + dxR * dUR, dxL + dxR);
+  const Rcp rM = recip_of(dxM);
+  double slope = np_min(abs_bits(div_by(2.0 * dUL * dxL, dxM, rM)), abs_bits(div_by(2.0 * dUR * dxR, dxM, rM)));
   slope = np_sign(dUC) * np_min(slope, abs_bits(dUC));
   return fge(dUL * dUR, 0.0) ? slope : 0.0;
 }

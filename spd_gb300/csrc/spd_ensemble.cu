@@ -294,7 +294,7 @@ const char* spd_ensemble_last_error(const spd_ensemble* E) { return E ? E->err.c
 
 int spd_set_cells_per_block(spd_ctx* C, int cpb) {
   if (!C || cpb < 1 || cpb > C->stepper->max_cpb || (cpb & (cpb - 1))) return SPD_ERR_ARG;
-  if (C->stepper->cpb != cpb && C->step_exec) {
+  if ((C->stepper->cpb != cpb || C->stepper->auto_cpb) && C->step_exec) {
     // the captured step carries the old launch shape
     cudaStreamSynchronize(C->stream);
     cudaGraphExecDestroy(C->step_exec);
@@ -307,6 +307,7 @@ int spd_set_cells_per_block(spd_ctx* C, int cpb) {
     C->dt_graph = nullptr;
   }
   C->stepper->cpb = cpb;
+  C->stepper->auto_cpb = false;
   return SPD_OK;
 }
 

@@ -13,10 +13,11 @@ struct FvGeo {
   const double* centers[3];  // extended subcell centres, Xe_d values
   const double* hfp[3];      // extended subcell widths, Xe_d values
   const double* hcv[3];      // extended centre distances, Xe_d - 1 values
-  const double* rdx[3];      // 1 / dx (correctly rounded)
-  const double* rhcv[3];     // 1 / hcv (correctly rounded)
+  const Rcp* rdx[3];      // reciprocals of dx
+  const Rcp* rhcv[3];     // reciprocals of hcv
+  const double* ihcv[3];  // 1 / hcv (the adjoint's products)
   const double* c2[3];       // centres[j+1] - centres[j-1], Xe_d values (ends unused)
-  const double* rc2[3];      // 1 / c2 (correctly rounded)
+  const Rcp* rc2[3];      // reciprocals of c2
 };
 
 __device__ __forceinline__ void q_coords(const Geo& g, long long q, int& ix, int& iy, int& iz) {
@@ -84,13 +85,13 @@ __device__ __forceinline__ void prims_cv(const Geo& g, const double* u, double* 
                                          const double* __restrict__ Weq, long long q) {
   constexpr int V = D + 2;
   if (Ueq == nullptr) {
-    prim<D>(u, W, g.gamma, 0, (double*)nullptr, g.iso != 0);
+    prim<D>(u, W, g.gamma, 0, nullptr, g.iso != 0);
     return;
   }
   double uf[V];
 #pragma unroll
   for (int v = 0; v < V; ++v) uf[v] = u[v] + Ueq[(long long)v * g.Nq + q];
-  prim<D>(uf, W, g.gamma, 0, (double*)nullptr, g.iso != 0);
+  prim<D>(uf, W, g.gamma, 0, nullptr, g.iso != 0);
 #pragma unroll
   for (int v = 0; v < V; ++v) W[v] = W[v] - Weq[(long long)v * g.Nq + q];
 }
@@ -106,7 +107,7 @@ __device__ __forceinline__ void flux_divergence(const Geo& g, const FvGeo& fg, i
     const long long nf = n_faces(g, d);
     const long long fl = face_id(g, d, ix, iy, iz);
     const long long fr = face_id(g, d, ix + (d == 0), iy + (d == 1), iz + (d == 2));
-    const double part = div_rcp(F[d][(long long)v * nf + fr] - F[d][(long long)v * nf + fl], fg.dx[d][ii[d]],
+    const double part = div_by(F[d][(long long)v * nf + fr] - F[d][(long long)v * nf + fl], fg.dx[d][ii[d]],
                                 fg.rdx[d][ii[d]]);
     acc = (d == 0) ? part : acc + part;
   }
@@ -340,7 +341,7 @@ __global__ void k_nad(Geo g, double tol, int delta, int relax, const double* __r
 // active subcell i (src/trouble_detection.py:104-137, including its
 // one-sided minimum at the first and last active subcell).
 __device__ __forceinline__ double sed_alpha_dir(const double* W, long long e0, long long st, int i, int Xd,
-                                                const double* c2, const double* rc2, const double* hfp) {
+                                                const double* c2, const Rcp* rc2, const double* hfp) {
   // line accessors in extended coordinates j along d; c2[j] = cen[j+1] -
   // cen[j-1] and rc2[j] its correctly rounded reciprocal (the quotients
   // below are the IEEE ones, div_rcp)
@@ -352,23 +353,23 @@ __device__ __forceinline__ double sed_alpha_dir(const double* W, long long e0, l
 #pragma unroll
   for (int o = 0; o < 5; ++o) {
     const int j = k - 2 + o;
-    if (j >= lo && j <= hi) dUs[o] = div_rcp(U(j + 1) - U(j - 1), c2[j], rc2[j]);
+    if (j >= lo && j <= hi) dUs[o] = div_by(U(j + 1) - U(j - 1), c2[j], rc2[j]);
   }
   auto dU = [&](int j) { return dUs[j - (k - 2)]; };
   auto aLR = [&](int kk, double& aL, double& aR) {
     const double dUm = dU(kk - 1), dU0 = dU(kk), dUp = dU(kk + 1);
-    const double d2U = div_rcp(dUp - dUm, c2[kk], rc2[kk]);
+    const double d2U = div_by(dUp - dUm, c2[kk], rc2[kk]);
     const double dv = 0.5 * hfp[kk] * d2U;
-    const double rdv = 1.0 / dv;
+    const Rcp rdv = recip_of(dv);
     const double vL = dUm - dU0;
     const double vR = dUp - dU0;
     // comparisons on the integer keys / words (IEEE semantics)
     const double selL = fgt(0.0, dv) ? (fgt(vL, 0.0) ? vL : 0.0) : (fgt(0.0, vL) ? vL : 0.0);
-    aL = div_rcp(-selL, dv, rdv);
+    aL = div_by(-selL, dv, rdv);
     if (!nonzero_w(dv)) aL = 1.0;  // |dv| <= 0
     aL = fgt(1.0, aL) ? aL : 1.0;
     const double selR = fgt(dv, 0.0) ? (fgt(vR, 0.0) ? vR : 0.0) : (fgt(0.0, vR) ? vR : 0.0);
-    aR = div_rcp(selR, dv, rdv);
+    aR = div_by(selR, dv, rdv);
     if (!nonzero_w(dv)) aR = 1.0;
     aR = fgt(1.0, aR) ? aR : 1.0;
   };
@@ -716,12 +717,12 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, const FvGeo& fg,
     const long long st = ext_stride(g, d);
     const int k = c[d];
     const double hl = fg.hcv[d][k - 1], hr = fg.hcv[d][k], hm = fg.hfp[d][k];
-    const double rhl = fg.rhcv[d][k - 1], rhr = fg.rhcv[d][k];
+    const Rcp rhl = fg.rhcv[d][k - 1], rhr = fg.rhcv[d][k];
 #pragma unroll
     for (int v = 0; v < V; ++v) {
       const double* M = W_ext + (long long)v * g.Nqe;
-      const double SL = div_rcp(M[e] - M[e - st], hl, rhl);
-      const double SR = div_rcp(M[e + st] - M[e], hr, rhr);
+      const double SL = div_by(M[e] - M[e - st], hl, rhl);
+      const double SR = div_by(M[e + st] - M[e], hr, rhr);
       double dm;
       if (BM == 0) dm = (limiter == LIM_MINMOD) ? minmod(SL, SR) : moncen(SL, SR, hl, hr, hm);
       else dm = limiter_br<BM>(limiter, SL, SR, hl, hr, hm, &ltape[((long long)d * V + v) * g.Nqe + e]);
@@ -730,8 +731,8 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, const FvGeo& fg,
       if (wb) {
         // the equilibrium's limited gradient (src/muscl.py:203-204)
         const double* Q = Meq + (long long)v * g.Nqe;
-        const double QL = div_rcp(Q[e] - Q[e - st], hl, rhl);
-        const double QR = div_rcp(Q[e + st] - Q[e], hr, rhr);
+        const double QL = div_by(Q[e] - Q[e - st], hl, rhl);
+        const double QR = div_by(Q[e + st] - Q[e], hr, rhr);
         dMq[d][v] = (limiter == LIM_MINMOD) ? minmod(QL, QR) : moncen(QL, QR, hl, hr, hm);
       }
     }
@@ -741,6 +742,7 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, const FvGeo& fg,
   double Wf[V];
 #pragma unroll
   for (int v = 0; v < V; ++v) Wf[v] = wb ? W[v] + Meq[(long long)v * g.Nqe + e] : W[v];
+  const Rcp rrho = recip_of(Wf[0]);
   double dtW[V];
 #pragma unroll
   for (int v = 0; v < V; ++v) dtW[v] = 0.0;
@@ -750,7 +752,7 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, const FvGeo& fg,
     const double* dW = dMh[d];
     dtW[0] = dtW[0] - (Wf[vel] * dW[0] + Wf[0] * dW[vel]);
     dtW[P_] = dtW[P_] - (Wf[vel] * dW[P_] + g.gamma * Wf[P_] * dW[vel]);
-    dtW[vel] = dtW[vel] - (Wf[vel] * dW[vel] + dW[P_] / Wf[0]);
+    dtW[vel] = dtW[vel] - (Wf[vel] * dW[vel] + div_by(dW[P_], Wf[0], rrho));
     if (wb) {
       // src/muscl.py:167-170; the transverse terms then use the
       // equilibrium gradient, as the reference's reassigned dW does
@@ -768,7 +770,7 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, const FvGeo& fg,
 #pragma unroll
     for (int d = 0; d < D; ++d) active = active && c[d] >= NGH && c[d] < NGH + g.X[d];
     if (active) {
-      const double drho = (Wf[0] - Meq[e]) / Wf[0];
+      const double drho = div_by(Wf[0] - Meq[e], Wf[0], rrho);
       const long long q = (c[0] - NGH) + (long long)g.X[0] * ((D > 1 ? c[1] - NGH : 0) +
                                                             (long long)g.X[1] * (D > 2 ? c[2] - NGH : 0));
 #pragma unroll
@@ -841,7 +843,7 @@ static __device__ __forceinline__ void face(const Geo& g, int d, int solver, lon
   }
   Br<BM> br;
   if (BM == 2) br.w = ftape[fidx];
-  riemann<D, double, BM>(solver, ML, MR, F, g.gamma, g.min_c2, d, true, &br, g.iso != 0);
+  riemann<D, double, BM>(solver, ML, MR, F, g.gamma, g.min_c2, d, true, &br, g.iso != 0, &g.rgm1);
   if (BM == 1) ftape[fidx] = br.w;
 #pragma unroll
   for (int v = 0; v < V; ++v) F_FB[(long long)v * nf + fidx] = Fq ? F[v] - Fq[(long long)v * nf + fidx] : F[v];
@@ -898,7 +900,7 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, const FvGeo& fg,
         else if (a != 0.0) Fv[s] = a * FB[d][(long long)v * nf + fs[s]] + (1.0 - a) * ho;
         else Fv[s] = ho;
       }
-      const double part = div_rcp(Fv[1] - Fv[0], fg.dx[d][ii[d]], fg.rdx[d][ii[d]]);
+      const double part = div_by(Fv[1] - Fv[0], fg.dx[d][ii[d]], fg.rdx[d][ii[d]]);
       acc = (d == 0) ? part : acc + part;
     }
     dudt[v] = acc;
@@ -962,7 +964,7 @@ struct WbEnd {
       u[v] = U_cv[(long long)v * g.Nq + q] + Ueq[(long long)v * g.Nq + q];
       U_cv[(long long)v * g.Nq + q] = u[v];
     }
-    prim<D>(u, W, g.gamma, 0, (double*)nullptr, g.iso != 0);
+    prim<D>(u, W, g.gamma, 0, nullptr, g.iso != 0);
 #pragma unroll
     for (int v = 0; v < V; ++v) W_cv[(long long)v * g.Nq + q] = W[v];
   }

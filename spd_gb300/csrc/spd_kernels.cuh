@@ -12,9 +12,12 @@
 //   FV     [v][iz][iy][ix]         subcell arrays (U_cv, W_cv, U_new)
 //   ext    [v][ze][ye][xe]         subcell arrays with 2 ghost layers
 #pragma once
-#include "spd_device.cuh"
+#include "spd_lines.cuh"
 
 namespace spd {
+
+// threads per block of the interior kernel at most
+constexpr int INTERIOR_THREADS = 512;
 
 struct Ops {
   double sp_to_fp[MAXNF * MAXN];
@@ -22,10 +25,19 @@ struct Ops {
   double sp_to_cv[MAXN * MAXN];
   double invader[MAXT * MAXT];
   double w_tp[MAXT];
-  // dfp_to_sp * (1/h_d) for directions whose h_d is a power of two: scaling
-  // every product and partial sum of the derivative by 2^k is exact (away
-  // from underflow and overflow), so sum(dfp*F)*(1/h) == sum((dfp/h)*F)
-  double dfp_h[3][MAXN * MAXNF];
+  // the same matrices as operands of the integer-pipe products; ``soft``:
+  // every entry is in their range
+  Coef c_sp_to_fp[MAXNF * MAXN];
+  Coef c_dfp[MAXN * MAXNF];
+  Coef c_sp_to_cv[MAXN * MAXN];
+  Coef c_invader[MAXT * MAXT];
+  Coef c_w_tp[MAXT];
+  int soft;
+  // 1/h_d as a power of two, k << 20, for directions whose h_d is one
+  // (Geo::h_pow2), else 0: scaling every product and partial sum of the
+  // derivative by 2^k is exact (away from underflow and overflow), so
+  // sum(dfp*F)*(1/h) == sum((dfp/h)*F)
+  unsigned dfp_eoff[3];
 };
 
 struct Geo {
@@ -37,7 +49,9 @@ struct Geo {
   long long Nq;    // subcells
   long long Nqe;   // extended subcells
   double h[3];
-  double inv_h[3];  // 1/h, used only when h is a power of two (then x/h == x*(1/h) exactly)
+  double inv_h[3];  // 1/h (the adjoint's products)
+  Rcp rh[3];        // reciprocals of h and gamma - 1 for quotients
+  Rcp rgm1;
   int h_pow2[3];
   double gamma, min_c2;
   int bc[3][2];
@@ -81,28 +95,37 @@ __host__ __device__ __forceinline__ long long n_iface(const Geo& g, int d) {
 }
 
 // ---------------------------------------------------------------------------
-// edge traces of one (cell, time node): sp -> fp 0 and fp nf-1 along every
-// direction (src/sdader_simulator.py:220, src/transforms.py:3-25)
+// edge traces of one line along DIR: sp -> fp 0 and fp nf-1
+// (src/sdader_simulator.py:220, src/transforms.py:3-25).  ``at(v, s)`` gives
+// variable v at solution point s.
 // ---------------------------------------------------------------------------
-template <int D, int P>
-__device__ __forceinline__ void write_traces(const Ops& op, const Geo& g, const double* __restrict__ U, int Tu,
-                                             int tu, long long c, double* const* trace, int t_out) {
+template <int D, int P, bool LANES2, class At>
+__device__ __forceinline__ void trace_line(const Ops& op, const Geo& g, At at, long long c, double* trace, int t_out,
+                                           int d, int j) {
   using k = K<D, P>;
-  for (int d = 0; d < D; ++d) {
-    for (int j = 0; j < k::NJ; ++j) {
+  // one variable at a time, rolled: the products are inlined (spd_soft.cuh),
+  // and the loop keeps the kernel in the instruction cache
+#pragma unroll 1
+  for (int v = 0; v < k::V; ++v) {
+    Line<k::n> ln;
 #pragma unroll
-      for (int v = 0; v < k::V; ++v) {
-        double x[k::n];
-#pragma unroll
-        for (int s = 0; s < k::n; ++s)
-          x[s] = U[(((long long)v * Tu + tu) * k::NS + sp_index<D, P>(d, j, s)) * g.Nc + c];
-        const double l = dot_dir<k::n>(op.sp_to_fp, x, d);
-        const double r = dot_dir<k::n>(op.sp_to_fp + (k::nf - 1) * k::n, x, d);
-        trace[d][(((long long)(0 * k::V + v) * g.T + t_out) * k::NJ + j) * g.Nc + c] = l;
-        trace[d][(((long long)(1 * k::V + v) * g.T + t_out) * k::NJ + j) * g.Nc + c] = r;
-      }
-    }
+    for (int s = 0; s < k::n; ++s) ln.v[s] = at(v, sp_index<D, P>(d, j, s));
+    line_ready<k::n>(ln, op.soft);
+    double e[2];
+    line_apply<k::n, 2, LANES2>(op.c_sp_to_fp, 0, k::nf - 1, ln, e);
+    trace[(((long long)(0 * k::V + v) * g.T + t_out) * k::NJ + j) * g.Nc + c] = e[0];
+    trace[(((long long)(1 * k::V + v) * g.T + t_out) * k::NJ + j) * g.Nc + c] = e[1];
   }
+}
+// traces of line r = d*NJ + j of time node tu of an iterate U (Tu stored)
+template <int D, int P>
+__device__ __forceinline__ void write_trace(const Ops& op, const Geo& g, const double* __restrict__ U, int Tu, int tu,
+                                            long long c, int r, double* t0, double* t1, double* t2, int t_out) {
+  using k = K<D, P>;
+  auto at = [&](int v, int s) { return U[(((long long)v * Tu + tu) * k::NS + s) * g.Nc + c]; };
+  const int d = r / k::NJ;
+  if (d == 0) trace_line<D, P, true>(op, g, at, c, t0, t_out, 0, r % k::NJ);
+  else trace_line<D, P, false>(op, g, at, c, d == 1 ? t1 : t2, t_out, d, r % k::NJ);
 }
 
 // Every kernel of the step is a body ``run(Blk, args...)`` plus a plain
@@ -112,10 +135,10 @@ template <int D, int P>
 struct TracesSp {
   static __device__ __forceinline__ void run(Blk B, const Ops& op, const Geo& g, const double* __restrict__ U_sp,
                                              double* t0, double* t1, double* t2) {
-    const long long c = B.id * (long long)blockDim.x + threadIdx.x;
-    if (c >= g.Nc) return;
-    double* tr[3] = {t0, t1, t2};
-    write_traces<D, P>(op, g, U_sp, 1, 0, c, tr, 0);
+    // one thread per (cell, line)
+    const long long tid = B.id * (long long)blockDim.x + threadIdx.x;
+    if (tid >= g.Nc * (D * K<D, P>::NJ)) return;
+    write_trace<D, P>(op, g, U_sp, 1, 0, tid % g.Nc, (int)(tid / g.Nc), t0, t1, t2, 0);
   }
 };
 template <int D, int P>
@@ -128,11 +151,11 @@ template <int D, int P>
 __global__ void k_traces_ader(Ops op, Geo g, const double* __restrict__ U, int Tu, int Teff, double* t0, double* t1,
                               double* t2) {
   const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (tid >= g.Nc * Teff) return;
-  const long long c = tid % g.Nc;
-  const int t = (int)(tid / g.Nc);
-  double* tr[3] = {t0, t1, t2};
-  write_traces<D, P>(op, g, U, Tu, (Tu == 1) ? 0 : t, c, tr, t);
+  constexpr int lines = D * K<D, P>::NJ;
+  if (tid >= g.Nc * Teff * lines) return;
+  const int r = (int)(tid / g.Nc);
+  const int t = r / lines;
+  write_trace<D, P>(op, g, U, Tu, (Tu == 1) ? 0 : t, tid % g.Nc, r % lines, t0, t1, t2, t);
 }
 
 // ---------------------------------------------------------------------------
@@ -237,7 +260,8 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, int d_rt, int Te
   if (BM == 2) br.w = tape[tid];
   // the isothermal system only in the EQ form: a runtime flag costs the
   // plain form an FP64 multiply per flux (the compiler predicates it)
-  riemann<D, double, BM>(solver, ML, MR, F, g.gamma, g.min_c2, d, false, &br, EQ && g.iso != 0);
+  riemann<D, double, BM>(solver, ML, MR, F, g.gamma, g.min_c2, d, false, &br, EQ && g.iso != 0,
+                         &g.rgm1);
   if (BM == 1) tape[tid] = br.w;
 #pragma unroll
   for (int v = 0; v < k::V; ++v) Fi[(((long long)v * g.T + t) * k::NJ + j) * nI + iface] = F[v];
@@ -256,14 +280,26 @@ __global__ void k_riemann_sd(Geo g, int d_rt, int Teff, int solver, const double
 // ---------------------------------------------------------------------------
 // interior flux points, derivative, Picard update (src/sdader_simulator.py:
 // 148-200) or the final SD update (:202-208) or the flux-point output for
-// the FV update (:288-298).  Block = (CPB cells) x (rows >= Teff): rows
-// tl < Teff compute the flux derivative of time node tl (Teff = 1 in the
-// first Picard iteration, else T); after the barrier every row writes its
-// share of the outputs (time node t_out = tl, tl + rows, ...), so the first
-// iteration may run with T rows and its single computed node spread over
-// them (CPB a multiple of 32 keeps every warp in one row).
-// mode: 0 = Picard (writes U_ader and next traces), 1 = SD update of U_sp,
-//       2 = write Ffp.
+// the FV update (:288-298).  mode: 0 = Picard (writes U_ader and the next
+// traces), 1 = SD update of U_sp, 2 = write Ffp.
+//
+// Block = CPB cells x rows of threads; a row takes one (time node, line) of
+// the cells at a time.  Shared memory holds the flux derivative of the cells'
+// nodes, [(v*NS + s)*Tn + t][cell], Tn nodes stored, and per thread the
+// states and then fluxes at its line's interior flux points,
+// [v*(nf-2) + f][thread].  Lines of one direction own their points, so a
+// barrier between directions is all the accumulation needs.  Then each row
+// takes (variable, point) pairs: the T values of the derivative are read
+// once, prepared once and contracted into the T new nodes, which replace
+// them, and the lines of the new nodes give the next traces.
+//
+// Bound: the FP64 additions beside the integer pipes (spd_soft.cuh).  Rows
+// are lines, not time nodes, because the tile leaves few cells per SM: 2 KB
+// a cell in 2D at degree 3 and 25 KB in 3D at degree 4, where one block of 8
+// cells x 5 nodes was all an SM held.  The loops over variables and
+// directions are rolled, and the per-thread array is in shared memory so that
+// they can be: with every product inlined the unrolled kernel is over 100 KB
+// of instructions.
 // ---------------------------------------------------------------------------
 // EXT: optional terms, each present when its pointer is not null -- the
 // viscous fluxes G[d] (src/sdader_simulator.py:268, layout of Ffp),
@@ -273,6 +309,139 @@ __global__ void k_riemann_sd(Geo g, int d_rt, int Teff, int solver, const double
 // (src/sdader_simulator.py:154-157, src/simulator.py:197-203).
 template <int D, int P, bool EXT = false>
 struct Interior {
+using k = K<D, P>;
+struct Args {
+  int mode, Teff, Tu, Tn;
+  const double* Uin;
+  bool visc, wb, iso;
+};
+
+// lines of direction d: fluxes at the flux points, then their derivative
+// into the tile (added to the lower directions') or the flux-point output
+template <bool LANES2>
+static __device__ __forceinline__ void lines(const Ops& op, const Geo& g, const Args& a, int dd, long long c,
+                                             double* tile, double* scr, const double* __restrict__ Fi,
+                                             double* __restrict__ Ffp, const double* __restrict__ Gv,
+                                             const double* __restrict__ meq, const double* __restrict__ feq) {
+  const int d = LANES2 ? 0 : dd;
+  int cx, cy, cz;
+  cell_coords(g, c, cx, cy, cz);
+  const long long nI = n_iface(g, d);
+  const int cd = (d == 0) ? cx : (d == 1 ? cy : cz);
+  const long long il = iface_id(g, d, cx, cy, cz, cd);
+  const long long ir = iface_id(g, d, cx, cy, cz, cd + 1);
+  const int CPB = blockDim.x, NT = blockDim.x * blockDim.y;
+  constexpr int ni = k::nf - 2;
+  for (int item = threadIdx.y; item < a.Teff * k::NJ; item += (int)blockDim.y) {
+    const int t = item / k::NJ, j = item % k::NJ;
+    const int tu = (a.Tu == 1) ? 0 : t;
+#pragma unroll 1
+    for (int v = 0; v < k::V; ++v) {
+      Line<k::n> ln;
+#pragma unroll
+      for (int s = 0; s < k::n; ++s)
+        ln.v[s] = a.Uin[(((long long)v * a.Tu + tu) * k::NS + sp_index<D, P>(d, j, s)) * g.Nc + c];
+      line_ready<k::n>(ln, op.soft);
+      double m[ni];
+      line_apply<k::n, ni, LANES2>(op.c_sp_to_fp, 1, 1, ln, m);
+#pragma unroll
+      for (int f = 0; f < ni; ++f) scr[(v * ni + f) * NT] = m[f];
+    }
+#pragma unroll
+    for (int f = 0; f < ni; ++f) {
+      double M[k::V], W[k::V], Wr[k::V], F[k::V];
+#pragma unroll
+      for (int v = 0; v < k::V; ++v) M[v] = scr[(v * ni + f) * NT];
+      if (a.wb) {
+#pragma unroll
+        for (int v = 0; v < k::V; ++v) M[v] = M[v] + meq[(((long long)v * k::NJ + j) * k::nf + f + 1) * g.Nc + c];
+      }
+      prim<D>(M, W, g.gamma, 0, nullptr, a.iso);
+      // the velocities in the rotated order of direction d, as flux's own
+      // order for direction 0
+      Wr[0] = W[0];
+      Wr[D + 1] = W[D + 1];
+#pragma unroll
+      for (int q = 0; q < D; ++q) {
+        double w = W[1 + q];
+        if (D > 1) w = (d == 1) ? W[1 + (q + 1) % D] : w;
+        if (D > 2) w = (d == 2) ? W[1 + (q + 2) % D] : w;
+        Wr[1 + q] = w;
+      }
+      flux<D>(Wr, F, g.gamma, 0, a.iso, &g.rgm1);
+      scr[f * NT] = F[0];
+      scr[((D + 1) * ni + f) * NT] = F[D + 1];
+#pragma unroll
+      for (int q = 0; q < D; ++q) scr[(rvel<D>(d, q) * ni + f) * NT] = F[1 + q];
+    }
+    const bool pow2 = g.h_pow2[d] != 0;
+#pragma unroll 1
+    for (int v = 0; v < k::V; ++v) {
+      Line<k::nf> lf;
+      const double* fe = Fi + (((long long)v * g.T + t) * k::NJ + j) * nI;
+      lf.v[0] = fe[il];
+      lf.v[k::nf - 1] = fe[ir];
+#pragma unroll
+      for (int f = 0; f < ni; ++f) lf.v[f + 1] = scr[(v * ni + f) * NT];
+      if (a.wb) {
+        // F -> F' (src/sdader_simulator.py:235-237), before the viscous flux
+#pragma unroll
+        for (int f = 0; f < k::nf; ++f)
+          lf.v[f] = lf.v[f] - feq[(((long long)v * k::NJ + j) * k::nf + f) * g.Nc + c];
+      }
+      if (a.visc) {
+#pragma unroll
+        for (int f = 0; f < k::nf; ++f)
+          lf.v[f] = lf.v[f] - Gv[((((long long)v * g.T + t) * k::NJ + j) * k::nf + f) * g.Nc + c];
+      }
+      if (a.mode == 2) {
+#pragma unroll
+        for (int f = 0; f < k::nf; ++f)
+          Ffp[((((long long)v * g.T + t) * k::NJ + j) * k::nf + f) * g.Nc + c] = lf.v[f];
+        continue;
+      }
+      line_ready<k::nf>(lf, op.soft, op.dfp_eoff[d]);
+      double val[k::n];
+      line_apply<k::nf, k::n, LANES2>(op.c_dfp, 0, 1, lf, val);
+#pragma unroll
+      for (int so = 0; so < k::n; ++so) {
+        const double x = pow2 ? val[so] : div_by(val[so], g.h[d], g.rh[d]);
+        double* slot = &tile[((v * k::NS + sp_index<D, P>(d, j, so)) * a.Tn + t) * CPB + threadIdx.x];
+        *slot = LANES2 ? x : *slot + x;
+      }
+    }
+  }
+}
+
+// U_ader of one (variable, point) from the derivative of its TT nodes
+template <int TT>
+static __device__ __forceinline__ void picard(const Ops& op, const Geo& g, double* slot, int CPB, int Teff, double dt,
+                                              double usp, double* __restrict__ out, long long stride) {
+  double acc[TT];
+  if (Teff == 1) {
+    // one derivative for all nodes: one operand, TT x TT products
+    Line<1> one;
+    one.v[0] = slot[0];
+    line_ready<1>(one, op.soft);
+    double p[TT * TT];
+    line_apply<1, TT * TT, false>(op.c_invader, 0, 1, one, p);
+#pragma unroll
+    for (int t = 0; t < TT; ++t) acc[t] = sum_terms<TT, false>(p + t * TT);
+  } else {
+    Line<TT> ln;
+#pragma unroll
+    for (int p = 0; p < TT; ++p) ln.v[p] = slot[p * CPB];
+    line_ready<TT>(ln, op.soft);
+    line_apply<TT, TT, false>(op.c_invader, 0, 1, ln, acc);
+  }
+#pragma unroll
+  for (int t = 0; t < TT; ++t) {
+    const double u = usp - acc[t] * dt;
+    out[t * stride] = u;
+    slot[t * CPB] = u;
+  }
+}
+
 static __device__ __forceinline__ void run(Blk B, const Ops& op, const Geo& g, int mode, int Teff,
                                            const double* __restrict__ Uin, int Tu, const double* __restrict__ dt_ptr,
                                            double* __restrict__ U_sp, double* __restrict__ U_ader, const double* Fi0,
@@ -280,151 +449,106 @@ static __device__ __forceinline__ void run(Blk B, const Ops& op, const Geo& g, i
                                            double* tr2, double* Ffp0, double* Ffp1, double* Ffp2,
                                            const double* G0 = nullptr, const double* G1 = nullptr,
                                            const double* G2 = nullptr, const double* gphi = nullptr,
-                                           const double* const* meqs = nullptr,
-                                           const double* const* feqs = nullptr) {
-  using k = K<D, P>;
-  const double* Gv[3] = {G0, G1, G2};
-  const bool visc = EXT && G0 != nullptr;
+                                           const double* M0 = nullptr, const double* M1 = nullptr,
+                                           const double* M2 = nullptr, const double* E0 = nullptr,
+                                           const double* E1 = nullptr, const double* E2 = nullptr) {
   const bool pot = EXT && gphi != nullptr;
-  const bool wb = EXT && meqs != nullptr;
   // the isothermal system runs in the EXT form only (a runtime flag would
   // cost the plain form a predicated FP64 multiply per flux point)
-  const bool iso = EXT && g.iso != 0;
-  extern __shared__ double dudt_s[];  // [(v*NS + s)*Teff + tl][CPB]
-  const int CPB = blockDim.x;
-  const int cl = threadIdx.x, tl = threadIdx.y;
+  const Args a{mode, Teff, Tu, (mode == 0) ? g.T : Teff, Uin, EXT && G0 != nullptr, EXT && M0 != nullptr,
+               EXT && g.iso != 0};
+  extern __shared__ double dudt_s[];
+  const int CPB = blockDim.x, rows = blockDim.y;
+  const int cl = threadIdx.x, row = threadIdx.y;
   const long long c = B.id * (long long)CPB + cl;
   const bool active = c < g.Nc;
-  const double* Fi[3] = {Fi0, Fi1, Fi2};
-  double* Ffp[3] = {Ffp0, Ffp1, Ffp2};
-  const int tu = (Tu == 1) ? 0 : tl;
-  if (active && tl < Teff) {
-    int cx, cy, cz;
-    cell_coords(g, c, cx, cy, cz);
+  double* scr = dudt_s + (mode == 2 ? 0 : k::V * k::NS * a.Tn * CPB) + row * CPB + cl;
+  if (active) lines<true>(op, g, a, 0, c, dudt_s, scr, Fi0, Ffp0, G0, M0, E0);
+#pragma unroll 1
+  for (int d = 1; d < D; ++d) {
+    if (mode != 2) __syncthreads();
+    if (active)
+      lines<false>(op, g, a, d, c, dudt_s, scr, d == 1 ? Fi1 : Fi2, d == 1 ? Ffp1 : Ffp2, d == 1 ? G1 : G2,
+                   d == 1 ? M1 : M2, d == 1 ? E1 : E2);
+  }
+  if (mode == 2) return;
+  if (pot) {
+    __syncthreads();
+    // dUdt[vel] += rho * dphi_vel, dUdt[P] += m_vel * dphi_vel, direction by
+    // direction, with the iterate the fluxes came from
+    for (int i = row; active && i < Teff * k::NS; i += rows) {
+      const int s = i % k::NS, t = i / k::NS;
+      const int tu = (Tu == 1) ? 0 : t;
 #pragma unroll
-    for (int d = 0; d < D; ++d) {
-      const long long nI = n_iface(g, d);
-      const int cd = (d == 0) ? cx : (d == 1 ? cy : cz);
-      const long long il = iface_id(g, d, cx, cy, cz, cd);
-      const long long ir = iface_id(g, d, cx, cy, cz, cd + 1);
-      for (int j = 0; j < k::NJ; ++j) {
-        double u[k::V][k::n];
-#pragma unroll
-        for (int v = 0; v < k::V; ++v)
-#pragma unroll
-          for (int s = 0; s < k::n; ++s)
-            u[v][s] = Uin[(((long long)v * Tu + tu) * k::NS + sp_index<D, P>(d, j, s)) * g.Nc + c];
-        double Fl[k::V][k::nf];
-#pragma unroll
-        for (int f = 1; f < k::nf - 1; ++f) {
-          double M[k::V], W[k::V], F[k::V];
-#pragma unroll
-          for (int v = 0; v < k::V; ++v) M[v] = dot_dir<k::n>(op.sp_to_fp + f * k::n, u[v], d);
-          if (wb) {
-#pragma unroll
-            for (int v = 0; v < k::V; ++v)
-              M[v] = M[v] + meqs[d][((((long long)v * k::NJ + j) * k::nf + f)) * g.Nc + c];
-          }
-          prim<D>(M, W, g.gamma, 0, (double*)nullptr, iso);
-          flux<D>(W, F, g.gamma, d, iso);
-#pragma unroll
-          for (int v = 0; v < k::V; ++v) Fl[v][f] = F[v];
-        }
-#pragma unroll
-        for (int v = 0; v < k::V; ++v) {
-          Fl[v][0] = Fi[d][(((long long)v * g.T + tl) * k::NJ + j) * nI + il];
-          Fl[v][k::nf - 1] = Fi[d][(((long long)v * g.T + tl) * k::NJ + j) * nI + ir];
-        }
-        if (wb) {
-          // F -> F' (src/sdader_simulator.py:235-237), before the viscous flux
-#pragma unroll
-          for (int v = 0; v < k::V; ++v)
-#pragma unroll
-            for (int f = 0; f < k::nf; ++f)
-              Fl[v][f] = Fl[v][f] - feqs[d][(((long long)v * k::NJ + j) * k::nf + f) * g.Nc + c];
-        }
-        if (visc) {
-#pragma unroll
-          for (int v = 0; v < k::V; ++v)
-#pragma unroll
-            for (int f = 0; f < k::nf; ++f)
-              Fl[v][f] = Fl[v][f] - Gv[d][((((long long)v * g.T + tl) * k::NJ + j) * k::nf + f) * g.Nc + c];
-        }
-        if (mode == 2) {
-#pragma unroll
-          for (int v = 0; v < k::V; ++v)
-#pragma unroll
-            for (int f = 0; f < k::nf; ++f)
-              Ffp[d][((((long long)v * g.T + tl) * k::NJ + j) * k::nf + f) * g.Nc + c] = Fl[v][f];
-        } else {
-          const double hd = g.h[d], ihd = g.inv_h[d];
-          const bool pow2 = g.h_pow2[d] != 0;
-#pragma unroll
-          for (int v = 0; v < k::V; ++v) {
-#pragma unroll
-            for (int so = 0; so < k::n; ++so) {
-              const double val = pow2 ? dot_dir<k::nf>(op.dfp_h[d] + so * k::nf, Fl[v], d)
-                                      : div_rcp(dot_dir<k::nf>(op.dfp_to_sp + so * k::nf, Fl[v], d), hd, ihd);
-              const int s = sp_index<D, P>(d, j, so);
-              double* slot = &dudt_s[(((long long)v * k::NS + s) * Teff + tl) * CPB + cl];
-              *slot = (d == 0) ? val : *slot + val;
-            }
-          }
-        }
-      }
-    }
-    if (pot && mode != 2) {
-      // dUdt[vel] += rho * dphi_vel, dUdt[P] += m_vel * dphi_vel, direction by
-      // direction, with the iterate the fluxes came from
-      for (int s = 0; s < k::NS; ++s) {
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-          const double gp = gphi[((long long)d * k::NS + s) * g.Nc + c];
-          const double u0 = Uin[(((long long)0 * Tu + tu) * k::NS + s) * g.Nc + c];
-          const double uv = Uin[(((long long)(d + 1) * Tu + tu) * k::NS + s) * g.Nc + c];
-          double* sv = &dudt_s[((((long long)(d + 1)) * k::NS + s) * Teff + tl) * CPB + cl];
-          *sv = *sv + u0 * gp;
-          if (!iso) {
-            double* sp = &dudt_s[((((long long)(D + 1)) * k::NS + s) * Teff + tl) * CPB + cl];
-            *sp = *sp + uv * gp;
-          }
+      for (int d = 0; d < D; ++d) {
+        const double gp = gphi[((long long)d * k::NS + s) * g.Nc + c];
+        const double u0 = Uin[(((long long)0 * Tu + tu) * k::NS + s) * g.Nc + c];
+        const double uv = Uin[(((long long)(d + 1) * Tu + tu) * k::NS + s) * g.Nc + c];
+        double* sv = &dudt_s[(((d + 1) * k::NS + s) * a.Tn + t) * CPB + cl];
+        *sv = *sv + u0 * gp;
+        if (!a.iso) {
+          double* sp = &dudt_s[(((D + 1) * k::NS + s) * a.Tn + t) * CPB + cl];
+          *sp = *sp + uv * gp;
         }
       }
     }
   }
-  if (mode == 2) return;
   __syncthreads();
-  if (!active) return;
   const double dt = *dt_ptr;
-  auto dudt = [&](int v, int s, int p) -> double {
-    return dudt_s[(((long long)v * k::NS + s) * Teff + (Teff == 1 ? 0 : p)) * CPB + cl];
-  };
-  if (mode == 0) {
-    double* tr[3] = {tr0, tr1, tr2};
-    for (int t_out = tl; t_out < g.T; t_out += (int)blockDim.y) {
-      for (int v = 0; v < k::V; ++v) {
-        for (int s = 0; s < k::NS; ++s) {
-          double acc = op.invader[t_out * g.T + 0] * dudt(v, s, 0);
-          for (int p = 1; p < g.T; ++p) acc = acc + op.invader[t_out * g.T + p] * dudt(v, s, p);
-          const double usp = U_sp[((long long)v * k::NS + s) * g.Nc + c];
-          U_ader[(((long long)v * g.T + t_out) * k::NS + s) * g.Nc + c] = usp - acc * dt;
-        }
+  if (mode == 1) {
+    for (int kk = row; active && kk < k::V * k::NS; kk += rows) {
+      const double* slot = &dudt_s[kk * Teff * CPB + cl];
+      double acc;
+      if (Teff == k::n) {
+        Line<k::n> ln;
+#pragma unroll
+        for (int t = 0; t < k::n; ++t) ln.v[t] = slot[t * CPB];
+        line_ready<k::n>(ln, op.soft);
+        line_apply<k::n, 1, false>(op.c_w_tp, 0, 1, ln, &acc);
+      } else {
+        // m != p (or T = 1): Teff counts the stored nodes
+        acc = op.w_tp[0] * slot[0];
+        for (int t = 1; t < g.T; ++t) acc = acc + op.w_tp[t] * slot[(Teff == 1 ? 0 : t) * CPB];
       }
-      write_traces<D, P>(op, g, U_ader, g.T, t_out, c, tr, t_out);
-    }
-  } else {
-    for (int kk = tl; kk < k::V * k::NS; kk += (int)blockDim.y) {
-      const int v = kk / k::NS, s = kk % k::NS;
-      double acc = op.w_tp[0] * dudt(v, s, 0);
-      for (int t = 1; t < g.T; ++t) acc = acc + op.w_tp[t] * dudt(v, s, t);
-      double* u = &U_sp[((long long)v * k::NS + s) * g.Nc + c];
+      double* u = &U_sp[(long long)kk * g.Nc + c];
       *u = *u - acc * dt;
     }
+    return;
+  }
+  for (int kk = row; active && kk < k::V * k::NS; kk += rows) {
+    const int v = kk / k::NS, s = kk % k::NS;
+    double* slot = &dudt_s[kk * a.Tn * CPB + cl];
+    const double usp = U_sp[(long long)kk * g.Nc + c];
+    double* out = &U_ader[(((long long)v * g.T) * k::NS + s) * g.Nc + c];
+    const long long stride = (long long)k::NS * g.Nc;
+    if (g.T == k::n) {
+      picard<k::n>(op, g, slot, CPB, Teff, dt, usp, out, stride);
+    } else {
+      // m != p
+      double x[MAXT];
+      for (int p = 0; p < g.T; ++p) x[p] = slot[(Teff == 1 ? 0 : p) * CPB];
+      for (int t = 0; t < g.T; ++t) {
+        double acc = op.invader[t * g.T + 0] * x[0];
+        for (int p = 1; p < g.T; ++p) acc = acc + op.invader[t * g.T + p] * x[p];
+        const double u = usp - acc * dt;
+        out[t * stride] = u;
+        slot[t * CPB] = u;
+      }
+    }
+  }
+  __syncthreads();
+  if (!active) return;
+  for (int item = row; item < g.T * D * k::NJ; item += rows) {
+    const int d = item / (g.T * k::NJ), r = item % (g.T * k::NJ);
+    const int t = r / k::NJ, j = r % k::NJ;
+    auto at = [&](int v, int s) { return dudt_s[((v * k::NS + s) * g.T + t) * CPB + cl]; };
+    if (d == 0) trace_line<D, P, true>(op, g, at, c, tr0, t, 0, j);
+    else trace_line<D, P, false>(op, g, at, c, d == 1 ? tr1 : tr2, t, d, j);
   }
 }
 };
 template <int D, int P>
-__global__ void k_interior(Ops op, Geo g, int mode, int Teff, const double* __restrict__ Uin, int Tu,
+__global__ void __launch_bounds__(INTERIOR_THREADS) k_interior(Ops op, Geo g, int mode, int Teff, const double* __restrict__ Uin, int Tu,
                            const double* __restrict__ dt_ptr, double* __restrict__ U_sp, double* __restrict__ U_ader,
                            const double* Fi0, const double* Fi1, const double* Fi2, double* tr0, double* tr1,
                            double* tr2, double* Ffp0, double* Ffp1, double* Ffp2) {
@@ -442,14 +566,12 @@ struct InteriorExt {
                                              const double* gphi, const double* M0, const double* M1,
                                              const double* M2, const double* E0, const double* E1,
                                              const double* E2) {
-    const double* meqs[3] = {M0, M1, M2};
-    const double* feqs[3] = {E0, E1, E2};
     Interior<D, P, true>::run(B, op, g, mode, Teff, Uin, Tu, dt_ptr, U_sp, U_ader, Fi0, Fi1, Fi2, tr0, tr1, tr2, Ffp0,
-                              Ffp1, Ffp2, G0, G1, G2, gphi, M0 ? meqs : nullptr, feqs);
+                              Ffp1, Ffp2, G0, G1, G2, gphi, M0, M1, M2, E0, E1, E2);
   }
 };
 template <int D, int P>
-__global__ void k_interior_ext(Ops op, Geo g, int mode, int Teff, const double* __restrict__ Uin, int Tu,
+__global__ void __launch_bounds__(INTERIOR_THREADS) k_interior_ext(Ops op, Geo g, int mode, int Teff, const double* __restrict__ Uin, int Tu,
                                const double* __restrict__ dt_ptr, double* __restrict__ U_sp,
                                double* __restrict__ U_ader, const double* Fi0, const double* Fi1, const double* Fi2,
                                double* tr0, double* tr1, double* tr2, double* Ffp0, double* Ffp1, double* Ffp2,
@@ -502,20 +624,24 @@ static __device__ __forceinline__ void run(Blk B, const Ops& op, const Geo& g, i
       // along o0 (index a)
 #pragma unroll
       for (int b = 0; b < k::NJ / k::n; ++b) {
-        double x[k::n];
+        Line<k::n> ln;
 #pragma unroll
-        for (int a = 0; a < k::n; ++a) x[a] = G[a + k::n * b];
-#pragma unroll
-        for (int ao = 0; ao < k::n; ++ao) G1[ao + k::n * b] = dot_dir<k::n>(op.sp_to_cv + ao * k::n, x, o0);
+        for (int a = 0; a < k::n; ++a) ln.v[a] = G[a + k::n * b];
+        line_ready<k::n>(ln, op.soft);
+        if (o0 == 0) line_apply<k::n, k::n, true>(op.c_sp_to_cv, 0, 1, ln, &G1[k::n * b]);
+        else line_apply<k::n, k::n, false>(op.c_sp_to_cv, 0, 1, ln, &G1[k::n * b]);
       }
       if (D == 3) {
 #pragma unroll
         for (int a = 0; a < k::n; ++a) {
-          double x[k::n];
+          Line<k::n> ln;
 #pragma unroll
-          for (int b = 0; b < k::n; ++b) x[b] = G1[a + k::n * b];
+          for (int b = 0; b < k::n; ++b) ln.v[b] = G1[a + k::n * b];
+          line_ready<k::n>(ln, op.soft);
+          double o[k::n];
+          line_apply<k::n, k::n, false>(op.c_sp_to_cv, 0, 1, ln, o);  // o1 is y or z
 #pragma unroll
-          for (int bo = 0; bo < k::n; ++bo) G[a + k::n * bo] = dot_dir<k::n>(op.sp_to_cv + bo * k::n, x, o1);
+          for (int bo = 0; bo < k::n; ++bo) G[a + k::n * bo] = o[bo];
         }
       } else {
 #pragma unroll
@@ -542,87 +668,127 @@ __global__ void k_integrate_faces(Ops op, Geo g, int d, const double* __restrict
 
 // ---------------------------------------------------------------------------
 // whole-cell transforms sp <-> subcell averages (src/transforms.py:27-45)
-// Kfull[o][i] holds the operator product ((A*A)*A) of output point o and
-// input point i, formed exactly as the reference's einsum does.
-// rows = false: one left-to-right sum over all input points (contiguous
+// Kt[i][o] holds the operator product ((A*A)*A) of input point i and output
+// point o, formed exactly as the reference's einsum does.
+// ROWS = false: one left-to-right sum over all input points (contiguous
 //               input), 1D: two-lane sum, 2D with n = 2: row pairs;
-// rows = true : per-row sums along x, then the row sums in order (strided
+// ROWS = true : per-row sums along x, then the row sums in order (strided
 //               input, src/sdader_simulator.py:302-307).
+//
+// One thread per (cell, variable, tile of O output points); the input points
+// are taken in the order of the sums, each prepared once for the tile's
+// products (spd_soft.cuh).  The bound is the FP64 addition per term; a tile
+// keeps the sums in registers, where all n^d inputs of a cell at once were
+// 250 registers in 3D at degree 4.  A sum starts from -0, which leaves its
+// first term as it is.
 // ---------------------------------------------------------------------------
 template <int D, int P>
-__device__ __forceinline__ double full_dot(const double* __restrict__ Krow, const double* x, bool rows) {
+struct Full {
   using k = K<D, P>;
-  if (D == 1) return dot_lanes2<k::n>(Krow, x);
-  if (rows || (D == 2 && k::n == 2)) {
-    double acc = 0.0;
-#pragma unroll
-    for (int r = 0; r < k::NS / k::n; ++r) {
-      double rs = Krow[r * k::n] * x[r * k::n];
-#pragma unroll
-      for (int l = 1; l < k::n; ++l) rs = rs + Krow[r * k::n + l] * x[r * k::n + l];
-      acc = (r == 0) ? rs : acc + rs;
-    }
-    return acc;
+  static constexpr int O = (k::NS <= 9) ? k::NS : (k::NS % 9 == 0 ? 9 : (k::NS % 8 == 0 ? 8 : 5));
+  static constexpr int tiles = k::NS / O;
+  static_assert(k::NS % O == 0, "tiles of outputs");
+  // subcell index of point s of cell c
+  static __device__ __forceinline__ long long subcell(const Geo& g, long long c, int s) {
+    int cx, cy, cz;
+    cell_coords(g, c, cx, cy, cz);
+    const int kx = s % k::n, ky = (s / k::n) % k::n, kz = s / (k::n * k::n);
+    return (cx * k::n + kx) + (long long)g.X[0] * ((D >= 2 ? cy * k::n + ky : 0) +
+                                                  (long long)g.X[1] * (D >= 3 ? cz * k::n + kz : 0));
   }
-  return dot_seq<k::NS>(Krow, x);
-}
+  template <bool ROWS, class Get>
+  static __device__ __forceinline__ void apply(const Coef* __restrict__ Kt, int soft, int o0, Get get, double* acc) {
+    double part[O];  // the row's sum, or in 1D the sum of the odd terms
+#pragma unroll
+    for (int o = 0; o < O; ++o) acc[o] = part[o] = -0.0;
+#pragma unroll 1
+    for (int r = 0; r < k::NS / k::n; ++r) {
+#pragma unroll
+      for (int l = 0; l < k::n; ++l) {
+        const int s = r * k::n + l;
+        const Coef* K = Kt + (long long)s * k::NS + o0;
+        const double x = get(s);
+        double p[O];
+#ifdef SPD_FUSED
+#pragma unroll
+        for (int o = 0; o < O; ++o) p[o] = K[o].a * x;
+#else
+        uint32_t ok = soft ? 0x40000000u : 0u;
+        const Opnd xo = opnd_of(x, ok);
+        if (ok != 0u) {
+#pragma unroll
+          for (int o = 0; o < O; ++o) p[o] = soft_prod(K[o], xo);
+        } else {
+#pragma unroll
+          for (int o = 0; o < O; ++o) p[o] = coef_value(K[o], 0u) * x;
+        }
+#endif
+#pragma unroll
+        for (int o = 0; o < O; ++o) {
+          if (D == 1 ? l % 2 == 1 : ROWS || (D == 2 && k::n == 2))
+            part[o] = (D > 1 && l == 0) ? p[o] : part[o] + p[o];
+          else
+            acc[o] = acc[o] + p[o];
+        }
+      }
+      if (D > 1 && (ROWS || (D == 2 && k::n == 2))) {
+#pragma unroll
+        for (int o = 0; o < O; ++o) acc[o] = acc[o] + part[o];
+      }
+    }
+    if (D == 1) {
+#pragma unroll
+      for (int o = 0; o < O; ++o) acc[o] = acc[o] + part[o];
+    }
+  }
+};
 
 // U_cv (FV layout) = sp_to_cv(U_sp) for every cell and variable
 template <int D, int P>
 struct SpToCv {
-static __device__ __forceinline__ void run(Blk B, const Geo& g, const double* __restrict__ Kfull,
+static __device__ __forceinline__ void run(Blk B, const Geo& g, const Coef* __restrict__ Kt, int soft,
                                            const double* __restrict__ U_sp, double* __restrict__ U_cv) {
   using k = K<D, P>;
+  using F = Full<D, P>;
   const long long tid = B.id * (long long)blockDim.x + threadIdx.x;
-  if (tid >= g.Nc * k::V) return;
+  if (tid >= g.Nc * (k::V * F::tiles)) return;
   const long long c = tid % g.Nc;
-  const int v = (int)(tid / g.Nc);
-  int cx, cy, cz;
-  cell_coords(g, c, cx, cy, cz);
-  double x[k::NS];
+  const int r = (int)(tid / g.Nc);
+  const int v = r / F::tiles, o0 = r % F::tiles * F::O;
+  double acc[F::O];
+  F::template apply<false>(Kt, soft, o0, [&](int s) { return U_sp[((long long)v * k::NS + s) * g.Nc + c]; }, acc);
 #pragma unroll
-  for (int s = 0; s < k::NS; ++s) x[s] = U_sp[((long long)v * k::NS + s) * g.Nc + c];
-  for (int o = 0; o < k::NS; ++o) {
-    const int kx = o % k::n, ky = (o / k::n) % k::n, kz = o / (k::n * k::n);
-    const long long q = (cx * k::n + kx) + (long long)g.X[0] * ((D >= 2 ? cy * k::n + ky : 0) +
-                                                               (long long)g.X[1] * (D >= 3 ? cz * k::n + kz : 0));
-    U_cv[(long long)v * g.Nq + q] = full_dot<D, P>(Kfull + (long long)o * k::NS, x, false);
-  }
+  for (int o = 0; o < F::O; ++o) U_cv[(long long)v * g.Nq + F::subcell(g, c, o0 + o)] = acc[o];
 }
 };
 template <int D, int P>
-__global__ void k_sp_to_cv(Geo g, const double* __restrict__ Kfull, const double* __restrict__ U_sp,
+__global__ void k_sp_to_cv(Geo g, const Coef* __restrict__ Kt, int soft, const double* __restrict__ U_sp,
                            double* __restrict__ U_cv) {
-  SpToCv<D, P>::run(hw_blk(), g, Kfull, U_sp, U_cv);
+  SpToCv<D, P>::run(hw_blk(), g, Kt, soft, U_sp, U_cv);
 }
 
 // U_sp = cv_to_sp(U_cv) (strided view order)
 template <int D, int P>
 struct CvToSp {
-static __device__ __forceinline__ void run(Blk B, const Geo& g, const double* __restrict__ Kfull,
+static __device__ __forceinline__ void run(Blk B, const Geo& g, const Coef* __restrict__ Kt, int soft,
                                            const double* __restrict__ U_cv, double* __restrict__ U_sp) {
   using k = K<D, P>;
+  using F = Full<D, P>;
   const long long tid = B.id * (long long)blockDim.x + threadIdx.x;
-  if (tid >= g.Nc * k::V) return;
+  if (tid >= g.Nc * (k::V * F::tiles)) return;
   const long long c = tid % g.Nc;
-  const int v = (int)(tid / g.Nc);
-  int cx, cy, cz;
-  cell_coords(g, c, cx, cy, cz);
-  double x[k::NS];
+  const int r = (int)(tid / g.Nc);
+  const int v = r / F::tiles, o0 = r % F::tiles * F::O;
+  double acc[F::O];
+  F::template apply<true>(Kt, soft, o0, [&](int s) { return U_cv[(long long)v * g.Nq + F::subcell(g, c, s)]; }, acc);
 #pragma unroll
-  for (int s = 0; s < k::NS; ++s) {
-    const int kx = s % k::n, ky = (s / k::n) % k::n, kz = s / (k::n * k::n);
-    const long long q = (cx * k::n + kx) + (long long)g.X[0] * ((D >= 2 ? cy * k::n + ky : 0) +
-                                                               (long long)g.X[1] * (D >= 3 ? cz * k::n + kz : 0));
-    x[s] = U_cv[(long long)v * g.Nq + q];
-  }
-  for (int o = 0; o < k::NS; ++o) U_sp[((long long)v * k::NS + o) * g.Nc + c] = full_dot<D, P>(Kfull + (long long)o * k::NS, x, true);
+  for (int o = 0; o < F::O; ++o) U_sp[((long long)v * k::NS + o0 + o) * g.Nc + c] = acc[o];
 }
 };
 template <int D, int P>
-__global__ void k_cv_to_sp(Geo g, const double* __restrict__ Kfull, const double* __restrict__ U_cv,
+__global__ void k_cv_to_sp(Geo g, const Coef* __restrict__ Kt, int soft, const double* __restrict__ U_cv,
                            double* __restrict__ U_sp) {
-  CvToSp<D, P>::run(hw_blk(), g, Kfull, U_cv, U_sp);
+  CvToSp<D, P>::run(hw_blk(), g, Kt, soft, U_cv, U_sp);
 }
 
 }  // namespace spd

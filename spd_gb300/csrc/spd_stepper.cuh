@@ -1,6 +1,5 @@
 // Launch sequence of one SD-ADER step for dimension D and degree P
-// (src/sdader_simulator.py:361-378); instantiated per dimension in
-// spd_step_d1.cu, spd_step_d2.cu and spd_step_d3.cu.
+// (src/sdader_simulator.py:361-378); instantiated in spd_step.cu.
 #pragma once
 #include "spd_ctx.cuh"
 
@@ -52,7 +51,7 @@ struct PrimOnly {
     double u[V], W[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) u[v] = U_cv[(long long)v * g.Nq + q];
-    prim<D>(u, W, g.gamma, 0, (double*)nullptr, g.iso != 0);
+    prim<D>(u, W, g.gamma, 0, nullptr, g.iso != 0);
 #pragma unroll
     for (int v = 0; v < V; ++v) W_cv[(long long)v * g.Nq + q] = W[v];
   }
@@ -67,19 +66,66 @@ template <int D, int P>
 struct Stepper : StepperBase {
   using k = K<D, P>;
 
+  // Block shape of the interior kernel.  Its shared memory: the tile of
+  // (variable, point, node) values per cell and the flux points of each
+  // thread's line (mode 2 writes those out and has no tile).
+  static constexpr size_t SMEM_MAX = 227 * 1024;
+  static size_t tile_bytes(int nodes) { return (size_t)k::V * k::NS * nodes * sizeof(double); }
+  static constexpr size_t line_bytes() { return (size_t)k::V * (k::nf - 2) * sizeof(double); }
+  // thread rows: the (node, line) pairs of a cell in as few equal rounds as
+  // fit into ``threads`` per block and the shared memory
+  static int rows_for(int cells, int T, int threads) {
+    const int items = T * k::NJ;
+    int most = std::max(1, threads / cells);
+    const size_t tile = tile_bytes(T) * cells;
+    if (tile < SMEM_MAX) most = std::min<int>(most, (int)((SMEM_MAX - tile) / (line_bytes() * cells)));
+    if (tile >= SMEM_MAX || most < 1) return 0;
+    const int rounds = (items + most - 1) / most;
+    return (items + rounds - 1) / rounds;
+  }
+  static size_t interior_smem(int cells, int rows, int nodes) {
+    return (tile_bytes(nodes) + line_bytes() * rows) * cells;
+  }
+  // 256 threads where two such blocks fit an SM, else 512 (two blocks of 256
+  // overlap each other's barriers; a tile too large for that still gets its
+  // threads)
+  static int interior_rows(int cells, int T) {
+    const int r = rows_for(cells, T, 256);
+    if (r > 0 && 2 * interior_smem(cells, r, T) <= SMEM_MAX) return r;
+    return rows_for(cells, T, INTERIOR_THREADS);
+  }
+
   int configure(spd_ctx* C) override {
-    // cells per block of the interior kernel: bounded by the 227 KB of shared
-    // memory a block may use
-    const size_t per_cell = (size_t)k::V * k::NS * C->T * sizeof(double);
     max_cpb = 64;
-    while (max_cpb > 1 && per_cell * max_cpb > 227 * 1024) max_cpb /= 2;
-    cpb = std::min(32, max_cpb);
-    smem = per_cell * max_cpb;
-    CK(cudaFuncSetAttribute(k_interior<D, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CK(cudaFuncSetAttribute(k_interior_ext<D, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    while (max_cpb > 1 && interior_rows(max_cpb, C->T) < 1) max_cpb /= 2;
+    if (interior_rows(max_cpb, C->T) < 1) return fail(C, SPD_ERR_ARG, "the step's tile exceeds the shared memory");
+    // the widest block that keeps the most threads resident
+    int best = -1;
+    for (int cells = std::min(32, max_cpb); cells >= 4 || cells == max_cpb; cells /= 2) {
+      const int r = interior_rows(cells, C->T);
+      const int blocks = std::max(1, (int)(SMEM_MAX / interior_smem(cells, r, C->T)));
+      const int resident = std::min(512, blocks * r * cells);
+      if (resident > best) {
+        best = resident;
+        cpb = cells;
+      }
+      if (cells == 1) break;
+    }
+    CK(cudaFuncSetAttribute(k_interior<D, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+    CK(cudaFuncSetAttribute(k_interior_ext<D, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
     return 0;
   }
 
+  // cells per block of the interior kernel: the context's own number, or,
+  // while none was set and the step is not recorded for a batched launch
+  // (which needs one block shape for all instances), fewer where the grid
+  // would not give every SM two blocks
+  int interior_cells(const spd_ctx* C) const {
+    int cells = cpb;
+    if (auto_cpb && !C->brec)
+      while (cells > 4 && (C->geo.Nc + cells - 1) / cells < 2 * SMS) cells /= 2;
+    return cells;
+  }
   // the Riemann problems of one Picard iteration, one instantiation per
   // direction; EQ: the form with the well-balanced mode's equilibrium edge
   // values and the isothermal system
@@ -127,7 +173,7 @@ struct Stepper : StepperBase {
                          C->stream));
     {
       ProfScope ps_(C, "k_traces_sp");
-      launch<TracesSp<D, P>>(C, "k_traces_sp", k_traces_sp<D, P>, blocks_for(g.Nc, 128), 128, 0, C->ops, g, C->U_sp,
+      launch<TracesSp<D, P>>(C, "k_traces_sp", k_traces_sp<D, P>, blocks_for(g.Nc * (D * k::NJ), 128), 128, 0, C->ops, g, C->U_sp,
                              C->trace[0], C->trace[1], C->trace[2]);
     }
     CKL();
@@ -163,7 +209,8 @@ struct Stepper : StepperBase {
         // viscous fluxes of this iteration (src/sdader_simulator.py:239-268)
         {
           ProfScope ps_(C, "k_visc_grad");
-          launch<ViscGrad<D, P>>(C, "k_visc_grad", k_visc_grad<D, P>, blocks_for(g.Nc * Teff, 128), 128, 0, C->ops,
+          launch<ViscGrad<D, P>>(C, "k_visc_grad", k_visc_grad<D, P>,
+                                 blocks_for(g.Nc * (D * k::NJ) * Teff, VISC_THREADS), VISC_THREADS, 0, C->ops,
                                  g, Teff, Uin, Tu, C->trace[0], C->trace[1], C->trace[2], C->bcfix[0], C->bcfix[1],
                                  C->bcfix[2], C->Wfp[0], C->Wfp[1], C->Wfp[2], C->dWsp, (const double*)C->Meq_fp[0],
                                  (const double*)C->Meq_fp[1], (const double*)C->Meq_fp[2]);
@@ -171,21 +218,19 @@ struct Stepper : StepperBase {
         CKL();
         {
           ProfScope ps_(C, "k_visc_flux");
-          launch<ViscFlux<D, P>>(C, "k_visc_flux", k_visc_flux<D, P>, blocks_for(g.Nc * Teff, 128), 128, 0, C->ops,
+          launch<ViscFlux<D, P>>(C, "k_visc_flux", k_visc_flux<D, P>,
+                                 blocks_for(g.Nc * (D * k::NJ) * Teff, VISC_THREADS), VISC_THREADS, 0, C->ops,
                                  g, Teff, C->dWsp, C->Wfp[0], C->Wfp[1], C->Wfp[2], C->bcfix[0], C->bcfix[1],
                                  C->bcfix[2], C->cfg.nu, C->cfg.beta, C->Gv[0], C->Gv[1], C->Gv[2]);
         }
         CKL();
       }
-      // the first Picard iteration computes one time node but writes all T:
-      // T thread rows share its output (whole warps per row when cpb is a
-      // multiple of 32)
-      const int rows = (mode == 0 && Teff == 1 && cpb % 32 == 0) ? C->T : Teff;
-      dim3 block(cpb, rows);
-      const size_t sm = (mode == 2) ? 0 : (size_t)k::V * k::NS * Teff * cpb * sizeof(double);
+      const int cells = interior_cells(C);
+      const dim3 block(cells, interior_rows(cells, C->T));
+      const size_t sm = interior_smem(cells, block.y, mode == 2 ? 0 : (mode == 0 ? C->T : Teff));
       if (visc || C->gphi_sp || C->Ueq_sp || C->cfg.isothermal) {
         ProfScope ps_(C, "k_interior");
-        launch<InteriorExt<D, P>>(C, "k_interior", k_interior_ext<D, P>, blocks_for(g.Nc, cpb), block, sm, C->ops,
+        launch<InteriorExt<D, P>>(C, "k_interior", k_interior_ext<D, P>, blocks_for(g.Nc, cells), block, sm, C->ops,
                                   g, mode, Teff, Uin, Tu, C->dt, C->U_sp, C->U_ader, C->Fi[0], C->Fi[1], C->Fi[2],
                                   C->trace[0], C->trace[1], C->trace[2], C->Ffp[0], C->Ffp[1], C->Ffp[2],
                                   visc ? C->Gv[0] : nullptr, C->Gv[1], C->Gv[2], (const double*)C->gphi_sp,
@@ -194,7 +239,7 @@ struct Stepper : StepperBase {
                                   (const double*)C->Feq_fp[1], (const double*)C->Feq_fp[2]);
       } else {
         ProfScope ps_(C, "k_interior");
-        launch<Interior<D, P>>(C, "k_interior", k_interior<D, P>, blocks_for(g.Nc, cpb), block, sm, C->ops, g, mode,
+        launch<Interior<D, P>>(C, "k_interior", k_interior<D, P>, blocks_for(g.Nc, cells), block, sm, C->ops, g, mode,
                                Teff, Uin, Tu, C->dt, C->U_sp, C->U_ader, C->Fi[0], C->Fi[1], C->Fi[2], C->trace[0],
                                C->trace[1], C->trace[2], C->Ffp[0], C->Ffp[1], C->Ffp[2]);
       }
@@ -212,8 +257,9 @@ struct Stepper : StepperBase {
     const Geo& g = C->geo;
     {
       ProfScope ps_(C, "k_sp_to_cv");
-      launch<SpToCv<D, P>>(C, "k_sp_to_cv", k_sp_to_cv<D, P>, blocks_for(g.Nc * k::V, 128), 128, 0, g, C->K_sp_to_cv,
-                           C->U_sp, C->U_cv);
+      launch<SpToCv<D, P>>(C, "k_sp_to_cv", k_sp_to_cv<D, P>,
+                           blocks_for(g.Nc * (k::V * Full<D, P>::tiles), 128), 128, 0, g,
+                           (const Coef*)C->Kt_sp_to_cv, C->K_soft, C->U_sp, C->U_cv);
     }
     CKL();
     return 0;
@@ -441,8 +487,9 @@ struct Stepper : StepperBase {
     // switch_to_high_order (src/sdader_simulator.py:300-307)
     {
       ProfScope ps_(C, "k_cv_to_sp");
-      launch<CvToSp<D, P>>(C, "k_cv_to_sp", k_cv_to_sp<D, P>, blocks_for(g.Nc * k::V, 128), 128, 0, g, C->K_cv_to_sp,
-                           C->U_cv, C->U_sp);
+      launch<CvToSp<D, P>>(C, "k_cv_to_sp", k_cv_to_sp<D, P>,
+                           blocks_for(g.Nc * (k::V * Full<D, P>::tiles), 128), 128, 0, g,
+                           (const Coef*)C->Kt_cv_to_sp, C->K_soft, C->U_cv, C->U_sp);
     }
     CKL();
     return 0;
@@ -566,15 +613,9 @@ struct Stepper : StepperBase {
   }
 };
 
-template <int D>
-StepperBase* make_stepper_for(int P) {
-  switch (P) {
-    case 1: return new Stepper<D, 1>();
-    case 2: return new Stepper<D, 2>();
-    case 3: return new Stepper<D, 3>();
-    case 4: return new Stepper<D, 4>();
-    default: return nullptr;
-  }
+template <int D, int P>
+StepperBase* make_stepper_of() {
+  return new Stepper<D, P>();
 }
 
 }  // namespace spd_host

@@ -24,9 +24,15 @@
 // initial conservative edge traces, unchanged; pressure -> the same stored
 // values, which also overwrite the domain-edge point of the array itself.
 #pragma once
+#include <type_traits>
+
 #include "spd_kernels.cuh"
 
 namespace spd {
+
+// threads per block: the flux points of a line, 720 bytes a thread in 3D at
+// degree 4, in 48 KB of shared memory
+constexpr int VISC_THREADS = 64;
 
 template <int D, int P>
 struct ViscGrad {
@@ -37,21 +43,27 @@ struct ViscGrad {
                                              double* W2, double* __restrict__ dWsp, const double* mq0,
                                              const double* mq1, const double* mq2) {
     using k = K<D, P>;
+    // primitives at the flux points of the thread's line (shared memory, so
+    // that the loops over variables can stay rolled)
+    __shared__ double scr[k::V * k::nf * VISC_THREADS];
+    auto Wf = [&](int v, int f) -> double& { return scr[(v * k::nf + f) * VISC_THREADS + threadIdx.x]; };
     // well-balanced mode: the conservative equilibrium at the flux points is
     // part of the state whose primitives are taken (src/sdader_simulator.py:221-223)
     const double* meq[3] = {mq0, mq1, mq2};
     const long long tid = B.id * (long long)blockDim.x + threadIdx.x;
-    if (tid >= g.Nc * Teff) return;
+    // one thread per (cell, direction, node, line)
+    if (tid >= g.Nc * (D * k::NJ) * Teff) return;
     const long long c = tid % g.Nc;
-    const int t = (int)(tid / g.Nc);
+    const int r = (int)(tid / g.Nc);
+    const int dir = r / (Teff * k::NJ), t = r / k::NJ % Teff, j = r % k::NJ;
     const int tu = (Tu == 1) ? 0 : t;
     const double* trace[3] = {tr0, tr1, tr2};
     const double* bcfix[3] = {bf0, bf1, bf2};
     double* Wfp[3] = {W0, W1, W2};
     int cx, cy, cz;
     cell_coords(g, c, cx, cy, cz);
-#pragma unroll 1
-    for (int d = 0; d < D; ++d) {
+    auto line = [&](auto dc) {
+      constexpr int d = decltype(dc)::value;
       const int cd = (d == 0) ? cx : (d == 1 ? cy : cz);
       const int Nd = g.N[d];
       const int b0 = g.bc[d][0], b1 = g.bc[d][1];
@@ -59,7 +71,7 @@ struct ViscGrad {
       const long long ntrans = g.Nc / Nd;
       const long long ct = (d == 0) ? (cy + (long long)g.N[1] * cz) : (d == 1 ? (cx + (long long)g.N[0] * cz)
                                                                               : (cx + (long long)g.N[0] * cy));
-      for (int j = 0; j < k::NJ; ++j) {
+      {
         auto tr = [&](int side, int v, long long cell) -> double {
           double val = trace[d][(((long long)(side * k::V + v) * g.T + t) * k::NJ + j) * g.Nc + cell];
           if (meq[0]) val = val + meq[d][(((long long)v * k::NJ + j) * k::nf + (side ? k::nf - 1 : 0)) * g.Nc + cell];
@@ -68,24 +80,29 @@ struct ViscGrad {
         auto fix = [&](int side, int v) -> double {
           return bcfix[d][(((long long)side * k::V + v) * k::NJ + j) * ntrans + ct];
         };
-        double Wf[k::V][k::nf];
-        double u[k::V][k::n];
-#pragma unroll
-        for (int v = 0; v < k::V; ++v)
+#pragma unroll 1
+        for (int v = 0; v < k::V; ++v) {
+          Line<k::n> ln;
 #pragma unroll
           for (int s = 0; s < k::n; ++s)
-            u[v][s] = Uin[(((long long)v * Tu + tu) * k::NS + sp_index<D, P>(d, j, s)) * g.Nc + c];
+            ln.v[s] = Uin[(((long long)v * Tu + tu) * k::NS + sp_index<D, P>(d, j, s)) * g.Nc + c];
+          line_ready<k::n>(ln, op.soft);
+          double m[k::nf - 2];
+          line_apply<k::n, k::nf - 2, d == 0>(op.c_sp_to_fp, 1, 1, ln, m);
+#pragma unroll
+          for (int f = 1; f < k::nf - 1; ++f) Wf(v, f) = m[f - 1];
+        }
 #pragma unroll
         for (int f = 1; f < k::nf - 1; ++f) {
           double M[k::V], W[k::V];
 #pragma unroll
           for (int v = 0; v < k::V; ++v) {
-            M[v] = dot_dir<k::n>(op.sp_to_fp + f * k::n, u[v], d);
+            M[v] = Wf(v, f);
             if (meq[0]) M[v] = M[v] + meq[d][(((long long)v * k::NJ + j) * k::nf + f) * g.Nc + c];
           }
-          prim<D>(M, W, g.gamma, 0, (double*)nullptr, g.iso != 0);
+          prim<D>(M, W, g.gamma, 0, nullptr, g.iso != 0);
 #pragma unroll
-          for (int v = 0; v < k::V; ++v) Wf[v][f] = W[v];
+          for (int v = 0; v < k::V; ++v) Wf(v, f) = W[v];
         }
         // right edge: the cell's own right-edge state (its trace), or the
         // stored state on a "pressure" side
@@ -97,10 +114,10 @@ struct ViscGrad {
           } else {
 #pragma unroll
             for (int v = 0; v < k::V; ++v) M[v] = tr(1, v, c);
-            prim<D>(M, W, g.gamma, 0, (double*)nullptr, g.iso != 0);
+            prim<D>(M, W, g.gamma, 0, nullptr, g.iso != 0);
           }
 #pragma unroll
-          for (int v = 0; v < k::V; ++v) Wf[v][k::nf - 1] = W[v];
+          for (int v = 0; v < k::V; ++v) Wf(v, k::nf - 1) = W[v];
         }
         // left edge: the right-edge state of the cell on the left, or the
         // boundary state
@@ -111,34 +128,38 @@ struct ViscGrad {
             const int side = (cd > 0 || b0 == BC_PERIODIC) ? 1 : 0;
 #pragma unroll
             for (int v = 0; v < k::V; ++v) M[v] = tr(side, v, src);
-            prim<D>(M, W, g.gamma, 0, (double*)nullptr, g.iso != 0);
+            prim<D>(M, W, g.gamma, 0, nullptr, g.iso != 0);
             if (cd == 0 && b0 == BC_REFLECTIVE) W[d + 1] = W[d + 1] * -1.0;
           } else {
 #pragma unroll
             for (int v = 0; v < k::V; ++v) W[v] = fix(0, v);
           }
 #pragma unroll
-          for (int v = 0; v < k::V; ++v) Wf[v][0] = W[v];
+          for (int v = 0; v < k::V; ++v) Wf(v, 0) = W[v];
         }
-#pragma unroll
-        for (int v = 0; v < k::V; ++v) {
-#pragma unroll
-          for (int f = 0; f < k::nf; ++f)
-            Wfp[d][((((long long)v * g.T + t) * k::NJ + j) * k::nf + f) * g.Nc + c] = Wf[v][f];
-        }
-        const double hd = g.h[d], ihd = g.inv_h[d];
         const bool pow2 = g.h_pow2[d] != 0;
-#pragma unroll
+#pragma unroll 1
         for (int v = 0; v < k::V; ++v) {
+          Line<k::nf> lf;
+#pragma unroll
+          for (int f = 0; f < k::nf; ++f) {
+            lf.v[f] = Wf(v, f);
+            Wfp[d][((((long long)v * g.T + t) * k::NJ + j) * k::nf + f) * g.Nc + c] = lf.v[f];
+          }
+          line_ready<k::nf>(lf, op.soft, op.dfp_eoff[d]);
+          double dv[k::n];
+          line_apply<k::nf, k::n, d == 0>(op.c_dfp, 0, 1, lf, dv);
 #pragma unroll
           for (int so = 0; so < k::n; ++so) {
-            const double val = pow2 ? dot_dir<k::nf>(op.dfp_h[d] + so * k::nf, Wf[v], d)
-                                    : div_rcp(dot_dir<k::nf>(op.dfp_to_sp + so * k::nf, Wf[v], d), hd, ihd);
+            const double val = pow2 ? dv[so] : div_by(dv[so], g.h[d], g.rh[d]);
             dWsp[((((long long)d * k::V + v) * g.T + t) * k::NS + sp_index<D, P>(d, j, so)) * g.Nc + c] = val;
           }
         }
       }
-    }
+    };
+    if (dir == 0) line(std::integral_constant<int, 0>());
+    if (D > 1 && dir == 1) line(std::integral_constant<int, (D > 1 ? 1 : 0)>());
+    if (D > 2 && dir == 2) line(std::integral_constant<int, (D > 2 ? 2 : 0)>());
   }
 };
 template <int D, int P>
@@ -158,17 +179,24 @@ struct ViscFlux {
                                              double* G2) {
     using k = K<D, P>;
     constexpr int P_ = D + 1;
+    // gradients at the flux points of the thread's line
+    __shared__ double scr[D * k::V * k::nf * VISC_THREADS];
+    auto gf = [&](int e, int v, int f) -> double& {
+      return scr[((e * k::V + v) * k::nf + f) * VISC_THREADS + threadIdx.x];
+    };
     const long long tid = B.id * (long long)blockDim.x + threadIdx.x;
-    if (tid >= g.Nc * Teff) return;
+    // one thread per (cell, direction, node, line)
+    if (tid >= g.Nc * (D * k::NJ) * Teff) return;
     const long long c = tid % g.Nc;
-    const int t = (int)(tid / g.Nc);
+    const int r = (int)(tid / g.Nc);
+    const int dir = r / (Teff * k::NJ), t = r / k::NJ % Teff, j = r % k::NJ;
     const double* bcfix[3] = {bf0, bf1, bf2};
     const double* Wfp[3] = {W0, W1, W2};
     double* G[3] = {G0, G1, G2};
     int cx, cy, cz;
     cell_coords(g, c, cx, cy, cz);
-#pragma unroll 1
-    for (int d = 0; d < D; ++d) {
+    auto line = [&](auto dc) {
+      constexpr int d = decltype(dc)::value;
       const int cd = (d == 0) ? cx : (d == 1 ? cy : cz);
       const int Nd = g.N[d];
       const int b0 = g.bc[d][0], b1 = g.bc[d][1];
@@ -177,7 +205,7 @@ struct ViscFlux {
       const long long ct = (d == 0) ? (cy + (long long)g.N[1] * cz) : (d == 1 ? (cx + (long long)g.N[0] * cz)
                                                                               : (cx + (long long)g.N[0] * cy));
       const int v1 = rvel<D>(d, 0);
-      for (int j = 0; j < k::NJ; ++j) {
+      {
         auto fix = [&](int side, int v) -> double {
           return bcfix[d][(((long long)side * k::V + v) * k::NJ + j) * ntrans + ct];
         };
@@ -185,35 +213,38 @@ struct ViscFlux {
           return dWsp[((((long long)e * k::V + v) * g.T + t) * k::NS + sp_index<D, P>(d, j, s)) * g.Nc + cell];
         };
         // gradients along every direction e at the flux points of d
-        double gf[D][k::V][k::nf];
+        {
+#pragma unroll 1
+          for (int ev = 0; ev < D * k::V; ++ev) {
+            const int e = ev / k::V, v = ev % k::V;
+            Line<k::n> ln;
 #pragma unroll
-        for (int e = 0; e < D; ++e) {
-#pragma unroll
-          for (int v = 0; v < k::V; ++v) {
-            double x[k::n];
-#pragma unroll
-            for (int s = 0; s < k::n; ++s) x[s] = sp_val(e, v, s, c);
-#pragma unroll
-            for (int f = 0; f < k::nf; ++f) gf[e][v][f] = dot_dir<k::n>(op.sp_to_fp + f * k::n, x, d);
+            for (int s = 0; s < k::n; ++s) ln.v[s] = sp_val(e, v, s, c);
+            line_ready<k::n>(ln, op.soft);
+            double gl[k::nf];
+            line_apply<k::n, k::nf, d == 0>(op.c_sp_to_fp, 0, 1, ln, gl);
             // left edge: the cell's own left-edge value (MR of its left
             // interface) unless a "pressure" side overwrote it
-            if (cd == 0 && b0 == BC_PRESSURE) gf[e][v][0] = fix(0, v);
+            if (cd == 0 && b0 == BC_PRESSURE) gl[0] = fix(0, v);
             // right edge: the left-edge value of the cell on the right, or
             // the boundary state
             double r;
             if (cd < Nd - 1 || b1 == BC_PERIODIC) {
               const long long nb = (cd < Nd - 1) ? c + step : c - (Nd - 1) * step;
-              double xn[k::n];
+              Line<k::n> ls;
 #pragma unroll
-              for (int s = 0; s < k::n; ++s) xn[s] = sp_val(e, v, s, nb);
-              r = dot_dir<k::n>(op.sp_to_fp, xn, d);
+              for (int s = 0; s < k::n; ++s) ls.v[s] = sp_val(e, v, s, nb);
+              line_ready<k::n>(ls, op.soft);
+              line_apply<k::n, 1, d == 0>(op.c_sp_to_fp, 0, 1, ls, &r);
             } else if (b1 == BC_REFLECTIVE || b1 == BC_GRADFREE) {
-              r = gf[e][v][k::nf - 1];
+              r = gl[k::nf - 1];
               if (b1 == BC_REFLECTIVE && v == d + 1) r = r * -1.0;
             } else {
               r = fix(1, v);
             }
-            gf[e][v][k::nf - 1] = r;
+            gl[k::nf - 1] = r;
+#pragma unroll
+            for (int f = 0; f < k::nf; ++f) gf(e, v, f) = gl[f];
           }
         }
 #pragma unroll
@@ -223,13 +254,13 @@ struct ViscFlux {
           for (int v = 0; v < k::V; ++v)
             W[v] = Wfp[d][((((long long)v * g.T + t) * k::NJ + j) * k::nf + f) * g.Nc + c];
           double F[k::V];
-          F[v1] = 2.0 * gf[d][v1][f] - beta * gf[d][v1][f];
+          F[v1] = 2.0 * gf(d, v1, f) - beta * gf(d, v1, f);
           F[P_] = W[v1] * F[v1];
 #pragma unroll
           for (int kk = 1; kk < D; ++kk) {
             const int vel = rvel<D>(d, kk);
-            F[v1] = F[v1] - beta * gf[vel - 1][vel][f];
-            F[vel] = gf[d][vel][f] + gf[vel - 1][v1][f];
+            F[v1] = F[v1] - beta * gf(vel - 1, vel, f);
+            F[vel] = gf(d, vel, f) + gf(vel - 1, v1, f);
             F[P_] = F[P_] + W[vel] * F[vel];
           }
           F[0] = 0.0;
@@ -238,7 +269,10 @@ struct ViscFlux {
             G[d][((((long long)v * g.T + t) * k::NJ + j) * k::nf + f) * g.Nc + c] = F[v] * W[0] * nu;
         }
       }
-    }
+    };
+    if (dir == 0) line(std::integral_constant<int, 0>());
+    if (D > 1 && dir == 1) line(std::integral_constant<int, (D > 1 ? 1 : 0)>());
+    if (D > 2 && dir == 2) line(std::integral_constant<int, (D > 2 ? 2 : 0)>());
   }
 };
 template <int D, int P>
