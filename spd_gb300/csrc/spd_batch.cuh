@@ -188,6 +188,9 @@ struct BatchRec {
   size_t cursor = 0;
   bool first = true;
   std::string err;
+  // whether all instances use LLF, or all an HLLC form, in the predictor (sd)
+  // and the fallback (fv): then the kernels of that solver are recorded
+  bool one_sd = false, one_fv = false;
 
   void begin_instance(bool is_first) {
     first = is_first;

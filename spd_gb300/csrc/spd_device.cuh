@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "spd_soft.cuh"
 
@@ -142,6 +143,14 @@ SPD_FN double div_rcp(double a, double b, double rb) {
   return div_ieee_slow(a, b);
 }
 
+// c ? a : b by value
+template <class S>
+SPD_FN S sel(bool c, const S& a, const S& b) { return c ? a : b; }
+#ifndef SPD_FUSED
+SPD_FN Num sel(bool c, const Num& a, const Num& b) { return Num(c ? a.v : b.v, c ? a.ok : b.ok); }
+#endif
+SPD_FN double half(double x) { return 0.5 * x; }
+template <int N> SPD_FN Dual<N> half(const Dual<N>& x) { return 0.5 * x; }
 SPD_FN double sval(double x) { return x; }
 template <int N> SPD_FN double sval(const Dual<N>& x) { return x.v; }
 #ifdef SPD_FUSED
@@ -186,6 +195,10 @@ SPD_FN double recip_of(double b) { return 1.0 / b; }
 #else
 template <>
 struct RecipOf<double> {
+  using T = Recip;
+};
+template <>
+struct RecipOf<Num> {
   using T = Recip;
 };
 SPD_FN double div_by(double a, double b, const Recip& rb) { return div_soft(a, b, rb); }
@@ -252,6 +265,13 @@ SPD_FN bool fge(double a, double b) {
   return a >= b;
 #endif
 }
+#ifndef SPD_FUSED
+SPD_FN bool fgt(const Num& a, const Num& b) { return fgt(a.v, b.v); }
+SPD_FN bool fgt(const Num& a, double b) { return fgt(a.v, b); }
+SPD_FN bool fgt(double a, const Num& b) { return fgt(a, b.v); }
+SPD_FN Num np_max(const Num& a, const Num& b) { return Num(np_max(a.v, b.v), a.ok & b.ok); }
+SPD_FN Num np_min(const Num& a, const Num& b) { return Num(np_min(a.v, b.v), a.ok & b.ok); }
+#endif
 template <int N> SPD_FN bool fgt(const Dual<N>& a, const Dual<N>& b) { return a.v > b.v; }
 template <int N> SPD_FN bool fgt(const Dual<N>& a, double b) { return a.v > b; }
 template <int N> SPD_FN bool fgt(double a, const Dual<N>& b) { return a > b.v; }
@@ -334,7 +354,7 @@ SPD_FN void prim(const S* U, S* W, double gamma, int idim_order, typename RecipO
     const S w2 = W[v] * W[v];
     K = (k == 0) ? w2 : K + w2;
   }
-  K = K * (0.5 * U[0]);
+  K = K * half(U[0]);
   if (iso) K = K * 0.0;
   W[P_] = (gamma - 1.0) * (U[P_] - K);
 }
@@ -352,7 +372,7 @@ SPD_FN void cons(const S* W, S* U, double gamma, int idim_order, bool iso = fals
     const S w2 = W[v] * W[v];
     K = (k == 0) ? w2 : K + w2;
   }
-  K = K * (0.5 * W[0]);
+  K = K * half(W[0]);
   if (iso) K = K * 0.0;
   U[P_] = div_by(W[P_], gamma - 1.0, rg ? *rg : recip_of(gamma - 1.0)) + K;
 }
@@ -371,7 +391,7 @@ SPD_FN void flux(const S* W, S* F, double gamma, int idim, bool iso = false, con
     K = (k == D - 1) ? mv : K + mv;
     F[v] = m * W[v1];
   }
-  const S E = div_by(W[P_], gamma - 1.0, rg ? *rg : recip_of(gamma - 1.0)) + 0.5 * K;
+  const S E = div_by(W[P_], gamma - 1.0, rg ? *rg : recip_of(gamma - 1.0)) + half(K);
   F[0] = m;
   F[v1] = m * W[v1] + W[P_];
   F[P_] = W[v1] * (E + W[P_]);
@@ -384,7 +404,7 @@ SPD_FN S sound_speed(const S& P, const S& rho, double gamma, double min_c2,
                                          Br<BM>* br = nullptr,
                                          const typename RecipOf<S>::T* rrho = nullptr) {
   S c2 = div_by(gamma * P, rho, rrho ? *rrho : recip_of(rho));
-  c2 = pick(br, fgt(c2, min_c2)) ? c2 : S(min_c2);
+  c2 = sel(pick(br, fgt(c2, min_c2)), c2, S(min_c2));
   return ad_sqrt(c2);
 }
 
@@ -401,10 +421,10 @@ SPD_FN void llf(const S* WL, const S* WR, const S* UL, const S* UR, S* F, double
   flux<D>(WR, FR, gamma, idim, iso, rg);
   const S cL = sound_speed(WL[P_], WL[0], gamma, min_c2, br, rL) + abs_br(WL[v1], br);
   const S cR = sound_speed(WR[P_], WR[0], gamma, min_c2, br, rR) + abs_br(WR[v1], br);
-  const S cmax = pick(br, fgt(cL, cR)) ? cL : cR;
-  const S hc = 0.5 * cmax;
+  const S cmax = sel(pick(br, fgt(cL, cR)), cL, cR);
+  const S hc = half(cmax);
 #pragma unroll
-  for (int v = 0; v < V; ++v) F[v] = 0.5 * (FR[v] + FL[v]) - hc * (UR[v] - UL[v]);
+  for (int v = 0; v < V; ++v) F[v] = half(FR[v] + FL[v]) - hc * (UR[v] - UL[v]);
 }
 
 // HLLC (src/riemann_solver.py:67-145) and its low-Mach variant (:147-212).
@@ -417,10 +437,10 @@ SPD_FN void hllc(const S* WL, const S* WR, const S* UL, const S* UR, S* F, doubl
   const int v1 = rvel<D>(idim, 0);
   const S cL = sound_speed(WL[P_], WL[0], gamma, min_c2, br, rL) + abs_br(WL[v1], br);
   const S cR = sound_speed(WR[P_], WR[0], gamma, min_c2, br, rR) + abs_br(WR[v1], br);
-  const S cmax = pick(br, fgt(cL, cR)) ? cL : cR;
+  const S cmax = sel(pick(br, fgt(cL, cR)), cL, cR);
   const S vL = WL[v1], vR = WR[v1];
-  const S sL = (pick(br, fgt(vR, vL)) ? vL : vR) - cmax;
-  const S sR = (pick(br, fgt(vL, vR)) ? vL : vR) + cmax;
+  const S sL = sel(pick(br, fgt(vR, vL)), vL, vR) - cmax;
+  const S sR = sel(pick(br, fgt(vL, vR)), vL, vR) + cmax;
   const S rcL = WL[0] * (vL - sL);
   const S rcR = WR[0] * (sR - vR);
   const S den = rcR + rcL;
@@ -429,7 +449,7 @@ SPD_FN void hllc(const S* WL, const S* WR, const S* UL, const S* UR, S* F, doubl
   S Pstar;
   if (low_mach) {
     S mx, Mach;
-    if (BM == 0) {
+    if constexpr (BM == 0) {
       mx = np_max(ad_abs(vL), ad_abs(vR)) / cmax;
       Mach = np_min(S(1.0), mx);
     } else {
@@ -452,8 +472,8 @@ SPD_FN void hllc(const S* WL, const S* WR, const S* UL, const S* UR, S* F, doubl
       r = WL[0]; vg = vL; Pg = WL[P_]; e = UL[P_];
     } else if (fgt(vstar, 0.0) || fgt(sR, 0.0)) {
       const bool lft = fgt(vstar, 0.0);
-      const S s = lft ? sL : sR, v = lft ? vL : vR;
-      const S w0 = lft ? WL[0] : WR[0], wP = lft ? WL[P_] : WR[P_], uP = lft ? UL[P_] : UR[P_];
+      const S s = sel(lft, sL, sR), v = sel(lft, vL, vR);
+      const S w0 = sel(lft, WL[0], WR[0]), wP = sel(lft, WL[P_], WR[P_]), uP = sel(lft, UL[P_], UR[P_]);
       const S d = s - vstar;
       const auto rd = recip_of(d);
       r = div_by(w0 * (s - v), d, rd);
@@ -487,18 +507,38 @@ SPD_FN void hllc(const S* WL, const S* WR, const S* UL, const S* UR, S* F, doubl
 #pragma unroll
     for (int k = 1; k < D; ++k) {
       const int v = rvel<D>(idim, k);
-      F[v] = F[0] * (left ? WL[v] : WR[v]);
+      F[v] = F[0] * sel(left, WL[v], WR[v]);
     }
   }
   if (iso) F[P_] = F[P_] * 0.0;
 }
 
+// the solver of a kernel instantiated for SV
+template <int SV>
+SPD_FN int solver_of(int solver) {
+  if (SV == RS_LLF) return RS_LLF;
+  if (SV == RS_HLLC) return solver == RS_LHLLC ? RS_LHLLC : RS_HLLC;
+  return solver;
+}
+#ifndef SPD_FUSED
+// LLF in plain FP64 arithmetic, out of line
+template <int D>
+#ifdef __CUDA_ARCH__
+__device__ __noinline__
+#else
+inline
+#endif
+    void
+    llf_plain(const double* WL, const double* WR, const double* UL, const double* UR, double* F, double gamma,
+              double min_c2, int idim, bool iso) {
+  llf<D, double>(WL, WR, UL, UR, F, gamma, min_c2, idim, (Br<0>*)nullptr, nullptr, nullptr, iso);
+}
+#endif
 // Riemann wrapper (src/riemann_solver.py:10-29): inputs conservative
 // (prims=false) or primitive (prims=true); rotated velocity order.
 template <int D, class S, int BM = 0>
-SPD_FN void riemann(int solver, const S* ML, const S* MR, S* F, double gamma, double min_c2,
-                                        int idim, bool prims, Br<BM>* br = nullptr, bool iso = false,
-                                        const Rcp* rg = nullptr) {
+SPD_FN void riemann(int solver, const S* ML, const S* MR, S* F, double gamma, double min_c2, int idim, bool prims,
+                       Br<BM>* br = nullptr, bool iso = false, const Rcp* rg = nullptr) {
   constexpr int V = D + 2;
   S WL[V], WR[V], UL[V], UR[V];
   typename RecipOf<S>::T rL, rR;  // 1/rho of the two states when the conversion computed it
@@ -517,8 +557,162 @@ SPD_FN void riemann(int solver, const S* ML, const S* MR, S* F, double gamma, do
     prL = &rL;
     prR = &rR;
   }
+#ifndef SPD_FUSED
+  if constexpr (BM == 0 && D <= 2 && std::is_same<S, double>::value) {
+    // (1D, 2D) LLF's products on the integer pipes, the conversions' on the FP64 pipe:
+    // an even split of the two (251x190, p=3: 1.40 -> 1.15 ms; all on the
+    // integer pipes 1.19).  HLLC, whose products hang on one another, keeps
+    // the FP64 pipe (512^2: 2.81 ms, 3.14 with integer products, 3.32 with
+    // those of the conversions too).  A problem with a value out of their
+    // range is solved again in plain FP64 arithmetic.
+    if (solver == RS_LLF) {
+      Num wl[V], wr[V], ul[V], ur[V], f[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        wl[v] = Num(WL[v]);
+        wr[v] = Num(WR[v]);
+        ul[v] = Num(UL[v]);
+        ur[v] = Num(UR[v]);
+      }
+      llf<D, Num>(wl, wr, ul, ur, f, gamma, min_c2, idim, (Br<0>*)nullptr, prL, prR, iso, rg);
+      uint32_t ok = 0x40000000u;
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        ok &= f[v].ok;
+        F[v] = f[v].v;
+      }
+      if (ok != 0u) return;
+      double a[V], b[V], c[V], e[V], o[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        a[v] = WL[v];
+        b[v] = WR[v];
+        c[v] = UL[v];
+        e[v] = UR[v];
+      }
+      llf_plain<D>(a, b, c, e, o, gamma, min_c2, idim, iso);
+#pragma unroll
+      for (int v = 0; v < V; ++v) F[v] = o[v];
+      return;
+    }
+  }
+#endif
   if (solver == RS_LLF) llf<D, S, BM>(WL, WR, UL, UR, F, gamma, min_c2, idim, br, prL, prR, iso, rg);
   else hllc<D, S, BM>(WL, WR, UL, UR, F, gamma, min_c2, idim, solver == RS_LHLLC, br, prL, prR, iso);
+}
+
+// U -> W (plain velocity order) and the Euler flux along direction d in the
+// rotated frame, in 1D and 2D with their products on the integer pipes as
+// above: k_interior 11.2 -> 10.6 ms and k_fv_candidate 1.22 -> 1.14 ms at
+// 512^2, p=3.  In 3D the integer pipes are the busier ones already (48^3,
+// p=2: 7.45 -> 7.87 and 1.2 -> 1.31 ms), so their products stay FP64.
+template <int D>
+constexpr bool num_euler() {
+#if defined(__CUDA_ARCH__) && !defined(SPD_FUSED)
+  return D <= 2;
+#else
+  return false;
+#endif
+}
+#if defined(__CUDA_ARCH__) && !defined(SPD_FUSED)
+template <int D>
+__device__ __noinline__ void euler_slow(const double* U, double* W, double* F, double gamma, int d, bool iso) {
+  prim<D>(U, W, gamma, 0, nullptr, iso);
+  if (F == nullptr) return;
+  double Wr[D + 2], Fr[D + 2];
+  Wr[0] = W[0];
+  Wr[D + 1] = W[D + 1];
+#pragma unroll
+  for (int q = 0; q < D; ++q) Wr[1 + q] = W[rvel<D>(d, q)];
+  flux<D>(Wr, Fr, gamma, 0, iso);
+  F[0] = Fr[0];
+  F[D + 1] = Fr[D + 1];
+#pragma unroll
+  for (int q = 0; q < D; ++q) F[rvel<D>(d, q)] = Fr[1 + q];
+}
+#endif
+template <int D>
+SPD_FN void prims(const double* U, double* W, double gamma, bool iso) {
+  constexpr int V = D + 2;
+#if defined(__CUDA_ARCH__) && !defined(SPD_FUSED)
+  if constexpr (num_euler<D>()) {
+    Num u[V], w[V];
+    uint32_t ok = 0x40000000u;
+#pragma unroll
+    for (int v = 0; v < V; ++v) u[v] = Num(U[v]);
+    prim<D>(u, w, gamma, 0, nullptr, iso);
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      ok &= w[v].ok;
+      W[v] = w[v].v;
+    }
+    if (ok != 0u) return;
+    double us[V], ws[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) us[v] = U[v];
+    euler_slow<D>(us, ws, nullptr, gamma, 0, iso);
+#pragma unroll
+    for (int v = 0; v < V; ++v) W[v] = ws[v];
+    return;
+  }
+#endif
+  prim<D>(U, W, gamma, 0, nullptr, iso);
+}
+// flux of the conservative state U; store(v, F_v) takes its components
+template <int D, class Store>
+SPD_FN void euler_flux(const double* U, double gamma, int d, bool iso, const Rcp* rg, Store store) {
+  constexpr int V = D + 2;
+#if defined(__CUDA_ARCH__) && !defined(SPD_FUSED)
+  using S = typename std::conditional<num_euler<D>(), Num, double>::type;
+#else
+  using S = double;
+#endif
+  // the velocities in the rotated order of direction d, as flux's own order
+  // for direction 0
+  S u[V], w[V], wr[V], f[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) u[v] = S(U[v]);
+  prim<D>(u, w, gamma, 0, nullptr, iso);
+  wr[0] = w[0];
+  wr[D + 1] = w[D + 1];
+#pragma unroll
+  for (int q = 0; q < D; ++q) {
+    S x = w[1 + q];
+    if (D > 1) x = sel(d == 1, w[1 + (q + 1) % D], x);
+    if (D > 2) x = sel(d == 2, w[1 + (q + 2) % D], x);
+    wr[1 + q] = x;
+  }
+  flux<D>(wr, f, gamma, 0, iso, rg);
+#if defined(__CUDA_ARCH__) && !defined(SPD_FUSED)
+  if constexpr (num_euler<D>()) {
+    uint32_t ok = 0x40000000u;
+#pragma unroll
+    for (int v = 0; v < V; ++v) ok &= f[v].ok;
+    double fs[V];
+    if (ok != 0u) {
+#pragma unroll
+      for (int v = 0; v < V; ++v) fs[v] = f[v].v;
+    } else {
+      double us[V], ws[V], fl[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) us[v] = U[v];
+      euler_slow<D>(us, ws, fl, gamma, d, iso);
+      fs[0] = fl[0];
+      fs[D + 1] = fl[D + 1];
+#pragma unroll
+      for (int q = 0; q < D; ++q) fs[1 + q] = fl[rvel<D>(d, q)];
+    }
+    store(0, fs[0]);
+    store(D + 1, fs[D + 1]);
+#pragma unroll
+    for (int q = 0; q < D; ++q) store(rvel<D>(d, q), fs[1 + q]);
+    return;
+  }
+#endif
+  store(0, sval(f[0]));
+  store(D + 1, sval(f[D + 1]));
+#pragma unroll
+  for (int q = 0; q < D; ++q) store(rvel<D>(d, q), sval(f[1 + q]));
 }
 
 // One output of a 1D operator contraction: sum_s A[s] * x[s].  ``lanes2``

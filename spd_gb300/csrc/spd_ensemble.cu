@@ -197,6 +197,12 @@ int spd_ensemble_create_packed(spd_ctx** ctxs, int n, int steps_per_launch, spd_
   // i-th launch of every instance into one batched launch
   E->packed.reset(new spd_batch::BatchRec());
   spd_batch::BatchRec* R = E->packed.get();
+  R->one_sd = R->one_fv = true;
+  for (const spd_ctx* C : E->ctx) {
+    const spd_config &a = C->cfg, &b = E->ctx[0]->cfg;
+    R->one_sd = R->one_sd && (a.riemann_solver_sd == RS_LLF) == (b.riemann_solver_sd == RS_LLF);
+    R->one_fv = R->one_fv && (a.riemann_solver_fv == RS_LLF) == (b.riemann_solver_fv == RS_LLF);
+  }
   const RolesGuard roles_before(E->ctx);
   for (int i = 0; i < n && R->err.empty(); ++i) {
     spd_ctx* C = E->ctx[i];

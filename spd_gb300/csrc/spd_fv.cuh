@@ -85,13 +85,13 @@ __device__ __forceinline__ void prims_cv(const Geo& g, const double* u, double* 
                                          const double* __restrict__ Weq, long long q) {
   constexpr int V = D + 2;
   if (Ueq == nullptr) {
-    prim<D>(u, W, g.gamma, 0, nullptr, g.iso != 0);
+    prims<D>(u, W, g.gamma, g.iso != 0);
     return;
   }
   double uf[V];
 #pragma unroll
   for (int v = 0; v < V; ++v) uf[v] = u[v] + Ueq[(long long)v * g.Nq + q];
-  prim<D>(uf, W, g.gamma, 0, nullptr, g.iso != 0);
+  prims<D>(uf, W, g.gamma, g.iso != 0);
 #pragma unroll
   for (int v = 0; v < V; ++v) W[v] = W[v] - Weq[(long long)v * g.Nq + q];
 }
@@ -795,11 +795,14 @@ __global__ void k_muscl_cells(Geo g, FvGeo fg, int limiter, const double* __rest
 
 // fallback Riemann flux on the affected faces of direction d
 // (src/muscl.py:217-221, src/fv_simulator.py:88-165)
-template <int D, int BM = 0>
+// DIR >= 0 fixes the direction at compile time (the rotated velocity indices
+// become constants: with a runtime direction the states are indexed in local
+// memory); DIR = -1 takes it from d_rt.  SV as in RiemannSd.
+template <int D, int BM = 0, int DIR = -1, int SV = -1>
 struct MusclFaces {
 // the affected faces of direction d from their compacted list (k_affected),
 // a grid-stride loop over full warps
-static __device__ __forceinline__ void run(Blk B, const Geo& g, int d, int solver,
+static __device__ __forceinline__ void run(Blk B, const Geo& g, int d_rt, int solver,
                                            const long long* __restrict__ flist,
                                            const unsigned long long* __restrict__ fcount,
                                            const double* __restrict__ Mpred, const double* __restrict__ S,
@@ -808,7 +811,7 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, int d, int solve
   const unsigned long long cnt = *fcount;
   for (unsigned long long idx = B.id * (unsigned long long)blockDim.x + threadIdx.x; idx < cnt;
        idx += (unsigned long long)B.n * blockDim.x)
-    face(g, d, solver, flist[idx], Mpred, S, F_FB, ftape, Mq, Fq);
+    face(g, DIR >= 0 ? DIR : d_rt, solver, flist[idx], Mpred, S, F_FB, ftape, Mq, Fq);
 }
 // Mq, Fq (well-balanced mode): the equilibrium's primitive state and flux
 // at the faces, added to both states and subtracted from the flux
@@ -843,18 +846,18 @@ static __device__ __forceinline__ void face(const Geo& g, int d, int solver, lon
   }
   Br<BM> br;
   if (BM == 2) br.w = ftape[fidx];
-  riemann<D, double, BM>(solver, ML, MR, F, g.gamma, g.min_c2, d, true, &br, g.iso != 0, &g.rgm1);
+  riemann<D, double, BM>(solver_of<SV>(solver), ML, MR, F, g.gamma, g.min_c2, d, true, &br, g.iso != 0, &g.rgm1);
   if (BM == 1) ftape[fidx] = br.w;
 #pragma unroll
   for (int v = 0; v < V; ++v) F_FB[(long long)v * nf + fidx] = Fq ? F[v] - Fq[(long long)v * nf + fidx] : F[v];
 }
 };
-template <int D, int BM = 0>
+template <int D, int BM = 0, int DIR = -1, int SV = -1>
 __global__ void k_muscl_faces(Geo g, int d, int solver, const long long* __restrict__ flist,
                               const unsigned long long* __restrict__ fcount, const double* __restrict__ Mpred,
                               const double* __restrict__ S, double* __restrict__ F_FB, unsigned* ftape,
                               const double* __restrict__ Mq, const double* __restrict__ Fq) {
-  MusclFaces<D, BM>::run(hw_blk(), g, d, solver, flist, fcount, Mpred, S, F_FB, ftape, Mq, Fq);
+  MusclFaces<D, BM, DIR, SV>::run(hw_blk(), g, d, solver, flist, fcount, Mpred, S, F_FB, ftape, Mq, Fq);
 }
 
 // corrected update of the subcells next to an affected face
@@ -964,7 +967,7 @@ struct WbEnd {
       u[v] = U_cv[(long long)v * g.Nq + q] + Ueq[(long long)v * g.Nq + q];
       U_cv[(long long)v * g.Nq + q] = u[v];
     }
-    prim<D>(u, W, g.gamma, 0, nullptr, g.iso != 0);
+    prims<D>(u, W, g.gamma, g.iso != 0);
 #pragma unroll
     for (int v = 0; v < V; ++v) W_cv[(long long)v * g.Nq + q] = W[v];
   }

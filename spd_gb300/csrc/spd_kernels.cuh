@@ -163,8 +163,10 @@ __global__ void k_traces_ader(Ops op, Geo g, const double* __restrict__ U, int T
 // (src/sdader_simulator.py:225-234, src/sd_boundary.py:7-76)
 // ---------------------------------------------------------------------------
 // DIR >= 0 fixes the direction at compile time (the rotated velocity
-// indices become constants); DIR = -1 takes it from d_rt.
-template <int D, int P, int BM = 0, int DIR = -1, bool EQ = false>
+// indices become constants); DIR = -1 takes it from d_rt.  SV: RS_LLF, RS_HLLC
+// (either HLLC form, by ``solver``) or -1 (any): one solver per kernel keeps
+// its registers its own.
+template <int D, int P, int BM = 0, int DIR = -1, bool EQ = false, int SV = -1>
 struct RiemannSd {
 static __device__ __forceinline__ void run(Blk B, const Geo& g, int d_rt, int Teff, int solver,
                                            const double* __restrict__ trace, const double* __restrict__ bcfix,
@@ -260,7 +262,7 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, int d_rt, int Te
   if (BM == 2) br.w = tape[tid];
   // the isothermal system only in the EQ form: a runtime flag costs the
   // plain form an FP64 multiply per flux (the compiler predicates it)
-  riemann<D, double, BM>(solver, ML, MR, F, g.gamma, g.min_c2, d, false, &br, EQ && g.iso != 0,
+  riemann<D, double, BM>(solver_of<SV>(solver), ML, MR, F, g.gamma, g.min_c2, d, false, &br, EQ && g.iso != 0,
                          &g.rgm1);
   if (BM == 1) tape[tid] = br.w;
 #pragma unroll
@@ -270,11 +272,11 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, int d_rt, int Te
 // EQ: the form for the well-balanced mode (meq non-null: the equilibrium
 // at the flux points added to every edge state) and the isothermal system;
 // the plain form reads neither
-template <int D, int P, int BM = 0, int DIR = -1, bool EQ = false>
+template <int D, int P, int BM = 0, int DIR = -1, bool EQ = false, int SV = -1>
 __global__ void k_riemann_sd(Geo g, int d_rt, int Teff, int solver, const double* __restrict__ trace,
                              const double* __restrict__ bcfix, double* __restrict__ Fi, unsigned* tape,
                              const double* __restrict__ meq) {
-  RiemannSd<D, P, BM, DIR, EQ>::run(hw_blk(), g, d_rt, Teff, solver, trace, bcfix, Fi, tape, meq);
+  RiemannSd<D, P, BM, DIR, EQ, SV>::run(hw_blk(), g, d_rt, Teff, solver, trace, bcfix, Fi, tape, meq);
 }
 
 // ---------------------------------------------------------------------------
@@ -349,30 +351,14 @@ static __device__ __forceinline__ void lines(const Ops& op, const Geo& g, const 
     }
 #pragma unroll
     for (int f = 0; f < ni; ++f) {
-      double M[k::V], W[k::V], Wr[k::V], F[k::V];
+      double M[k::V];
 #pragma unroll
       for (int v = 0; v < k::V; ++v) M[v] = scr[(v * ni + f) * NT];
       if (a.wb) {
 #pragma unroll
         for (int v = 0; v < k::V; ++v) M[v] = M[v] + meq[(((long long)v * k::NJ + j) * k::nf + f + 1) * g.Nc + c];
       }
-      prim<D>(M, W, g.gamma, 0, nullptr, a.iso);
-      // the velocities in the rotated order of direction d, as flux's own
-      // order for direction 0
-      Wr[0] = W[0];
-      Wr[D + 1] = W[D + 1];
-#pragma unroll
-      for (int q = 0; q < D; ++q) {
-        double w = W[1 + q];
-        if (D > 1) w = (d == 1) ? W[1 + (q + 1) % D] : w;
-        if (D > 2) w = (d == 2) ? W[1 + (q + 2) % D] : w;
-        Wr[1 + q] = w;
-      }
-      flux<D>(Wr, F, g.gamma, 0, a.iso, &g.rgm1);
-      scr[f * NT] = F[0];
-      scr[((D + 1) * ni + f) * NT] = F[D + 1];
-#pragma unroll
-      for (int q = 0; q < D; ++q) scr[(rvel<D>(d, q) * ni + f) * NT] = F[1 + q];
+      euler_flux<D>(M, g.gamma, d, a.iso, &g.rgm1, [&](int v, double F) { scr[(v * ni + f) * NT] = F; });
     }
     const bool pow2 = g.h_pow2[d] != 0;
 #pragma unroll 1

@@ -185,11 +185,10 @@ SPD_FN Prod soft_words(uint32_t cl, uint32_t ch, uint32_t e, const Opnd& x) {
   return o;
 }
 
-// RN(c * x).  Rounding adds 2^63 - 1 (2^63 when the result is odd) to words
+// The product rounded: adds 2^63 - 1 (2^63 when the result is odd) to words
 // 1:0; the carry into the exponent field is the rounding up to the next power
 // of two.
-SPD_FN double soft_prod(const Coef& c, const Opnd& x) {
-  Prod o = soft_words(c.ml, c.mh, c.e + x.e, x);
+SPD_FN double soft_round(Prod o, uint32_t keep) {
   const uint32_t t = o.p0 | (o.w2 & 1u);
 #ifdef __CUDA_ARCH__
   asm("{\n\t"
@@ -209,7 +208,10 @@ SPD_FN double soft_prod(const Coef& c, const Opnd& x) {
     o.w3 += o.e + (uint32_t)(u >> 32);
   }
 #endif
-  return from_words(o.w3 & x.keep, o.w2);
+  return from_words(o.w3 & keep, o.w2);
+}
+SPD_FN double soft_prod(const Coef& c, const Opnd& x) {
+  return soft_round(soft_words(c.ml, c.mh, c.e + x.e, x), x.keep);
 }
 
 // A divisor b prepared for several quotients: 2^63 over its significand,
@@ -278,10 +280,7 @@ SPD_FN Recip recip_soft(double b) {
 // b decides the last place.  A quotient of two 53-bit numbers is never a tie.
 // a: a zero or within opnd_of's window; any other pair is divided by the
 // FP64 unit.
-SPD_FN double div_soft(double a, double b, const Recip& rb) {
-  uint32_t ok = rb.ok;
-  const Opnd x = opnd_of(a, ok);
-  if (ok == 0u) return div_ieee_slow(a, b);
+SPD_FN double div_words(const Opnd& x, double b, const Recip& rb) {
   const Prod o = soft_words(rb.ml, rb.mh, rb.e + x.e, x);
   const uint32_t bl = lo_word(b), bh = (hi_word(b) & 0xfffffu) | 0x100000u;
   // b + 2 (b q - a 2^s), negative where the remainder exceeds b/2; a 2^s has
@@ -292,6 +291,12 @@ SPD_FN double div_soft(double a, double b, const Recip& rb) {
   const unsigned long long t = (((unsigned long long)bh << 32) | bl) + (p << 1) - ((unsigned long long)a2 << 32);
   const unsigned long long q = (((unsigned long long)(o.w3 + o.e) << 32) | o.w2) + (t >> 63);
   return from_words((uint32_t)(q >> 32) & x.keep, (uint32_t)q);
+}
+
+SPD_FN double div_soft(double a, double b, const Recip& rb) {
+  uint32_t ok = rb.ok;
+  const Opnd x = opnd_of(a, ok);
+  return ok != 0u ? div_words(x, b, rb) : div_ieee_slow(a, b);
 }
 
 // sqrt(x) rounded to nearest.  With x = m 4^k, m in [1, 4): the FP32
@@ -350,6 +355,49 @@ SPD_FN double sqrt_soft(double x) {
   const unsigned long long out = (((unsigned long long)(qh + eo) << 32) | ql) + ((q - rem) >> 63);
   return from_words((uint32_t)(out >> 32), (uint32_t)out);
 }
+
+// A double with its prepared operand, for expressions whose products all run
+// on the integer pipes (sums stay on the FP64 pipe).  ``ok`` (bit 30): the
+// value and every value it came from are zeros or within opnd_of's window.
+// A product of two such values is at least 2^-1022; one above the largest
+// double carries into the sign bit and leaves an exponent field below 8, so
+// it fails the window itself.  A result without ``ok`` is computed again in
+// plain FP64 arithmetic.  Unused preparations are dead code.
+struct Num {
+  double v;
+  Opnd o;
+  uint32_t ok;
+  SPD_FN Num() {}
+  SPD_FN Num(double x, uint32_t from = 0x40000000u) : v(x) {
+    ok = from;
+    o = opnd_of(x, ok);
+  }
+};
+SPD_FN Num operator+(const Num& a, const Num& b) { return Num(a.v + b.v, a.ok & b.ok); }
+SPD_FN Num operator-(const Num& a, const Num& b) { return Num(a.v - b.v, a.ok & b.ok); }
+SPD_FN Num operator-(const Num& a) { return Num(from_words(hi_word(a.v) ^ 0x80000000u, lo_word(a.v)), a.ok); }
+SPD_FN Num operator*(const Num& a, const Num& b) {
+  const uint32_t ch = (a.o.mh << 9) | (a.o.ml >> 23);
+  return Num(soft_round(soft_words(a.o.ml << 9, ch, a.o.e + b.o.e - (1023u << 20), b.o), a.o.keep & b.o.keep),
+             a.ok & b.ok);
+}
+SPD_FN Num operator+(const Num& a, double b) { return a + Num(b); }
+SPD_FN Num operator-(const Num& a, double b) { return a - Num(b); }
+SPD_FN Num operator-(double a, const Num& b) { return Num(a) - b; }
+SPD_FN Num operator*(const Num& a, double b) { return a * Num(b); }
+SPD_FN Num operator*(double a, const Num& b) { return Num(a) * b; }
+SPD_FN Num div_by(const Num& a, const Num& b, const Recip& rb) { return Num(div_words(a.o, b.v, rb), a.ok & b.ok & rb.ok); }
+SPD_FN Num div_by(const Num& a, double b, const Recip& rb) { return Num(div_words(a.o, b, rb), a.ok & rb.ok); }
+SPD_FN Recip recip_of(const Num& b) { return recip_soft(b.v); }
+SPD_FN Num operator/(const Num& a, const Num& b) { return div_by(a, b, recip_of(b)); }
+// x / 2: one less in the exponent
+SPD_FN Num half(const Num& a) {
+  const uint32_t h = hi_word(a.v);
+  return Num(from_words(a.o.keep == 0x80000000u ? h : h - 0x100000u, lo_word(a.v)), a.ok);
+}
+SPD_FN Num ad_sqrt(const Num& a) { return Num(sqrt_soft(a.v), a.ok); }
+SPD_FN Num ad_abs(const Num& a) { return Num(from_words(hi_word(a.v) & 0x7fffffffu, lo_word(a.v)), a.ok); }
+SPD_FN double sval(const Num& a) { return a.v; }
 #endif  // SPD_FUSED
 
 }  // namespace spd

@@ -51,7 +51,7 @@ struct PrimOnly {
     double u[V], W[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) u[v] = U_cv[(long long)v * g.Nq + q];
-    prim<D>(u, W, g.gamma, 0, nullptr, g.iso != 0);
+    prims<D>(u, W, g.gamma, g.iso != 0);
 #pragma unroll
     for (int v = 0; v < V; ++v) W_cv[(long long)v * g.Nq + q] = W[v];
   }
@@ -129,21 +129,19 @@ struct Stepper : StepperBase {
   // the Riemann problems of one Picard iteration, one instantiation per
   // direction; EQ: the form with the well-balanced mode's equilibrium edge
   // values and the isothermal system
-  template <bool EQ>
-  void riemann_plain(spd_ctx* C, int d, unsigned nb, int Teff, int solver) {
-    const Geo& g = C->geo;
-    constexpr int D1 = (D > 1 ? 1 : 0), D2 = (D > 2 ? 2 : 0);
+  template <bool EQ, int DIR, int SV>
+  void riemann_dir(spd_ctx* C, unsigned nb, int Teff, int solver) {
     unsigned* no_tape = nullptr;
-    const double* meq = C->Meq_fp[d];
-    if (d == 0)
-      launch<RiemannSd<D, P, 0, 0, EQ>>(C, "k_riemann_sd", k_riemann_sd<D, P, 0, 0, EQ>, nb, 128, 0, g, d, Teff,
-                                        solver, C->trace[d], C->bcfix[d], C->Fi[d], no_tape, meq);
-    else if (d == 1)
-      launch<RiemannSd<D, P, 0, D1, EQ>>(C, "k_riemann_sd", k_riemann_sd<D, P, 0, D1, EQ>, nb, 128, 0, g, d, Teff,
-                                         solver, C->trace[d], C->bcfix[d], C->Fi[d], no_tape, meq);
-    else
-      launch<RiemannSd<D, P, 0, D2, EQ>>(C, "k_riemann_sd", k_riemann_sd<D, P, 0, D2, EQ>, nb, 128, 0, g, d, Teff,
-                                         solver, C->trace[d], C->bcfix[d], C->Fi[d], no_tape, meq);
+    const double* meq = C->Meq_fp[DIR];
+    launch<RiemannSd<D, P, 0, DIR, EQ, SV>>(C, "k_riemann_sd", k_riemann_sd<D, P, 0, DIR, EQ, SV>, nb, 128, 0, C->geo,
+                                            DIR, Teff, solver, C->trace[DIR], C->bcfix[DIR], C->Fi[DIR], no_tape,
+                                            meq);
+  }
+  template <bool EQ, int SV>
+  void riemann_plain(spd_ctx* C, int d, unsigned nb, int Teff, int solver) {
+    if (d == 0) riemann_dir<EQ, 0, SV>(C, nb, Teff, solver);
+    else if (d == 1) riemann_dir<EQ, (D > 1 ? 1 : 0), SV>(C, nb, Teff, solver);
+    else riemann_dir<EQ, (D > 2 ? 2 : 0), SV>(C, nb, Teff, solver);
   }
 
   // the Riemann problems of one Picard iteration with every branch taped
@@ -187,10 +185,10 @@ struct Stepper : StepperBase {
           ProfScope ps_(C, "k_riemann_sd");
           if (C->tape_mode == 0) {
             const unsigned nb = blocks_for(tot, 128);
-            if (C->Meq_fp[d] || C->cfg.isothermal)
-              riemann_plain<true>(C, d, nb, Teff, solver);
-            else
-              riemann_plain<false>(C, d, nb, Teff, solver);
+            if (C->Meq_fp[d] || C->cfg.isothermal) riemann_plain<true, -1>(C, d, nb, Teff, solver);
+            else if (C->brec && !C->brec->one_sd) riemann_plain<false, -1>(C, d, nb, Teff, solver);
+            else if (solver == RS_LLF) riemann_plain<false, RS_LLF>(C, d, nb, Teff, solver);
+            else riemann_plain<false, RS_HLLC>(C, d, nb, Teff, solver);
           } else {
             unsigned* tp = C->tape_rs[d] + ((size_t)C->tape_step * C->T + it) * C->T * k::NJ * n_iface(g, d);
             if (C->tape_mode == 1)
@@ -453,10 +451,20 @@ struct Stepper : StepperBase {
             const unsigned nb = (unsigned)std::min<long long>(PERSIST_BLOCKS, blocks_for(nface[d], BS));
             const unsigned long long* fcount = C->counts + 4 + d;
             if (C->tape_mode == 0) {
-              unsigned* no_tape = nullptr;
-              launch<MusclFaces<D>>(C, "k_muscl_faces", k_muscl_faces<D>, nb, BS, 0, g, d, cf.riemann_solver_fv,
-                                    C->list_face[d], fcount, C->Mpred, C->S, C->F_FB[d], no_tape,
-                                    (const double*)C->Meq_faces[d], (const double*)C->Feq_faces[d]);
+              constexpr int D1 = (D > 1 ? 1 : 0), D2 = (D > 2 ? 2 : 0);
+              if (C->brec && !C->brec->one_fv) {
+                if (d == 0) muscl_faces<0, -1>(C, nb, fcount);
+                else if (d == 1) muscl_faces<D1, -1>(C, nb, fcount);
+                else muscl_faces<D2, -1>(C, nb, fcount);
+              } else if (cf.riemann_solver_fv == RS_LLF) {
+                if (d == 0) muscl_faces<0, RS_LLF>(C, nb, fcount);
+                else if (d == 1) muscl_faces<D1, RS_LLF>(C, nb, fcount);
+                else muscl_faces<D2, RS_LLF>(C, nb, fcount);
+              } else {
+                if (d == 0) muscl_faces<0, RS_HLLC>(C, nb, fcount);
+                else if (d == 1) muscl_faces<D1, RS_HLLC>(C, nb, fcount);
+                else muscl_faces<D2, RS_HLLC>(C, nb, fcount);
+              }
             } else {
               unsigned* tp = C->tape_fb[d] + ((size_t)C->tape_step * C->T + i) * nface[d];
               if (C->tape_mode == 1)
@@ -493,6 +501,14 @@ struct Stepper : StepperBase {
     }
     CKL();
     return 0;
+  }
+
+  template <int DIR, int SV>
+  void muscl_faces(spd_ctx* C, unsigned nb, const unsigned long long* fcount) {
+    unsigned* no_tape = nullptr;
+    launch<MusclFaces<D, 0, DIR, SV>>(C, "k_muscl_faces", k_muscl_faces<D, 0, DIR, SV>, nb, BS, 0, C->geo, DIR,
+                                  C->cfg.riemann_solver_fv, C->list_face[DIR], fcount, C->Mpred, C->S, C->F_FB[DIR],
+                                  no_tape, (const double*)C->Meq_faces[DIR], (const double*)C->Feq_faces[DIR]);
   }
 
   void k_muscl_cells_grid(spd_ctx* C, double w_i, int i) {

@@ -100,7 +100,7 @@ struct ViscGrad {
             M[v] = Wf(v, f);
             if (meq[0]) M[v] = M[v] + meq[d][(((long long)v * k::NJ + j) * k::nf + f) * g.Nc + c];
           }
-          prim<D>(M, W, g.gamma, 0, nullptr, g.iso != 0);
+          prims<D>(M, W, g.gamma, g.iso != 0);
 #pragma unroll
           for (int v = 0; v < k::V; ++v) Wf(v, f) = W[v];
         }
@@ -114,7 +114,7 @@ struct ViscGrad {
           } else {
 #pragma unroll
             for (int v = 0; v < k::V; ++v) M[v] = tr(1, v, c);
-            prim<D>(M, W, g.gamma, 0, nullptr, g.iso != 0);
+            prims<D>(M, W, g.gamma, g.iso != 0);
           }
 #pragma unroll
           for (int v = 0; v < k::V; ++v) Wf(v, k::nf - 1) = W[v];
@@ -128,7 +128,7 @@ struct ViscGrad {
             const int side = (cd > 0 || b0 == BC_PERIODIC) ? 1 : 0;
 #pragma unroll
             for (int v = 0; v < k::V; ++v) M[v] = tr(side, v, src);
-            prim<D>(M, W, g.gamma, 0, nullptr, g.iso != 0);
+            prims<D>(M, W, g.gamma, g.iso != 0);
             if (cd == 0 && b0 == BC_REFLECTIVE) W[d + 1] = W[d + 1] * -1.0;
           } else {
 #pragma unroll
