@@ -110,8 +110,7 @@ int adjoint_vjp(spd_ctx* C) {
           const int o1 = (d == 2) ? 1 : 2;
           const long long tot = 2LL * k::V * NGH * g.Xe[o0] * g.Xe[o1];
           ProfScope ps_(C, "k_ghost");
-          k_ghost<D><<<blocks_for(tot, BS), BS, 0, C->stream>>>(g, d, 1, k::V, k::V, C->W_ext, C->bcbuf_a[d],
-                                                                nullptr);
+          k_ghost<D><<<blocks_for(tot, BS), BS, 0, C->stream>>>(g, d, k::V, C->W_ext, C->bcbuf_a[d]);
           CKL();
         }
         // the used faces and the cells bordering them, compacted into the

@@ -335,6 +335,8 @@ int spd_create(const spd_config* cfg, const spd_operators* ops, spd_ctx** out) {
   if (int r = dalloc(C, &C->dt, 1)) return r;
   if (int r = dalloc(C, &C->flags, 4)) return r;
   if (int r = dalloc(C, &C->counts, 8)) return r;
+  CK(cudaMemset(C->flags, 0, 4 * sizeof(int)));
+  CK(cudaMemset(C->counts, 0, 8 * sizeof(unsigned long long)));
   for (int d = 0; d < D; ++d) {
     const long long nI = Nc / g.N[d] * (g.N[d] + 1);
     if (int r = dalloc(C, &C->trace[d], (size_t)2 * V * T * NJ * Nc)) return r;
@@ -397,8 +399,6 @@ int spd_create(const spd_config* cfg, const spd_operators* ops, spd_ctx** out) {
       if (int r = dalloc(C, &C->theta_b, (size_t)Nqe)) return r;
       // whole 32-bit words: k_sed clears mask bits with a word-wide atomic AND
       if (int r = dalloc(C, &C->mask, (size_t)(Nq + 3) / 4 * 4)) return r;
-      if (int r = dalloc(C, &C->mark_cell, (size_t)Nqe)) return r;
-      if (int r = dalloc(C, &C->mark_q, (size_t)Nq)) return r;
       if (int r = dalloc(C, &C->list_cell, (size_t)Nqe)) return r;
       if (int r = dalloc(C, &C->list_q, (size_t)Nq)) return r;
       if (int r = dalloc(C, &C->list_sed, (size_t)2 * Nq)) return r;
@@ -429,10 +429,7 @@ int spd_create(const spd_config* cfg, const spd_operators* ops, spd_ctx** out) {
 int spd_destroy(spd_ctx* C) {
   if (!C) return SPD_ERR_ARG;
   if (C->stream) cudaStreamSynchronize(C->stream);
-  if (C->step_exec) cudaGraphExecDestroy(C->step_exec);
-  if (C->step_graph) cudaGraphDestroy(C->step_graph);
-  if (C->dt_exec) cudaGraphExecDestroy(C->dt_exec);
-  if (C->dt_graph) cudaGraphDestroy(C->dt_graph);
+  C->drop_step_graphs();
   for (void* p : C->allocs) cudaFree(p);
   for (void* p : C->adj_allocs) cudaFree(p);
   for (void* p : C->tape_allocs) cudaFree(p);
@@ -777,22 +774,24 @@ int spd_perform_update(spd_ctx* C, double* time_inout) {
   return SPD_OK;
 }
 
-// Capture one step into two graphs: the dt graph (CFL reduction, then the
-// clip of perform_time_evolution: dt = t_end - t where t + dt >= t_end, with
-// t and t_end in t_dev[0..1]) and the update graph (update, t_dev[0] += dt).
+// Capture of a step: part 0 is the dt graph (CFL reduction, then the clip of
+// perform_time_evolution: dt = t_end - t where t + dt >= t_end, with t and
+// t_end in t_dev[0..1]), part 1 the update graph (update, t_dev[0] += dt),
+// part 2 both in one graph, for runs whose host reads no dt between them.
 // Returns false (and leaves the context as it was) when capture is not
 // possible; the caller then steps launch by launch.
-static bool capture(spd_ctx* C, int part, cudaGraph_t* gout, cudaGraphExec_t* xout) {
+static bool capture(spd_ctx* C, int part, spd_ctx::StepGraph* out) {
   cudaStream_t s = C->stream;
   if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return false;
-  int rc;
-  if (part == 0) {
+  int rc = 0;
+  if (part != 1) {
     rc = C->stepper->cmax(C);
     if (!rc) {
       k_clip_dt<<<1, 1, 0, s>>>(C->t_dev, C->dt);
       if (cudaGetLastError() != cudaSuccess) rc = SPD_ERR_CUDA;
     }
-  } else {
+  }
+  if (part != 0 && !rc) {
     rc = C->stepper->update(C);
     if (!rc) {
       k_time_add_dev<<<1, 1, 0, s>>>(C->t_dev, C->dt);
@@ -801,18 +800,19 @@ static bool capture(spd_ctx* C, int part, cudaGraph_t* gout, cudaGraphExec_t* xo
   }
   cudaGraph_t g = nullptr;
   const cudaError_t ec = cudaStreamEndCapture(s, &g);
-  if (rc || ec != cudaSuccess || cudaGraphInstantiate(xout, g, 0) != cudaSuccess) {
+  if (rc || ec != cudaSuccess || cudaGraphInstantiate(&out->exec, g, 0) != cudaSuccess) {
     if (g) cudaGraphDestroy(g);
-    *xout = nullptr;
+    out->exec = nullptr;
     cudaGetLastError();
     return false;
   }
-  *gout = g;
+  out->graph = g;
   return true;
 }
 
-static bool build_step_graph(spd_ctx* C) {
-  if (C->step_exec) return true;
+// the graphs of one mode of spd_step, captured on first use
+static bool build_step_graph(spd_ctx* C, int mode) {
+  if (mode == 0 ? C->both.exec != nullptr : C->step.exec != nullptr) return true;
   if (C->step_graph_failed) return false;
   if (!C->t_dev_pair) {
     void* p = nullptr;
@@ -829,67 +829,62 @@ static bool build_step_graph(spd_ctx* C) {
   double* keep_new = C->U_new;
   double* keep_theta = C->theta_final;
   const long long launches = C->launches;
-  const bool ok = capture(C, 0, &C->dt_graph, &C->dt_exec) && capture(C, 1, &C->step_graph, &C->step_exec);
-  C->graph_kernels = C->launches - launches + 2;  // the step's kernels, the clip and the time add
-  C->launches = launches;                          // capture launched nothing
-  C->graph_U_cv = C->U_cv;
-  C->graph_U_new = C->U_new;
-  C->graph_theta = C->theta_final;
+  const bool ok = mode == 0 ? capture(C, 2, &C->both) : capture(C, 0, &C->dtg) && capture(C, 1, &C->step);
+  spd_ctx::StepGraph& sg = mode == 0 ? C->both : C->step;
+  sg.kernels = C->launches - launches + 2;  // the step's kernels, the clip and the time add
+  C->launches = launches;                   // capture launched nothing
+  sg.U_cv = C->U_cv;
+  sg.U_new = C->U_new;
+  sg.theta = C->theta_final;
   C->t_dev = keep_t;
+  // the roles as before: spd_step applies those of after once a step has run
+  C->U_cv = keep_cv;
+  C->U_new = keep_new;
+  C->theta_final = keep_theta;
   if (!ok) {
-    if (C->dt_exec) cudaGraphExecDestroy(C->dt_exec);
-    if (C->dt_graph) cudaGraphDestroy(C->dt_graph);
-    C->dt_exec = nullptr;
-    C->dt_graph = nullptr;
-    C->step_exec = nullptr;
-    C->U_cv = keep_cv;
-    C->U_new = keep_new;
-    C->theta_final = keep_theta;
+    C->drop_step_graphs();
     C->step_graph_failed = true;
-    return false;
   }
-  return true;
+  return ok;
 }
 
 int spd_step(spd_ctx* C, int nsteps, double t_end, int mode, double* time_inout, int* nsteps_done) {
   if (!C || !time_inout) return SPD_ERR_ARG;
   int done = 0;
   bool nonfinite = false;
-  const bool graphs = !C->prof && C->tape_mode == 0 && !C->recording && build_step_graph(C);
+  const bool graphs = !C->prof && C->tape_mode == 0 && !C->recording && build_step_graph(C, mode);
   if (graphs) {
-    // the step as two graph launches; time and the clip in the same double
+    // the step as one or two graph launches; time and the clip in the same double
     // operations as the host loop below
     const double te = (mode == 0) ? HUGE_VAL : t_end;
     const double tt[2] = {*time_inout, te};
     CK(cudaMemcpyAsync(C->t_dev_pair, tt, sizeof(tt), cudaMemcpyHostToDevice, C->stream));
     if (mode == 0) {
-      for (int i = 0; i < nsteps; ++i) {
-        CK(cudaGraphLaunch(C->dt_exec, C->stream));
-        CK(cudaGraphLaunch(C->step_exec, C->stream));
-      }
+      for (int i = 0; i < nsteps; ++i) CK(cudaGraphLaunch(C->both.exec, C->stream));
       done = nsteps > 0 ? nsteps : 0;
     } else {
       double t = *time_inout;
       while (t < t_end) {
-        CK(cudaGraphLaunch(C->dt_exec, C->stream));
+        CK(cudaGraphLaunch(C->dtg.exec, C->stream));
         double dt = 0.0;
         CK(cudaMemcpyAsync(&dt, C->dt, sizeof(double), cudaMemcpyDeviceToHost, C->stream));
         CK(cudaStreamSynchronize(C->stream));
         if (dt < 1e-14) break;
-        CK(cudaGraphLaunch(C->step_exec, C->stream));
+        CK(cudaGraphLaunch(C->step.exec, C->stream));
         t = t + dt;
         nonfinite = nonfinite || !std::isfinite(dt);
         ++done;
         if (nsteps > 0 && done >= nsteps) break;
       }
     }
-    C->launches += (long long)done * C->graph_kernels;
+    const spd_ctx::StepGraph& sg = mode == 0 ? C->both : C->step;
+    C->launches += (long long)done * sg.kernels;
     CK(cudaMemcpyAsync(time_inout, C->t_dev_pair, sizeof(double), cudaMemcpyDeviceToHost, C->stream));
     CK(cudaStreamSynchronize(C->stream));
     if (done) {
-      C->U_cv = C->graph_U_cv;
-      C->U_new = C->graph_U_new;
-      C->theta_final = C->graph_theta;
+      C->U_cv = sg.U_cv;
+      C->U_new = sg.U_new;
+      C->theta_final = sg.theta;
       if (C->cfg.update == SPD_UPDATE_FV && C->cfg.FB) C->fb_ran = true;
     }
     nonfinite = nonfinite || !std::isfinite(*time_inout);

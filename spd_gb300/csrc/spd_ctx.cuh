@@ -34,15 +34,26 @@ struct spd_ctx {
   double *U_sp = nullptr, *U_cv = nullptr, *W_cv = nullptr, *U_new = nullptr;
   double* dt = nullptr;
   double* t_dev = nullptr;  // simulated time kept on the device (ensemble driver, step graph)
-  // one captured step (dt graph: CFL dt and the t_end clip; update graph:
-  // update and time += dt) replayed by spd_step; the host-side buffer roles
-  // it leaves behind are restored after each replay
-  cudaGraph_t step_graph = nullptr, dt_graph = nullptr;
-  cudaGraphExec_t step_exec = nullptr, dt_exec = nullptr;
+  // one captured step (dtg: CFL dt and the t_end clip; step: update and time
+  // += dt; both: one graph of the two) replayed by spd_step; the host-side
+  // buffer roles it leaves behind are restored after each replay
+  struct StepGraph {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    // buffer roles after a replay, and its kernels
+    double *U_cv = nullptr, *U_new = nullptr, *theta = nullptr;
+    long long kernels = 0;
+  };
+  StepGraph dtg, step, both;
+  void drop_step_graphs() {
+    for (StepGraph* g : {&dtg, &step, &both}) {
+      if (g->exec) cudaGraphExecDestroy(g->exec);
+      if (g->graph) cudaGraphDestroy(g->graph);
+      *g = StepGraph{};
+    }
+  }
   double* t_dev_pair = nullptr;  // [time, t_end] of the step graphs
   bool step_graph_failed = false;
-  double *graph_U_cv = nullptr, *graph_U_new = nullptr, *graph_theta = nullptr;
-  long long graph_kernels = 0;
   // adjoint: record slots of forward intermediates and the adjoint work
   // arrays (allocated by spd_adjoint_enable, freed on re-enable and destroy)
   bool recording = false;
@@ -110,8 +121,8 @@ struct spd_ctx {
   double *ext_old = nullptr, *ext_new = nullptr, *theta_src = nullptr, *theta_a = nullptr, *theta_b = nullptr;
   double* theta_final = nullptr;
   double* bcbuf[3] = {nullptr, nullptr, nullptr};
-  unsigned char *mask = nullptr, *mark_cell = nullptr, *mark_q = nullptr;
-  int* flags = nullptr;  // [0] any possible trouble, [1] nan in cmax, [2] marked faces
+  unsigned char* mask = nullptr;
+  int* flags = nullptr;  // [0] any possible trouble, [1] nan in cmax
   // [0] marked extended cells, [1] marked subcells, [2] cmax bits, [3] subcells
   // with a NAD flag on density or pressure, [4 + d] affected faces of direction d
   unsigned long long* counts = nullptr;

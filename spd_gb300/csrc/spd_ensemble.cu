@@ -300,17 +300,10 @@ const char* spd_ensemble_last_error(const spd_ensemble* E) { return E ? E->err.c
 
 int spd_set_cells_per_block(spd_ctx* C, int cpb) {
   if (!C || cpb < 1 || cpb > C->stepper->max_cpb || (cpb & (cpb - 1))) return SPD_ERR_ARG;
-  if ((C->stepper->cpb != cpb || C->stepper->auto_cpb) && C->step_exec) {
-    // the captured step carries the old launch shape
+  if (C->stepper->cpb != cpb || C->stepper->auto_cpb) {
+    // a captured step carries the old launch shape
     cudaStreamSynchronize(C->stream);
-    cudaGraphExecDestroy(C->step_exec);
-    cudaGraphDestroy(C->step_graph);
-    cudaGraphExecDestroy(C->dt_exec);
-    cudaGraphDestroy(C->dt_graph);
-    C->step_exec = nullptr;
-    C->step_graph = nullptr;
-    C->dt_exec = nullptr;
-    C->dt_graph = nullptr;
+    C->drop_step_graphs();
   }
   C->stepper->cpb = cpb;
   C->stepper->auto_cpb = false;

@@ -114,6 +114,103 @@ __device__ __forceinline__ void flux_divergence(const Geo& g, const FvGeo& fg, i
   out = acc;
 }
 
+// Ghost layers written by the active subcells they mirror.
+//
+// The reference fills them direction by direction (src/fv_simulator.py:
+// 224-273), each fill reading the ghosts of the directions before it, so a
+// ghost subcell's value follows from one active subcell: along every ghost
+// direction the periodic or the nearest-edge image (whose layers are not
+// mirrored), the normal velocity negated at a reflective side, and at a side
+// with a fixed state the stored layer.  Writing it from that subcell saves
+// the fills: at 32^2 a substep launched six of them, 4 us each.
+//
+// for_ghosts calls f(e, choice) for every ghost position e (extended
+// coordinates) of the active subcell a; choice[d] is -1 (not a ghost along
+// d) or the side.
+template <int D, class F>
+__device__ __forceinline__ void for_ghosts(const Geo& g, const int* a, F f) {
+  int pos[3][2];  // image at either side, or -1
+  bool any = false;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    const int X = g.X[d], i = a[d];
+    const bool lo = i < NGH, hi = i >= X - NGH;
+    pos[d][0] = (g.bc[d][0] == BC_PERIODIC) ? (hi ? i - (X - NGH) : -1) : (lo ? i : -1);
+    pos[d][1] = (g.bc[d][1] == BC_PERIODIC) ? (lo ? X + NGH + i : -1) : (hi ? i + 2 * NGH : -1);
+    any = any || lo || hi;
+  }
+  if (!any) return;
+  constexpr int combos = (D == 1) ? 3 : (D == 2 ? 9 : 27);
+#pragma unroll 1
+  for (int m = 1; m < combos; ++m) {
+    int e[3] = {0, 0, 0}, choice[3] = {-1, -1, -1};
+    bool ok = true;
+    int r = m;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      choice[d] = r % 3 - 1;
+      r /= 3;
+      const int p = (choice[d] < 0) ? a[d] + NGH : (choice[d] == 0 ? pos[d][0] : pos[d][1]);
+      ok = ok && p >= 0;
+      e[d] = p;
+    }
+    if (ok) f(e, choice);
+  }
+}
+__device__ __forceinline__ long long ext_at(const Geo& g, const int* e) {
+  return e[0] + (long long)g.Xe[0] * (e[1] + (long long)g.Xe[1] * e[2]);
+}
+// entry of direction d's boundary buffer [side][v][layer][other] for the ghost
+// position e
+__device__ __forceinline__ long long bc_entry(const Geo& g, int d, int side, int nv, int v, const int* e) {
+  const int o0 = (d == 0) ? 1 : 0, o1 = (d == 2) ? 1 : 2;
+  const long long nother = (long long)g.Xe[o0] * g.Xe[o1];
+  const int layer = (side == 0) ? e[d] : e[d] - (g.X[d] + NGH);
+  return (((long long)side * nv + v) * NGH + layer) * nother + e[o0] + (long long)g.Xe[o0] * e[o1];
+}
+struct BcBufs {
+  double* b[3];
+};
+// the primitives W of the active subcell a into the ghosts it owns
+template <int D>
+__device__ __forceinline__ void write_ghosts(const Geo& g, const BcBufs& bc, const int* a, const double* W,
+                                             double* __restrict__ ext) {
+  constexpr int V = D + 2;
+  for_ghosts<D>(g, a, [&](const int* e, const int* choice) {
+    double w[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) w[v] = W[v];
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      if (choice[d] < 0) continue;
+      const int kind = g.bc[d][choice[d]];
+      if (kind == BC_REFLECTIVE) {
+        w[d + 1] = w[d + 1] * -1.0;
+      } else if (kind == BC_EQ) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) w[v] = 0.0;
+      } else if (kind != BC_PERIODIC && kind != BC_GRADFREE) {
+        // the stored layer, at this ghost along the directions before d and
+        // at the active position along those after
+        int at[3] = {0, 0, 0};
+#pragma unroll
+        for (int q = 0; q < D; ++q) at[q] = (q <= d) ? e[q] : a[q] + NGH;
+#pragma unroll
+        for (int v = 0; v < V; ++v) w[v] = bc.b[d][bc_entry(g, d, choice[d], V, v, at)];
+      }
+    }
+    const long long x = ext_at(g, e);
+#pragma unroll
+    for (int v = 0; v < V; ++v) ext[(long long)v * g.Nqe + x] = w[v];
+  });
+}
+
+// counters that a substep accumulates, zeroed by its first kernel
+struct Counters {
+  int* flags;                  // [0] any possible trouble
+  unsigned long long* counts;  // [0..1], [3] and [4..4+D) of spd_ctx::counts
+};
+
 // candidate update with the high-order fluxes of time node i, W_old and
 // W_new into the extended arrays (src/sdader_simulator.py:336-340,
 // src/trouble_detection.py:10-13)
@@ -123,15 +220,23 @@ struct FvCandidate {
 // W_new = prim(U_new) into ext_old / ext_new; 2 = as 1 with W_old read from
 // ext_new, which holds prim(U_cv) at this point (the previous substep's
 // W_new, refreshed by k_fv_correct where the fallback changed U_cv): the
-// same values without a second primitive conversion.
+// same values without a second primitive conversion.  W_cv (the step's last
+// substep, else null): the primitives of the new state in the subcell layout,
+// which k_fv_correct refreshes likewise (src/sdader_simulator.py:351-359).
 static __device__ __forceinline__ void run(Blk B, const Geo& g, const FvGeo& fg, const double* __restrict__ dt_ptr,
                                            double w_i, const double* F0, const double* F1, const double* F2,
                                            const double* __restrict__ U_cv, double* __restrict__ U_new,
-                                           double* ext_old, double* ext_new, int write_ext,
+                                           double* ext_old, double* ext_new, int write_ext, const BcBufs& bc,
+                                           const Counters& ct, double* __restrict__ W_cv,
                                            const double* __restrict__ gphi, const double* __restrict__ Ueq,
                                            const double* __restrict__ Weq) {
   constexpr int V = D + 2;
   const long long q = B.id * (long long)blockDim.x + threadIdx.x;
+  if (q == 0 && write_ext) {
+    ct.flags[0] = 0;
+    ct.counts[0] = ct.counts[1] = ct.counts[3] = 0;
+    for (int d = 0; d < D; ++d) ct.counts[4 + d] = 0;
+  }
   if (q >= g.Nq) return;
   int ix, iy, iz;
   q_coords(g, q, ix, iy, iz);
@@ -159,9 +264,16 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, const FvGeo& fg,
     }
 #pragma unroll
     for (int v = 0; v < V; ++v) ext_old[(long long)v * g.Nqe + e] = W[v];
+    const int a[3] = {ix, iy, iz};
+    write_ghosts<D>(g, bc, a, W, ext_old);
     prims_cv<D>(g, un, W, Ueq, Weq, q);
 #pragma unroll
     for (int v = 0; v < V; ++v) ext_new[(long long)v * g.Nqe + e] = W[v];
+    write_ghosts<D>(g, bc, a, W, ext_new);
+    if (W_cv != nullptr) {
+#pragma unroll
+      for (int v = 0; v < V; ++v) W_cv[(long long)v * g.Nq + q] = W[v];
+    }
   }
 }
 };
@@ -169,45 +281,21 @@ template <int D>
 __global__ void k_fv_candidate(Geo g, FvGeo fg, const double* __restrict__ dt_ptr, double w_i,
                                const double* F0, const double* F1, const double* F2,
                                const double* __restrict__ U_cv, double* __restrict__ U_new, double* ext_old,
-                               double* ext_new, int write_ext, const double* __restrict__ gphi,
-                               const double* __restrict__ Ueq, const double* __restrict__ Weq) {
-  FvCandidate<D>::run(hw_blk(), g, fg, dt_ptr, w_i, F0, F1, F2, U_cv, U_new, ext_old, ext_new, write_ext, gphi, Ueq,
-                      Weq);
-}
-
-// W_cv (subcell layout) from the active region of an extended primitive
-// array: the end-of-step primitives when ext_new holds prim of the final
-// subcell state (src/sdader_simulator.py:351-359 computed once, in the last
-// substep's candidate update and corrected update)
-template <int D>
-struct ExtToPlain {
-  static __device__ __forceinline__ void run(Blk B, const Geo& g, const double* __restrict__ ext,
-                                             double* __restrict__ W_cv) {
-    constexpr int V = D + 2;
-    const long long q = B.id * (long long)blockDim.x + threadIdx.x;
-    if (q >= g.Nq) return;
-    int ix, iy, iz;
-    q_coords(g, q, ix, iy, iz);
-    const long long e = ext_of<D>(g, ix, iy, iz);
-#pragma unroll
-    for (int v = 0; v < V; ++v) W_cv[(long long)v * g.Nq + q] = ext[(long long)v * g.Nqe + e];
-  }
-};
-template <int D>
-__global__ void k_ext_to_plain(Geo g, const double* __restrict__ ext, double* __restrict__ W_cv) {
-  ExtToPlain<D>::run(hw_blk(), g, ext, W_cv);
+                               double* ext_new, int write_ext, BcBufs bc, Counters ct,
+                               double* __restrict__ W_cv, const double* __restrict__ gphi, const double* __restrict__ Ueq,
+                               const double* __restrict__ Weq) {
+  FvCandidate<D>::run(hw_blk(), g, fg, dt_ptr, w_i, F0, F1, F2, U_cv, U_new, ext_old, ext_new, write_ext, bc, ct, W_cv,
+                      gphi, Ueq, Weq);
 }
 
 // ghost fill of one direction (src/fv_simulator.py:224-273): store the
 // boundary buffer when the reference does, then copy it into the ghost
 // layers.  bcbuf layout [side][v][g][other], other = the extended index of
-// the remaining directions (lower direction fastest).  When ``gate`` is
-// non-null the fill runs only if *gate != 0.
+// the remaining directions (lower direction fastest).  The adjoint rebuilds a
+// substep's primitives with it; the step writes its ghosts with write_ghosts.
 template <int D>
 struct Ghost {
-static __device__ __forceinline__ void run(Blk B, const Geo& g, int d, int all, int nv, int nv_buf, double* ext,
-                                           double* bcbuf, const int* gate) {
-  if (gate != nullptr && *gate == 0) return;
+static __device__ __forceinline__ void run(Blk B, const Geo& g, int d, int nv, double* ext, double* bcbuf) {
   const int o0 = (d == 0) ? 1 : 0;
   const int o1 = (d == 2) ? 1 : 2;
   const long long nother = (long long)g.Xe[o0] * g.Xe[o1];
@@ -231,17 +319,17 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, int d, int all, 
     c[o1] = b;
     return c[0] + (long long)g.Xe[0] * (c[1] + (long long)g.Xe[1] * c[2]);
   };
-  const long long bidx = (((long long)side * nv_buf + v) * NGH + gi) * nother + other;
+  const long long bidx = (((long long)side * nv + v) * NGH + gi) * nother + other;
   double val;
   bool store = false;
   int src = 0;
   if (kind == BC_PERIODIC) { store = true; src = (side == 0) ? Xd + gi : NGH + gi; }
-  else if ((kind == BC_REFLECTIVE || kind == BC_GRADFREE) && all) { store = true; src = (side == 0) ? NGH + gi : Xd + gi; }
+  else if (kind == BC_REFLECTIVE || kind == BC_GRADFREE) { store = true; src = (side == 0) ? NGH + gi : Xd + gi; }
   if (store) {
     val = ext[(long long)v * g.Nqe + ext_index(src)];
     if (kind == BC_REFLECTIVE && v == d + 1) val = val * -1.0;
     bcbuf[bidx] = val;
-  } else if (kind == BC_EQ && all) {
+  } else if (kind == BC_EQ) {
     val = 0.0;
     bcbuf[bidx] = val;
   } else {
@@ -252,8 +340,8 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, int d, int all, 
 }
 };
 template <int D>
-__global__ void k_ghost(Geo g, int d, int all, int nv, int nv_buf, double* ext, double* bcbuf, const int* gate) {
-  Ghost<D>::run(hw_blk(), g, d, all, nv, nv_buf, ext, bcbuf, gate);
+__global__ void k_ghost(Geo g, int d, int nv, double* ext, double* bcbuf) {
+  Ghost<D>::run(hw_blk(), g, d, nv, ext, bcbuf);
 }
 
 // NAD: relaxed discrete maximum principle over the cross stencil
@@ -433,13 +521,22 @@ __global__ void k_sed(Geo g, FvGeo fg, const long long* __restrict__ list, const
 // trouble flags (NAD flags of density or pressure after the smooth-extrema
 // relaxation) and PAD; writes the troubles into var 0 of the theta-source
 // extended array and the troubles array.
+//
+// The troubles' ghosts: at periodic sides the image's trouble; elsewhere the
+// reference leaves its boundary buffer as the last fill of the primitives
+// left it, whose variable 0 is the density of W_new where any subcell was
+// flagged (and the smoothness relaxation ran), else of W_old
+// (src/fv_simulator.py:224-273, src/trouble_detection.py:40-72).  The buffers
+// themselves are kept as the fills leave them.
 template <int D>
 struct Troubles {
 static __device__ __forceinline__ void run(Blk B, const Geo& g, int pad, double min_rho, double max_rho, double min_P,
-                                           const unsigned char* __restrict__ mask,
-                                           const double* __restrict__ ext_new, double* __restrict__ theta_src,
-                                           double* __restrict__ troubles, const double* __restrict__ Weq) {
-  constexpr int P_ = D + 1;
+                                           const unsigned char* __restrict__ mask, const int* __restrict__ flags,
+                                           int sed, const double* __restrict__ ext_old,
+                                           const double* __restrict__ ext_new, const BcBufs& bc,
+                                           double* __restrict__ theta_src, double* __restrict__ troubles,
+                                           const double* __restrict__ Weq) {
+  constexpr int V = D + 2, P_ = D + 1;
   const long long q = B.id * (long long)blockDim.x + threadIdx.x;
   if (q >= g.Nq) return;
   int ix, iy, iz;
@@ -464,14 +561,36 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, int pad, double 
   }
   theta_src[e] = t;
   troubles[q] = t;
+  const int a[3] = {ix, iy, iz};
+  for_ghosts<D>(g, a, [&](const int* x, const int* choice) {
+    const double* W = (sed && *flags != 0) ? ext_new : ext_old;
+    const long long xe = ext_at(g, x);
+    double th = t;
+    int last = 0;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      if (choice[d] < 0) continue;
+      if (g.bc[d][choice[d]] != BC_PERIODIC) th = W[xe];
+      last = d;
+    }
+    theta_src[xe] = th;
+    const int side = choice[last], kind = g.bc[last][side];
+    if (kind != BC_PERIODIC && kind != BC_REFLECTIVE && kind != BC_GRADFREE && kind != BC_EQ) return;
+    double* b = last == 0 ? bc.b[0] : (last == 1 ? bc.b[1] : bc.b[2]);
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+      b[bc_entry(g, last, side, V, v, x)] = (v == 0 && kind == BC_PERIODIC) ? th : W[(long long)v * g.Nqe + xe];
+  });
 }
 };
 template <int D>
 __global__ void k_troubles(Geo g, int pad, double min_rho, double max_rho, double min_P,
-                           const unsigned char* __restrict__ mask, const double* __restrict__ ext_new,
+                           const unsigned char* __restrict__ mask, const int* __restrict__ flags, int sed,
+                           const double* __restrict__ ext_old, const double* __restrict__ ext_new, BcBufs bc,
                            double* __restrict__ theta_src, double* __restrict__ troubles,
                            const double* __restrict__ Weq) {
-  Troubles<D>::run(hw_blk(), g, pad, min_rho, max_rho, min_P, mask, ext_new, theta_src, troubles, Weq);
+  Troubles<D>::run(hw_blk(), g, pad, min_rho, max_rho, min_P, mask, flags, sed, ext_old, ext_new, bc, theta_src,
+                   troubles, Weq);
 }
 
 // extended-grid coordinates
@@ -546,116 +665,44 @@ __global__ void k_blend_neighbours(Geo g, const double* __restrict__ src, double
   BlendNeighbours<D>::run(hw_blk(), g, src, out);
 }
 
-// last blending layer along direction d (src/trouble_detection.py:167-169):
-// two sequential in-place sweeps, fused with a one-cell halo.
+// last blending layer (src/trouble_detection.py:167-169): per direction two
+// sequential in-place sweeps, the directions one after the other.  The value
+// after the sweeps of the directions below LEVEL, from the 3^LEVEL input
+// values it depends on: one launch reading 9 (27) cached values instead of
+// one per direction.
+template <int LEVEL>
+__device__ __forceinline__ double blended(const Geo& g, const int* c, long long e, const double* __restrict__ in) {
+  if constexpr (LEVEL == 0) {
+    return in[e];
+  } else {
+    constexpr int d = LEVEL - 1;
+    const long long st = ext_stride(g, d);
+    const int k = c[d];
+    const double t0 = blended<d>(g, c, e, in);
+    // after the first sweep: here and at the cell before
+    double a0 = t0;
+    if (k < g.Xe[d] - 1) a0 = np_max_key(gt0_key(blended<d>(g, c, e + st, in)) ? 0.25 : 0.0, t0);
+    if (k < 1) return a0;
+    const double am = np_max_key(gt0_key(t0) ? 0.25 : 0.0, blended<d>(g, c, e - st, in));
+    return np_max_key(gt0_key(am) ? 0.25 : 0.0, a0);
+  }
+}
 template <int D>
 struct BlendLast {
-static __device__ __forceinline__ void run(Blk B, const Geo& g, int d, const double* __restrict__ in,
+static __device__ __forceinline__ void run(Blk B, const Geo& g, const double* __restrict__ in,
                                            double* __restrict__ out) {
   const long long e = B.id * (long long)blockDim.x + threadIdx.x;
   if (e >= g.Nqe) return;
   int c[3];
   e_coords(g, e, c[0], c[1], c[2]);
-  const long long st = ext_stride(g, d);
-  const int last = g.Xe[d] - 1;
-  auto th_a = [&](int k, long long ek) {  // after the first sweep
-    const double t = in[ek];
-    if (k < last) return np_max_key(gt0_key(in[ek + st]) ? 0.25 : 0.0, t);
-    return t;
-  };
-  const int k = c[d];
-  const double a0 = th_a(k, e);
-  if (k >= 1) {
-    const double am = th_a(k - 1, e - st);
-    out[e] = np_max_key(gt0_key(am) ? 0.25 : 0.0, a0);
-  } else {
-    out[e] = a0;
-  }
+  out[e] = blended<D>(g, c, e, in);
 }
 };
 template <int D>
-__global__ void k_blend_last(Geo g, int d, const double* __restrict__ in, double* __restrict__ out) {
-  BlendLast<D>::run(hw_blk(), g, d, in, out);
+__global__ void k_blend_last(Geo g, const double* __restrict__ in, double* __restrict__ out) {
+  BlendLast<D>::run(hw_blk(), g, in, out);
 }
 
-// affected faces of direction d (src/trouble_detection.py:81-87) and the
-// marks for the fallback fluxes and the corrected update.  With theta ==
-// nullptr the affected faces already in ``aff`` are used (replayed
-// decisions).
-template <int D>
-struct Affected {
-static __device__ __forceinline__ void run(Blk B, const Geo& g, int d, int godunov, const double* __restrict__ theta,
-                                           double* __restrict__ aff, unsigned char* __restrict__ mark_cell,
-                                           unsigned char* __restrict__ mark_q, int* __restrict__ nmarked,
-                                           long long* __restrict__ flist, unsigned long long* __restrict__ fcount) {
-  const long long nf = n_faces(g, d);
-  const long long fidx = B.id * (long long)blockDim.x + threadIdx.x;
-  bool need = false;
-  if (fidx < nf) {
-    const int FX = g.X[0] + (d == 0), FY = g.X[1] + (d == 1);
-    int f[3];
-    f[0] = (int)(fidx % FX);
-    long long r = fidx / FX;
-    f[1] = (int)(r % FY);
-    f[2] = (int)(r / FY);
-    int e1[3], e2[3];
-    for (int k = 0; k < 3; ++k) {
-      const int base = (k < D) ? f[k] + NGH : 0;
-      e1[k] = base;
-      e2[k] = base;
-    }
-    e1[d] = f[d] + 1;
-    e2[d] = f[d] + 2;
-    const long long i1 = e1[0] + (long long)g.Xe[0] * (e1[1] + (long long)g.Xe[1] * e1[2]);
-    const long long i2 = e2[0] + (long long)g.Xe[0] * (e2[1] + (long long)g.Xe[1] * e2[2]);
-    double a;
-    if (theta) {
-      a = np_max_key(theta[i1], theta[i2]);
-      aff[fidx] = a;
-    } else {
-      a = aff[fidx];
-    }
-    need = godunov || nonzero_bits(a);
-    if (need) {
-      mark_cell[i1] = 1;
-      mark_cell[i2] = 1;
-      int q[3] = {f[0], f[1], f[2]};
-      if (f[d] >= 1) {
-        q[d] = f[d] - 1;
-        mark_q[q[0] + (long long)g.X[0] * (q[1] + (long long)g.X[1] * q[2])] = 1;
-      }
-      if (f[d] < g.X[d]) {
-        q[d] = f[d];
-        mark_q[q[0] + (long long)g.X[0] * (q[1] + (long long)g.X[1] * q[2])] = 1;
-      }
-    }
-  }
-  const unsigned b = __ballot_sync(0xffffffffu, need);
-  if (b != 0) {
-    // the faces that need a fallback flux, compacted by warp ballot: an FP64
-    // warp instruction costs the same with 1 or 32 active lanes, so the
-    // fallback Riemann problems run on full warps over this list
-    const int lane = threadIdx.x & 31;
-    unsigned long long base = 0;
-    if (lane == 0) {
-      atomicAdd(nmarked, __popc(b));
-      base = atomicAdd(fcount, (unsigned long long)__popc(b));
-    }
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (need) flist[base + __popc(b & ((1u << lane) - 1u))] = fidx;
-  }
-}
-};
-template <int D>
-__global__ void k_affected(Geo g, int d, int godunov, const double* __restrict__ theta, double* __restrict__ aff,
-                           unsigned char* __restrict__ mark_cell, unsigned char* __restrict__ mark_q,
-                           int* __restrict__ nmarked, long long* __restrict__ flist,
-                           unsigned long long* __restrict__ fcount) {
-  Affected<D>::run(hw_blk(), g, d, godunov, theta, aff, mark_cell, mark_q, nmarked, flist, fcount);
-}
-
-// compaction of marked indices by warp ballot: writes the marked indices
-// into list and their count into *count.
 // Appends ``value`` of every lane with ``keep`` to list (order within the
 // list unspecified), one atomic per warp.  All 32 lanes of the warp must
 // call it.
@@ -670,23 +717,71 @@ __device__ __forceinline__ void warp_append(bool keep, long long value, long lon
   if (keep) list[base + __popc(b & ((1u << lane) - 1u))] = value;
 }
 
-struct Compact {
-  static __device__ __forceinline__ void run(Blk B, long long total, const unsigned char* __restrict__ mark,
-                                             long long* __restrict__ list, unsigned long long* __restrict__ count) {
-    const long long i = B.id * (long long)blockDim.x + threadIdx.x;
-    const bool m = (i < total) && mark[i];
-    const unsigned b = __ballot_sync(0xffffffffu, m);
-    if (b == 0) return;
-    const int lane = threadIdx.x & 31;
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(count, (unsigned long long)__popc(b));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (m) list[base + __popc(b & ((1u << lane) - 1u))] = i;
-  }
+// Affected faces of every direction (src/trouble_detection.py:81-87) and the
+// lists of what the fallback needs, one thread per extended subcell, which
+// looks at the faces on both of its sides: the faces that need a fallback
+// flux, the extended subcells next to one (their slopes and predictions) and
+// the active subcells next to one (the corrected update).  Compacted lists,
+// because an FP64 warp instruction costs the same with 1 or 32 active lanes.
+// With theta == nullptr the affected faces already in ``aff`` are used
+// (replayed decisions).
+struct AffectedOut {
+  double* aff[3];
+  long long* flist[3];
+  long long *cells, *active;
+  unsigned long long* counts;  // [0] cells, [1] active, [4 + d] faces
 };
-static __global__ void k_compact(long long total, const unsigned char* __restrict__ mark, long long* __restrict__ list,
-                          unsigned long long* __restrict__ count) {
-  Compact::run(hw_blk(), total, mark, list, count);
+template <int D>
+struct AffectedAll {
+static __device__ __forceinline__ void run(Blk B, const Geo& g, int godunov, const double* __restrict__ theta,
+                                           const AffectedOut& out) {
+  const long long e = B.id * (long long)blockDim.x + threadIdx.x;
+  bool mark = false, inside = e < g.Nqe;
+  int c[3] = {0, 0, 0};
+  if (inside) e_coords(g, e, c[0], c[1], c[2]);
+  bool in_dir[3] = {true, true, true};
+#pragma unroll
+  for (int d = 0; d < D; ++d) in_dir[d] = inside && c[d] >= NGH && c[d] < NGH + g.X[d];
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    // the other coordinates are active
+    const bool row = inside && (D < 2 || in_dir[d == 0 ? 1 : 0]) && (D < 3 || in_dir[d == 2 ? 1 : 2]);
+    const long long st = ext_stride(g, d);
+    const int fr = c[d] - 1;  // the face above; fr - 1 is the one below
+    int f[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) f[q] = (q < D) ? c[q] - NGH : 0;
+    bool need = false;
+    long long fid = 0;
+    if (row && fr >= 0 && fr <= g.X[d]) {
+      f[d] = fr;
+      fid = face_id(g, d, f[0], f[1], f[2]);
+      double a;
+      if (theta) {
+        a = np_max_key(theta[e], theta[e + st]);
+        out.aff[d][fid] = a;
+      } else {
+        a = out.aff[d][fid];
+      }
+      need = godunov || nonzero_bits(a);
+      mark = mark || need;
+    }
+    if (row && fr >= 1 && fr - 1 <= g.X[d]) {
+      f[d] = fr - 1;
+      const double a = theta ? np_max_key(theta[e - st], theta[e]) : out.aff[d][face_id(g, d, f[0], f[1], f[2])];
+      mark = mark || godunov || nonzero_bits(a);
+    }
+    warp_append(need, fid, out.flist[d], out.counts + 4 + d);
+  }
+  warp_append(mark, e, out.cells, out.counts);
+  const long long q = (c[0] - NGH) + (long long)g.X[0] * ((D > 1 ? c[1] - NGH : 0) +
+                                                        (long long)g.X[1] * (D > 2 ? c[2] - NGH : 0));
+  warp_append(mark && in_dir[0] && in_dir[1] && in_dir[2], q, out.active, out.counts + 1);
+}
+};
+template <int D>
+__global__ void k_affected_all(Geo g, int godunov, const double* __restrict__ theta, AffectedOut out) {
+  AffectedAll<D>::run(hw_blk(), g, godunov, theta, out);
 }
 
 // MUSCL-Hancock: limited gradients, slopes and the half-step primitive
@@ -793,15 +888,15 @@ __global__ void k_muscl_cells(Geo g, FvGeo fg, int limiter, const double* __rest
   MusclCells<D, BM>::run(hw_blk(), g, fg, limiter, dt_ptr, w_i, list, count, W_ext, Mpred, S, ltape, Meq, gphi);
 }
 
-// fallback Riemann flux on the affected faces of direction d
+// fallback Riemann flux on the affected faces
 // (src/muscl.py:217-221, src/fv_simulator.py:88-165)
 // DIR >= 0 fixes the direction at compile time (the rotated velocity indices
 // become constants: with a runtime direction the states are indexed in local
 // memory); DIR = -1 takes it from d_rt.  SV as in RiemannSd.
 template <int D, int BM = 0, int DIR = -1, int SV = -1>
 struct MusclFaces {
-// the affected faces of direction d from their compacted list (k_affected),
-// a grid-stride loop over full warps
+// direction d's affected faces from their compacted list (k_affected_all), a
+// grid-stride loop over full warps
 static __device__ __forceinline__ void run(Blk B, const Geo& g, int d_rt, int solver,
                                            const long long* __restrict__ flist,
                                            const unsigned long long* __restrict__ fcount,
@@ -860,6 +955,50 @@ __global__ void k_muscl_faces(Geo g, int d, int solver, const long long* __restr
   MusclFaces<D, BM, DIR, SV>::run(hw_blk(), g, d, solver, flist, fcount, Mpred, S, F_FB, ftape, Mq, Fq);
 }
 
+// the same over the lists of all directions in one launch, each list from the
+// next whole warp on
+struct FaceLists {
+  const long long* list[3];
+  const unsigned long long* count;  // [d]
+  double* F[3];
+  const double* Mq[3];
+  const double* Fq[3];
+};
+template <int D, int SV>
+struct MusclFacesAll {
+static __device__ __forceinline__ void run(Blk B, const Geo& g, int solver, const FaceLists& fl,
+                                           const double* __restrict__ Mpred, const double* __restrict__ S) {
+  unsigned long long end[3] = {0, 0, 0}, cnt[3];
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    cnt[d] = fl.count[d];
+    end[d] = (d > 0 ? end[d - 1] : 0) + ((cnt[d] + 31) & ~31ULL);
+  }
+  for (unsigned long long idx = B.id * (unsigned long long)blockDim.x + threadIdx.x; idx < end[D - 1];
+       idx += (unsigned long long)B.n * blockDim.x) {
+    if (idx < end[0]) {
+      if (idx < cnt[0])
+        MusclFaces<D, 0, 0, SV>::face(g, 0, solver, fl.list[0][idx], Mpred, S, fl.F[0], nullptr, fl.Mq[0], fl.Fq[0]);
+    } else if (D > 1 && idx < end[1]) {
+      const unsigned long long k = idx - end[0];
+      if (k < cnt[1])
+        MusclFaces<D, 0, (D > 1 ? 1 : 0), SV>::face(g, 1, solver, fl.list[1][k], Mpred, S, fl.F[1], nullptr, fl.Mq[1],
+                                                    fl.Fq[1]);
+    } else if (D > 2) {
+      const unsigned long long k = idx - end[1];
+      if (k < cnt[2])
+        MusclFaces<D, 0, (D > 2 ? 2 : 0), SV>::face(g, 2, solver, fl.list[2][k], Mpred, S, fl.F[2], nullptr, fl.Mq[2],
+                                                    fl.Fq[2]);
+    }
+  }
+}
+};
+template <int D, int SV>
+__global__ void k_muscl_faces_all(Geo g, int solver, FaceLists fl, const double* __restrict__ Mpred,
+                                  const double* __restrict__ S) {
+  MusclFacesAll<D, SV>::run(hw_blk(), g, solver, fl, Mpred, S);
+}
+
 // corrected update of the subcells next to an affected face
 // (src/sdader_simulator.py:325-331,346)
 template <int D>
@@ -870,7 +1009,8 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, const FvGeo& fg,
                                            const double* F1, const double* F2, const double* B0, const double* B1,
                                            const double* B2, const double* A0, const double* A1, const double* A2,
                                            const double* __restrict__ U_cv, double* __restrict__ U_new,
-                                           double* __restrict__ ext_new, const double* __restrict__ gphi,
+                                           double* __restrict__ ext_new, double* __restrict__ W_cv,
+                                           const double* __restrict__ gphi,
                                            const double* __restrict__ Ueq, const double* __restrict__ Weq) {
   constexpr int V = D + 2;
   const unsigned long long cnt = *count;
@@ -914,15 +1054,17 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, const FvGeo& fg,
     un[v] = u[v] - dudt[v] * dti;
     U_new[(long long)v * g.Nq + q] = un[v];
   }
-  if (ext_new != nullptr) {
+  {
     // the primitives of the corrected state: the next substep's W_old
-    // (k_fv_candidate with write_ext == 2) or, after the last substep, W_cv
-    // (k_ext_to_plain)
+    // (k_fv_candidate with write_ext == 2) and, in the last substep, W_cv
     double W[V];
     prims_cv<D>(g, un, W, Ueq, Weq, q);
     const long long e = ext_of<D>(g, ix, iy, iz);
 #pragma unroll
-    for (int v = 0; v < V; ++v) ext_new[(long long)v * g.Nqe + e] = W[v];
+    for (int v = 0; v < V; ++v) {
+      ext_new[(long long)v * g.Nqe + e] = W[v];
+      if (W_cv != nullptr) W_cv[(long long)v * g.Nq + q] = W[v];
+    }
   }
   }
 }
@@ -933,10 +1075,10 @@ __global__ void k_fv_correct(Geo g, FvGeo fg, const double* __restrict__ dt_ptr,
                              const double* F0, const double* F1, const double* F2, const double* B0,
                              const double* B1, const double* B2, const double* A0, const double* A1,
                              const double* A2, const double* __restrict__ U_cv, double* __restrict__ U_new,
-                             double* __restrict__ ext_new, const double* __restrict__ gphi,
-                             const double* __restrict__ Ueq, const double* __restrict__ Weq) {
+                             double* __restrict__ ext_new, double* __restrict__ W_cv,
+                             const double* __restrict__ gphi, const double* __restrict__ Ueq, const double* __restrict__ Weq) {
   FvCorrect<D>::run(hw_blk(), g, fg, dt_ptr, w_i, godunov, list, count, F0, F1, F2, B0, B1, B2, A0, A1, A2, U_cv,
-                    U_new, ext_new, gphi, Ueq, Weq);
+                    U_new, ext_new, W_cv, gphi, Ueq, Weq);
 }
 
 // Well-balanced mode around the step (src/sdader_simulator.py:363-376):
@@ -983,18 +1125,21 @@ __global__ void k_wb_end(Geo g, double* __restrict__ U_cv, const double* __restr
 // viscous limit only when dt_visc >= 0; Python's min keeps its first
 // argument unless the second is smaller, so a NaN dt stays NaN)
 struct DtFinal {
-  static __device__ __forceinline__ void run(Blk, double h, double cfl, const unsigned long long* cmax_bits,
-                                             const int* nan_flag, double* dt, double dt_visc) {
+  static __device__ __forceinline__ void run(Blk, double h, double cfl, unsigned long long* cmax_bits, int* nan_flag,
+                                             double* dt, double dt_visc) {
     if (threadIdx.x != 0) return;
     const double cmax = *nan_flag ? __longlong_as_double(0x7ff8000000000000LL)
                                   : __longlong_as_double((long long)*cmax_bits);
     double dtt = h / cmax;
     if (dt_visc >= 0.0 && dt_visc < dtt) dtt = dt_visc;
     *dt = cfl * dtt;
+    // for the next reduction
+    *cmax_bits = 0;
+    *nan_flag = 0;
   }
 };
-static __global__ void k_dt_final(double h, double cfl, const unsigned long long* cmax_bits, const int* nan_flag,
-                           double* dt, double dt_visc) {
+static __global__ void k_dt_final(double h, double cfl, unsigned long long* cmax_bits, int* nan_flag, double* dt,
+                                  double dt_visc) {
   DtFinal::run(hw_blk(), h, cfl, cmax_bits, nan_flag, dt, dt_visc);
 }
 

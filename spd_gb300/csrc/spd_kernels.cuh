@@ -269,6 +269,39 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, int d_rt, int Te
   for (int v = 0; v < k::V; ++v) Fi[(((long long)v * g.T + t) * k::NJ + j) * nI + iface] = F[v];
 }
 };
+// all directions in one launch, each from the next block on (on small grids a
+// launch costs more than its problems)
+struct RiemannDirs {
+  const double* trace[3];
+  const double* bcfix[3];
+  double* Fi[3];
+  const double* meq[3];
+  unsigned blocks[3];  // per direction
+};
+template <int D, int P, bool EQ, int SV>
+struct RiemannAll {
+  static __device__ __forceinline__ void run(Blk B, const Geo& g, int Teff, int solver, const RiemannDirs& r) {
+    if (B.id < r.blocks[0]) {
+      RiemannSd<D, P, 0, 0, EQ, SV>::run(B, g, 0, Teff, solver, r.trace[0], r.bcfix[0], r.Fi[0], nullptr, r.meq[0]);
+      return;
+    }
+    if (D > 1 && B.id < r.blocks[0] + r.blocks[1]) {
+      const Blk b{B.id - r.blocks[0], r.blocks[1]};
+      RiemannSd<D, P, 0, (D > 1 ? 1 : 0), EQ, SV>::run(b, g, 1, Teff, solver, r.trace[1], r.bcfix[1], r.Fi[1], nullptr,
+                                                       r.meq[1]);
+      return;
+    }
+    if (D > 2) {
+      const Blk b{B.id - r.blocks[0] - r.blocks[1], r.blocks[2]};
+      RiemannSd<D, P, 0, (D > 2 ? 2 : 0), EQ, SV>::run(b, g, 2, Teff, solver, r.trace[2], r.bcfix[2], r.Fi[2], nullptr,
+                                                       r.meq[2]);
+    }
+  }
+};
+template <int D, int P, bool EQ, int SV>
+__global__ void __launch_bounds__(128, 4) k_riemann_all(Geo g, int Teff, int solver, RiemannDirs r) {
+  RiemannAll<D, P, EQ, SV>::run(hw_blk(), g, Teff, solver, r);
+}
 // EQ: the form for the well-balanced mode (meq non-null: the equilibrium
 // at the flux points added to every edge state) and the isothermal system;
 // the plain form reads neither
@@ -571,17 +604,24 @@ __global__ void __launch_bounds__(INTERIOR_THREADS) k_interior_ext(Ops op, Geo g
 // ---------------------------------------------------------------------------
 // transverse subcell averaging of the flux points and scatter to the FV face
 // arrays of time node t (src/sd_simulator.py:208-212,
-// src/sdader_simulator.py:310-323).  One thread per (cell, t, fp along d).
+// src/sdader_simulator.py:310-323).  One thread per (direction, cell, t, fp).
 // F_HO layout [t][v][face], faces x-fastest with X_d + 1 along d.
 // ---------------------------------------------------------------------------
+struct FaceArrays {
+  const double* Ffp[3];
+  double* F_HO[3];
+};
 template <int D, int P>
 struct IntegrateFaces {
-static __device__ __forceinline__ void run(Blk B, const Ops& op, const Geo& g, int d, const double* __restrict__ Ffp,
-                                           double* __restrict__ F_HO) {
+static __device__ __forceinline__ void run(Blk B, const Ops& op, const Geo& g, const FaceArrays& fa) {
   using k = K<D, P>;
-  const long long total = g.Nc * g.T * k::nf;
-  const long long tid = B.id * (long long)blockDim.x + threadIdx.x;
-  if (tid >= total) return;
+  const long long total = g.Nc * g.T * k::nf;  // per direction
+  const long long gid = B.id * (long long)blockDim.x + threadIdx.x;
+  if (gid >= D * total) return;
+  const int d = (int)(gid / total);
+  const long long tid = gid - d * total;
+  const double* __restrict__ Ffp = d == 0 ? fa.Ffp[0] : (d == 1 ? fa.Ffp[1] : fa.Ffp[2]);
+  double* __restrict__ F_HO = d == 0 ? fa.F_HO[0] : (d == 1 ? fa.F_HO[1] : fa.F_HO[2]);
   const long long c = tid % g.Nc;
   const long long r = tid / g.Nc;
   const int f = (int)(r % k::nf);
@@ -599,6 +639,7 @@ static __device__ __forceinline__ void run(Blk B, const Ops& op, const Geo& g, i
     if (e == d) continue;
     if (o0 < 0) o0 = e; else o1 = e;
   }
+#pragma unroll 1
   for (int v = 0; v < k::V; ++v) {
     double G[k::NJ];
 #pragma unroll
@@ -648,8 +689,8 @@ static __device__ __forceinline__ void run(Blk B, const Ops& op, const Geo& g, i
 }
 };
 template <int D, int P>
-__global__ void k_integrate_faces(Ops op, Geo g, int d, const double* __restrict__ Ffp, double* __restrict__ F_HO) {
-  IntegrateFaces<D, P>::run(hw_blk(), op, g, d, Ffp, F_HO);
+__global__ void k_integrate_faces(Ops op, Geo g, FaceArrays fa) {
+  IntegrateFaces<D, P>::run(hw_blk(), op, g, fa);
 }
 
 // ---------------------------------------------------------------------------

@@ -126,22 +126,23 @@ struct Stepper : StepperBase {
       while (cells > 4 && (C->geo.Nc + cells - 1) / cells < 2 * SMS) cells /= 2;
     return cells;
   }
-  // the Riemann problems of one Picard iteration, one instantiation per
-  // direction; EQ: the form with the well-balanced mode's equilibrium edge
+  // the Riemann problems of one Picard iteration; EQ: the form with the well-balanced mode's equilibrium edge
   // values and the isothermal system
-  template <bool EQ, int DIR, int SV>
-  void riemann_dir(spd_ctx* C, unsigned nb, int Teff, int solver) {
-    unsigned* no_tape = nullptr;
-    const double* meq = C->Meq_fp[DIR];
-    launch<RiemannSd<D, P, 0, DIR, EQ, SV>>(C, "k_riemann_sd", k_riemann_sd<D, P, 0, DIR, EQ, SV>, nb, 128, 0, C->geo,
-                                            DIR, Teff, solver, C->trace[DIR], C->bcfix[DIR], C->Fi[DIR], no_tape,
-                                            meq);
-  }
   template <bool EQ, int SV>
-  void riemann_plain(spd_ctx* C, int d, unsigned nb, int Teff, int solver) {
-    if (d == 0) riemann_dir<EQ, 0, SV>(C, nb, Teff, solver);
-    else if (d == 1) riemann_dir<EQ, (D > 1 ? 1 : 0), SV>(C, nb, Teff, solver);
-    else riemann_dir<EQ, (D > 2 ? 2 : 0), SV>(C, nb, Teff, solver);
+  void riemann_all(spd_ctx* C, int Teff) {
+    const Geo& g = C->geo;
+    RiemannDirs r{};
+    unsigned nb = 0;
+    for (int d = 0; d < D; ++d) {
+      r.trace[d] = C->trace[d];
+      r.bcfix[d] = C->bcfix[d];
+      r.Fi[d] = C->Fi[d];
+      r.meq[d] = C->Meq_fp[d];
+      r.blocks[d] = blocks_for((long long)Teff * k::NJ * n_iface(g, d), 128);
+      nb += r.blocks[d];
+    }
+    launch<RiemannAll<D, P, EQ, SV>>(C, "k_riemann_sd", k_riemann_all<D, P, EQ, SV>, nb, 128, 0, g, Teff,
+                                     C->cfg.riemann_solver_sd, r);
   }
 
   // the Riemann problems of one Picard iteration with every branch taped
@@ -179,24 +180,20 @@ struct Stepper : StepperBase {
     for (int it = 0; it <= m; ++it) {
       const int Teff = (it == 0) ? 1 : C->T;
       const int solver = C->cfg.riemann_solver_sd;
-      for (int d = 0; d < D; ++d) {
-        const long long tot = (long long)Teff * k::NJ * n_iface(g, d);
-        {
-          ProfScope ps_(C, "k_riemann_sd");
-          if (C->tape_mode == 0) {
-            const unsigned nb = blocks_for(tot, 128);
-            if (C->Meq_fp[d] || C->cfg.isothermal) riemann_plain<true, -1>(C, d, nb, Teff, solver);
-            else if (C->brec && !C->brec->one_sd) riemann_plain<false, -1>(C, d, nb, Teff, solver);
-            else if (solver == RS_LLF) riemann_plain<false, RS_LLF>(C, d, nb, Teff, solver);
-            else riemann_plain<false, RS_HLLC>(C, d, nb, Teff, solver);
-          } else {
-            unsigned* tp = C->tape_rs[d] + ((size_t)C->tape_step * C->T + it) * C->T * k::NJ * n_iface(g, d);
-            if (C->tape_mode == 1)
-              riemann_taped<1>(C, d, blocks_for(tot, 128), Teff, solver, tp);
-            else
-              riemann_taped<2>(C, d, blocks_for(tot, 128), Teff, solver, tp);
-          }
-        }
+      if (C->tape_mode == 0) {
+        ProfScope ps_(C, "k_riemann_sd");
+        if (C->Meq_fp[0] || C->cfg.isothermal) riemann_all<true, -1>(C, Teff);
+        else if (C->brec && !C->brec->one_sd) riemann_all<false, -1>(C, Teff);
+        else if (solver == RS_LLF) riemann_all<false, RS_LLF>(C, Teff);
+        else riemann_all<false, RS_HLLC>(C, Teff);
+        CKL();
+      }
+      for (int d = 0; d < D && C->tape_mode != 0; ++d) {
+        const unsigned nb = blocks_for((long long)Teff * k::NJ * n_iface(g, d), 128);
+        unsigned* tp = C->tape_rs[d] + ((size_t)C->tape_step * C->T + it) * C->T * k::NJ * n_iface(g, d);
+        ProfScope ps_(C, "k_riemann_sd");
+        if (C->tape_mode == 1) riemann_taped<1>(C, d, nb, Teff, solver, tp);
+        else riemann_taped<2>(C, d, nb, Teff, solver, tp);
         CKL();
       }
       const int mode = (it < m) ? 0 : final_mode;
@@ -275,8 +272,6 @@ struct Stepper : StepperBase {
 
   int cmax(spd_ctx* C) override {
     const Geo& g = C->geo;
-    CK(zero_fill(C, C->flags + 1, sizeof(int)));
-    CK(zero_fill(C, C->counts + 2, sizeof(unsigned long long)));
     {
       ProfScope ps_(C, "k_cmax_only");
       launch<CmaxOnly<D, P>>(C, "k_cmax_only", k_cmax_only<D, P>, blocks_for(g.Nq, BS), BS, 0, g, C->W_cv,
@@ -307,16 +302,17 @@ struct Stepper : StepperBase {
     const spd_config& cf = C->cfg;
     // switch_to_finite_volume (src/sdader_simulator.py:288-298)
     if (int r = sp_to_cv(C)) return r;
-    for (int d = 0; d < D; ++d) {
-      {
-        ProfScope ps_(C, "k_integrate_faces");
-        launch<IntegrateFaces<D, P>>(C, "k_integrate_faces", k_integrate_faces<D, P>,
-                                     blocks_for(g.Nc * g.T * k::nf, 128), 128, 0, C->ops, g, d, C->Ffp[d], C->F_HO[d]);
-      }
-      CKL();
+    {
+      ProfScope ps_(C, "k_integrate_faces");
+      const FaceArrays fa{{C->Ffp[0], C->Ffp[1], C->Ffp[2]}, {C->F_HO[0], C->F_HO[1], C->F_HO[2]}};
+      launch<IntegrateFaces<D, P>>(C, "k_integrate_faces", k_integrate_faces<D, P>,
+                                   blocks_for(D * g.Nc * g.T * k::nf, 128), 128, 0, C->ops, g, fa);
     }
+    CKL();
     long long nface[3] = {1, 1, 1};
     for (int d = 0; d < D; ++d) nface[d] = n_faces(g, d);
+    const BcBufs bc{{C->bcbuf[0], C->bcbuf[1], C->bcbuf[2]}};
+    const Counters counters{C->flags, C->counts};
     for (int i = 0; i < C->T; ++i) {
       const double w_i = C->ops.w_tp[i];
       if (C->recording)
@@ -328,7 +324,8 @@ struct Stepper : StepperBase {
         ProfScope ps_(C, "k_fv_candidate");
         launch<FvCandidate<D>>(C, "k_fv_candidate", k_fv_candidate<D>, blocks_for(g.Nq, BS), BS, 0, g, C->fvg, C->dt,
                                w_i, FH[0], FH[1], FH[2], C->U_cv, C->U_new, C->ext_old, C->ext_new,
-                               cf.FB ? (i == 0 ? 1 : 2) : 0, (const double*)C->gphi_fv, (const double*)C->Ueq_cv,
+                               cf.FB ? (i == 0 ? 1 : 2) : 0, bc, counters, i == C->T - 1 ? C->W_cv : nullptr,
+                               (const double*)C->gphi_fv, (const double*)C->Ueq_cv,
                                (const double*)C->Weq_cv);
       }
       CKL();
@@ -340,17 +337,9 @@ struct Stepper : StepperBase {
                              C->stream));
           off += (size_t)nface[d];
         }
-        for (int d = 0; d < D; ++d) {
-          if (int r = ghost(C, d, 1, k::V, C->ext_old, nullptr)) return r;
-        }
       } else if (cf.FB) {
         // detect_troubles (src/trouble_detection.py:5-87)
-        for (int d = 0; d < D; ++d) {
-          if (int r = ghost(C, d, 1, k::V, C->ext_old, nullptr)) return r;
-        }
         const int sed = (P > 1 && cf.SED) ? 1 : 0;
-        CK(zero_fill(C, C->flags, sizeof(int)));
-        if (sed) CK(zero_fill(C, C->counts + 3, sizeof(unsigned long long)));
         {
           ProfScope ps_(C, "k_nad");
           long long* sed_list = sed ? C->list_sed : nullptr;
@@ -359,9 +348,6 @@ struct Stepper : StepperBase {
         }
         CKL();
         if (sed) {
-          for (int d = 0; d < D; ++d) {
-            if (int r = ghost(C, d, 1, k::V, C->ext_new, C->flags)) return r;
-          }
           ProfScope ps_(C, "k_sed");
           const unsigned nb = (unsigned)std::min<long long>(PERSIST_BLOCKS, blocks_for(2 * g.Nq, BS));
           launch<Sed<D>>(C, "k_sed", k_sed<D>, nb, BS, 0, g, C->fvg, C->list_sed, C->counts + 3, C->ext_new,
@@ -371,13 +357,10 @@ struct Stepper : StepperBase {
         {
           ProfScope ps_(C, "k_troubles");
           launch<Troubles<D>>(C, "k_troubles", k_troubles<D>, blocks_for(g.Nq, BS), BS, 0, g, cf.PAD, cf.min_rho,
-                              cf.max_rho, cf.min_P, C->mask, C->ext_new, C->theta_src, C->troubles,
-                              (const double*)C->Weq_cv);
+                              cf.max_rho, cf.min_P, C->mask, (const int*)C->flags, sed, (const double*)C->ext_old,
+                              C->ext_new, bc, C->theta_src, C->troubles, (const double*)C->Weq_cv);
         }
         CKL();
-        for (int d = 0; d < D; ++d) {
-          if (int r = ghost(C, d, 0, 1, C->theta_src, nullptr)) return r;
-        }
         double* th = C->theta_src;
         if (cf.blending) {
           {
@@ -386,46 +369,28 @@ struct Stepper : StepperBase {
                                        C->theta_src, C->theta_a);
           }
           CKL();
-          double* in = C->theta_a;
-          double* out = C->theta_b;
-          for (int d = 0; d < D; ++d) {
-            {
-              ProfScope ps_(C, "k_blend_last");
-              launch<BlendLast<D>>(C, "k_blend_last", k_blend_last<D>, blocks_for(g.Nqe, BS), BS, 0, g, d, in, out);
-            }
-            CKL();
-            std::swap(in, out);
+          {
+            ProfScope ps_(C, "k_blend_last");
+            launch<BlendLast<D>>(C, "k_blend_last", k_blend_last<D>, blocks_for(g.Nqe, BS), BS, 0, g, C->theta_a,
+                                 C->theta_b);
           }
-          th = in;
+          CKL();
+          th = C->theta_b;
         }
         C->theta_final = th;
       }
       if (cf.FB) {
         // affected faces, marks and the fallback fluxes (src/sdader_simulator.py:343-346)
-        CK(zero_fill(C, C->mark_cell, (size_t)g.Nqe));
-        CK(zero_fill(C, C->mark_q, (size_t)g.Nq));
-        CK(zero_fill(C, C->counts, 2 * sizeof(unsigned long long)));
-        CK(zero_fill(C, C->counts + 4, D * sizeof(unsigned long long)));
-        for (int d = 0; d < D; ++d) {
-          {
-            ProfScope ps_(C, "k_affected");
-            const double* th = C->tape_mode == 2 ? nullptr : C->theta_final;
-            launch<Affected<D>>(C, "k_affected", k_affected<D>, blocks_for(nface[d], BS), BS, 0, g, d, cf.godunov, th,
-                                C->aff[d], C->mark_cell, C->mark_q, C->flags + 2, C->list_face[d],
-                                C->counts + 4 + d);
-          }
-          CKL();
-        }
         {
-          ProfScope ps_(C, "k_compact");
-          launch<Compact>(C, "k_compact", k_compact, blocks_for(g.Nqe, BS), BS, 0, g.Nqe, C->mark_cell, C->list_cell,
-                          C->counts);
-        }
-        CKL();
-        {
-          ProfScope ps_(C, "k_compact");
-          launch<Compact>(C, "k_compact", k_compact, blocks_for(g.Nq, BS), BS, 0, g.Nq, C->mark_q, C->list_q,
-                          C->counts + 1);
+          ProfScope ps_(C, "k_affected_all");
+          const double* th = C->tape_mode == 2 ? nullptr : C->theta_final;
+          const AffectedOut out{{C->aff[0], C->aff[1], C->aff[2]},
+                                {C->list_face[0], C->list_face[1], C->list_face[2]},
+                                C->list_cell,
+                                C->list_q,
+                                C->counts};
+          launch<AffectedAll<D>>(C, "k_affected_all", k_affected_all<D>, blocks_for(g.Nqe, BS), BS, 0, g, cf.godunov,
+                                 th, out);
         }
         CKL();
         if (C->tape_mode == 1) {
@@ -444,40 +409,30 @@ struct Stepper : StepperBase {
           CK(cudaMemcpyAsync(dst, C->Mpred, sizeof(double) * nq, cudaMemcpyDeviceToDevice, C->stream));
           CK(cudaMemcpyAsync(dst + nq, C->S, sizeof(double) * D * nq, cudaMemcpyDeviceToDevice, C->stream));
         }
-        for (int d = 0; d < D; ++d) {
-          {
-            ProfScope ps_(C, "k_muscl_faces");
-            // grid-stride over the compacted list of affected faces
-            const unsigned nb = (unsigned)std::min<long long>(PERSIST_BLOCKS, blocks_for(nface[d], BS));
-            const unsigned long long* fcount = C->counts + 4 + d;
-            if (C->tape_mode == 0) {
-              constexpr int D1 = (D > 1 ? 1 : 0), D2 = (D > 2 ? 2 : 0);
-              if (C->brec && !C->brec->one_fv) {
-                if (d == 0) muscl_faces<0, -1>(C, nb, fcount);
-                else if (d == 1) muscl_faces<D1, -1>(C, nb, fcount);
-                else muscl_faces<D2, -1>(C, nb, fcount);
-              } else if (cf.riemann_solver_fv == RS_LLF) {
-                if (d == 0) muscl_faces<0, RS_LLF>(C, nb, fcount);
-                else if (d == 1) muscl_faces<D1, RS_LLF>(C, nb, fcount);
-                else muscl_faces<D2, RS_LLF>(C, nb, fcount);
-              } else {
-                if (d == 0) muscl_faces<0, RS_HLLC>(C, nb, fcount);
-                else if (d == 1) muscl_faces<D1, RS_HLLC>(C, nb, fcount);
-                else muscl_faces<D2, RS_HLLC>(C, nb, fcount);
-              }
-            } else {
-              unsigned* tp = C->tape_fb[d] + ((size_t)C->tape_step * C->T + i) * nface[d];
-              if (C->tape_mode == 1)
-                k_muscl_faces<D, 1><<<nb, BS, 0, C->stream>>>(g, d, cf.riemann_solver_fv, C->list_face[d], fcount,
-                                                             C->Mpred, C->S, C->F_FB[d], tp, nullptr, nullptr);
-              else
-                k_muscl_faces<D, 2><<<nb, BS, 0, C->stream>>>(g, d, cf.riemann_solver_fv, C->list_face[d], fcount,
-                                                             C->Mpred, C->S, C->F_FB[d], tp, nullptr, nullptr);
-            }
-          }
+        long long nface_all = 0;
+        for (int d = 0; d < D; ++d) nface_all += nface[d];
+        if (C->tape_mode == 0) {
+          ProfScope ps_(C, "k_muscl_faces");
+          const unsigned nb = (unsigned)std::min<long long>(PERSIST_BLOCKS, blocks_for(nface_all, 128));
+          if (C->brec && !C->brec->one_fv) muscl_faces<-1>(C, nb);
+          else if (cf.riemann_solver_fv == RS_LLF) muscl_faces<RS_LLF>(C, nb);
+          else muscl_faces<RS_HLLC>(C, nb);
           CKL();
         }
-        k_fv_correct_grid(C, w_i, FH, C->ext_new);
+        for (int d = 0; d < D && C->tape_mode != 0; ++d) {
+          ProfScope ps_(C, "k_muscl_faces");
+          const unsigned nb = (unsigned)std::min<long long>(PERSIST_BLOCKS, blocks_for(nface[d], BS));
+          const unsigned long long* fcount = C->counts + 4 + d;
+          unsigned* tp = C->tape_fb[d] + ((size_t)C->tape_step * C->T + i) * nface[d];
+          if (C->tape_mode == 1)
+            k_muscl_faces<D, 1><<<nb, BS, 0, C->stream>>>(g, d, cf.riemann_solver_fv, C->list_face[d], fcount,
+                                                         C->Mpred, C->S, C->F_FB[d], tp, nullptr, nullptr);
+          else
+            k_muscl_faces<D, 2><<<nb, BS, 0, C->stream>>>(g, d, cf.riemann_solver_fv, C->list_face[d], fcount,
+                                                         C->Mpred, C->S, C->F_FB[d], tp, nullptr, nullptr);
+          CKL();
+        }
+        k_fv_correct_grid(C, w_i, FH, i == C->T - 1 ? C->W_cv : nullptr);
         CKL();
         C->fb_ran = true;
         if (C->recording) {
@@ -503,12 +458,15 @@ struct Stepper : StepperBase {
     return 0;
   }
 
-  template <int DIR, int SV>
-  void muscl_faces(spd_ctx* C, unsigned nb, const unsigned long long* fcount) {
-    unsigned* no_tape = nullptr;
-    launch<MusclFaces<D, 0, DIR, SV>>(C, "k_muscl_faces", k_muscl_faces<D, 0, DIR, SV>, nb, BS, 0, C->geo, DIR,
-                                  C->cfg.riemann_solver_fv, C->list_face[DIR], fcount, C->Mpred, C->S, C->F_FB[DIR],
-                                  no_tape, (const double*)C->Meq_faces[DIR], (const double*)C->Feq_faces[DIR]);
+  template <int SV>
+  void muscl_faces(spd_ctx* C, unsigned nb) {
+    const FaceLists fl{{C->list_face[0], C->list_face[1], C->list_face[2]},
+                       C->counts + 4,
+                       {C->F_FB[0], C->F_FB[1], C->F_FB[2]},
+                       {C->Meq_faces[0], C->Meq_faces[1], C->Meq_faces[2]},
+                       {C->Feq_faces[0], C->Feq_faces[1], C->Feq_faces[2]}};
+    launch<MusclFacesAll<D, SV>>(C, "k_muscl_faces", k_muscl_faces_all<D, SV>, nb, 128, 0, C->geo,
+                                 C->cfg.riemann_solver_fv, fl, C->Mpred, C->S);
   }
 
   void k_muscl_cells_grid(spd_ctx* C, double w_i, int i) {
@@ -533,32 +491,16 @@ struct Stepper : StepperBase {
                                                                nullptr, nullptr);
   }
 
-  // ext_new non-null: also the primitives of the corrected subcells (the
-  // next substep's W_old, or the step's W_cv after the last substep)
-  void k_fv_correct_grid(spd_ctx* C, double w_i, const double* const* FH, double* ext_new) {
+  void k_fv_correct_grid(spd_ctx* C, double w_i, const double* const* FH, double* W_cv) {
     const Geo& g = C->geo;
     const long long nb = std::min<long long>(PERSIST_BLOCKS, blocks_for(g.Nq, 128));
     {
       ProfScope ps_(C, "k_fv_correct");
       launch<FvCorrect<D>>(C, "k_fv_correct", k_fv_correct<D>, (unsigned)nb, 128, 0, g, C->fvg, C->dt, w_i,
                            C->cfg.godunov, C->list_q, C->counts + 1, FH[0], FH[1], FH[2], C->F_FB[0], C->F_FB[1],
-                           C->F_FB[2], C->aff[0], C->aff[1], C->aff[2], C->U_cv, C->U_new, ext_new,
+                           C->F_FB[2], C->aff[0], C->aff[1], C->aff[2], C->U_cv, C->U_new, C->ext_new, W_cv,
                            (const double*)C->gphi_fv, (const double*)C->Ueq_cv, (const double*)C->Weq_cv);
     }
-  }
-
-  int ghost(spd_ctx* C, int d, int all, int nv, double* ext, const int* gate) {
-    const Geo& g = C->geo;
-    const int o0 = (d == 0) ? 1 : 0;
-    const int o1 = (d == 2) ? 1 : 2;
-    const long long tot = 2LL * nv * NGH * g.Xe[o0] * g.Xe[o1];
-    {
-      ProfScope ps_(C, "k_ghost");
-      launch<Ghost<D>>(C, "k_ghost", k_ghost<D>, blocks_for(tot, BS), BS, 0, g, d, all, nv, k::V, ext, C->bcbuf[d],
-                       gate);
-    }
-    CKL();
-    return 0;
   }
 
   // adjoint of the recorded step (spd_adjoint_exec.cuh, compiled in its own
@@ -611,18 +553,9 @@ struct Stepper : StepperBase {
     if (int r = predictor(C, final_mode)) return r;
     if (C->cfg.update == SPD_UPDATE_FV) {
       if (int r = fv_update(C)) return r;
-      if (C->cfg.FB) {
-        // W_cv = prim(U_cv) (src/sdader_simulator.py:376): ext_new already
-        // holds it (the last substep's W_new, refreshed where corrected)
-        const Geo& g = C->geo;
-        {
-          ProfScope ps_(C, "k_ext_to_plain");
-          launch<ExtToPlain<D>>(C, "k_ext_to_plain", k_ext_to_plain<D>, blocks_for(g.Nq, BS), BS, 0, g, C->ext_new,
-                                C->W_cv);
-        }
-        CKL();
-        return 0;
-      }
+      // W_cv = prim(U_cv) (src/sdader_simulator.py:376): written by the last
+      // substep's candidate and corrected updates
+      if (C->cfg.FB) return 0;
     }
     // W_cv = prim(U_cv) (src/sdader_simulator.py:376)
     return wcv(C);
