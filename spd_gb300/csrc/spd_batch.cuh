@@ -81,6 +81,7 @@ __host__ __device__ __forceinline__ int instance_of(const unsigned* __restrict__
 
 template <class Body, class... A>
 __global__ void k_batched(const Pack<A...>* __restrict__ packs, const unsigned* __restrict__ boff, int n) {
+  spd::step_kernel_begin();
   const int i = instance_of(boff, n, blockIdx.x);
   pack_call<Body>(Blk{blockIdx.x - boff[i], boff[i + 1] - boff[i]}, packs[i]);
 }
@@ -93,6 +94,7 @@ struct ZeroRange {
 // zero-fills of many instances' buffers in one launch: head bytes up to an
 // 8-byte boundary, 8-byte words, tail bytes
 static __global__ void k_zero_ranges(const ZeroRange* __restrict__ r, const unsigned* __restrict__ boff, int n) {
+  spd::step_kernel_begin();
   const int i = instance_of(boff, n, blockIdx.x);
   const ZeroRange z = r[i];
   const unsigned long long t = (unsigned long long)(blockIdx.x - boff[i]) * blockDim.x + threadIdx.x;
@@ -111,6 +113,24 @@ static __global__ void k_zero_ranges(const ZeroRange* __restrict__ r, const unsi
 // ---------------------------------------------------------------------------
 // host: launch sites and the recorder
 // ---------------------------------------------------------------------------
+#ifdef __CUDACC__
+// launch of a kernel that begins with step_kernel_begin
+template <class... P, class... A>
+cudaError_t launch_step(cudaStream_t s, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, A&&... a) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kern, std::forward<A>(a)...);
+}
+#endif
+
 constexpr unsigned MAX_GRID = 0x7fffffffu;
 
 struct SiteBase {
@@ -155,8 +175,7 @@ struct Site : SiteBase {
   }
   cudaError_t launch(cudaStream_t s) override {
     if (boff.back() == 0) return cudaSuccess;
-    k_batched<Body, A...><<<boff.back(), block, smem, s>>>(d_packs, d_boff, count());
-    return cudaGetLastError();
+    return launch_step(s, k_batched<Body, A...>, dim3(boff.back()), block, smem, d_packs, d_boff, count());
   }
 };
 
@@ -175,8 +194,7 @@ struct ZeroSite : SiteBase {
   }
   cudaError_t launch(cudaStream_t s) override {
     if (boff.back() == 0) return cudaSuccess;
-    k_zero_ranges<<<boff.back(), block, 0, s>>>(d_ranges, d_boff, count());
-    return cudaGetLastError();
+    return launch_step(s, k_zero_ranges, dim3(boff.back()), block, 0, d_ranges, d_boff, count());
   }
 };
 #endif

@@ -43,10 +43,14 @@ __global__ void k_sd_layout(Geo g, int D, int n, int V, const double* __restrict
   else dst[r] = src[di];
 }
 
-__global__ void k_time_add_dev(double* t, const double* dt) { *t = *t + *dt; }
+__global__ void k_time_add_dev(double* t, const double* dt) {
+  step_kernel_begin();
+  *t = *t + *dt;
+}
 // perform_time_evolution's clip (src/sdader_simulator.py:406-409) on the
 // device: t[0] = time, t[1] = t_end
 __global__ void k_clip_dt(const double* t, double* dt) {
+  step_kernel_begin();
   const double d = *dt;
   if (t[0] + d >= t[1]) *dt = t[1] - t[0];
 }
@@ -787,15 +791,13 @@ static bool capture(spd_ctx* C, int part, spd_ctx::StepGraph* out) {
   if (part != 1) {
     rc = C->stepper->cmax(C);
     if (!rc) {
-      k_clip_dt<<<1, 1, 0, s>>>(C->t_dev, C->dt);
-      if (cudaGetLastError() != cudaSuccess) rc = SPD_ERR_CUDA;
+      if (spd_batch::launch_step(s, k_clip_dt, 1, 1, 0, C->t_dev, C->dt) != cudaSuccess) rc = SPD_ERR_CUDA;
     }
   }
   if (part != 0 && !rc) {
     rc = C->stepper->update(C);
     if (!rc) {
-      k_time_add_dev<<<1, 1, 0, s>>>(C->t_dev, C->dt);
-      if (cudaGetLastError() != cudaSuccess) rc = SPD_ERR_CUDA;
+      if (spd_batch::launch_step(s, k_time_add_dev, 1, 1, 0, C->t_dev, C->dt) != cudaSuccess) rc = SPD_ERR_CUDA;
     }
   }
   cudaGraph_t g = nullptr;

@@ -192,7 +192,8 @@ void launch(spd_ctx* C, const char* name, void (*kern)(P...), dim3 grid, dim3 bl
     C->brec->add<Body>(name, grid, block, smem, spd_batch::PackBuild<P...>::make(std::forward<A>(a)...));
     return;
   }
-  kern<<<grid, block, smem, C->stream>>>(std::forward<A>(a)...);
+  // an error is seen by the caller's cudaGetLastError
+  spd_batch::launch_step(C->stream, kern, grid, block, smem, std::forward<A>(a)...);
 }
 
 // zero-fill of device bytes on the context's stream (recorded while a batch

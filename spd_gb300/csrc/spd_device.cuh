@@ -28,7 +28,22 @@ struct Blk {
   unsigned id, n;
 };
 #ifdef __CUDACC__
-__device__ __forceinline__ Blk hw_blk() { return Blk{blockIdx.x, gridDim.x}; }
+// Start of a kernel of the step.  The step's kernels are launched with
+// programmatic stream serialization (launch_step): a kernel may become
+// resident while the one before it drains, waits here until that one's writes
+// are visible, and then lets the next one be brought up.  A step of a 32^2
+// grid is about 56 dependent kernels of 2-5 us, so what lies between them
+// counts.  In a plain launch both instructions do nothing.
+__device__ __forceinline__ void step_kernel_begin() {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#endif
+}
+__device__ __forceinline__ Blk hw_blk() {
+  step_kernel_begin();
+  return Blk{blockIdx.x, gridDim.x};
+}
 #endif
 
 enum Riemann : int { RS_LLF = 0, RS_HLLC = 1, RS_LHLLC = 2 };

@@ -171,11 +171,21 @@ __device__ __forceinline__ long long bc_entry(const Geo& g, int d, int side, int
 struct BcBufs {
   double* b[3];
 };
-// the primitives W of the active subcell a into the ghosts it owns
+// whether an active subcell owns any ghost
 template <int D>
-__device__ __forceinline__ void write_ghosts(const Geo& g, const BcBufs& bc, const int* a, const double* W,
-                                             double* __restrict__ ext) {
+__device__ __forceinline__ bool near_side(const Geo& g, int ix, int iy, int iz) {
+  bool any = ix < NGH || ix >= g.X[0] - NGH;
+  if (D > 1) any = any || iy < NGH || iy >= g.X[1] - NGH;
+  if (D > 2) any = any || iz < NGH || iz >= g.X[2] - NGH;
+  return any;
+}
+// the primitives W of an active subcell into the ghosts it owns; out of line,
+// because few subcells own any
+template <int D>
+__device__ __noinline__ void write_ghosts(const Geo& g, const BcBufs& bc, int ix, int iy, int iz, const double* W,
+                                          double* __restrict__ ext) {
   constexpr int V = D + 2;
+  const int a[3] = {ix, iy, iz};
   for_ghosts<D>(g, a, [&](const int* e, const int* choice) {
     double w[V];
 #pragma unroll
@@ -264,12 +274,22 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, const FvGeo& fg,
     }
 #pragma unroll
     for (int v = 0; v < V; ++v) ext_old[(long long)v * g.Nqe + e] = W[v];
-    const int a[3] = {ix, iy, iz};
-    write_ghosts<D>(g, bc, a, W, ext_old);
+    const bool side = near_side<D>(g, ix, iy, iz);
+    if (side) {
+      double w[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) w[v] = W[v];
+      write_ghosts<D>(g, bc, ix, iy, iz, w, ext_old);
+    }
     prims_cv<D>(g, un, W, Ueq, Weq, q);
 #pragma unroll
     for (int v = 0; v < V; ++v) ext_new[(long long)v * g.Nqe + e] = W[v];
-    write_ghosts<D>(g, bc, a, W, ext_new);
+    if (side) {
+      double w[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) w[v] = W[v];
+      write_ghosts<D>(g, bc, ix, iy, iz, w, ext_new);
+    }
     if (W_cv != nullptr) {
 #pragma unroll
       for (int v = 0; v < V; ++v) W_cv[(long long)v * g.Nq + q] = W[v];
@@ -278,10 +298,10 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, const FvGeo& fg,
 }
 };
 template <int D>
-__global__ void k_fv_candidate(Geo g, FvGeo fg, const double* __restrict__ dt_ptr, double w_i,
+__global__ void k_fv_candidate(const __grid_constant__ Geo g, FvGeo fg, const double* __restrict__ dt_ptr, double w_i,
                                const double* F0, const double* F1, const double* F2,
                                const double* __restrict__ U_cv, double* __restrict__ U_new, double* ext_old,
-                               double* ext_new, int write_ext, BcBufs bc, Counters ct,
+                               double* ext_new, int write_ext, const __grid_constant__ BcBufs bc, Counters ct,
                                double* __restrict__ W_cv, const double* __restrict__ gphi, const double* __restrict__ Ueq,
                                const double* __restrict__ Weq) {
   FvCandidate<D>::run(hw_blk(), g, fg, dt_ptr, w_i, F0, F1, F2, U_cv, U_new, ext_old, ext_new, write_ext, bc, ct, W_cv,
