@@ -15,7 +15,7 @@ template <int D, int P>
 int adj_traces_of(spd_ctx* C, const double* U, int Tu, int Teff) {
   const Geo& g = C->geo;
   ProfScope ps_(C, "k_adj_traces_fwd");
-  k_traces_ader<D, P><<<blocks_for(g.Nc * (D * K<D, P>::NJ) * Teff, 128), 128, 0, C->stream>>>(C->ops, g, U, Tu, Teff, C->trace[0],
+  k_traces_ader<D, P><<<blocks_for(g.Nc * (D * K<D, P>::NJ * K<D, P>::V) * Teff, 128), 128, 0, C->stream>>>(C->ops, g, U, Tu, Teff, C->trace[0],
                                                                           C->trace[1], C->trace[2]);
   CKL();
   return 0;

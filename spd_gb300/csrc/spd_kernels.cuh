@@ -16,8 +16,10 @@
 
 namespace spd {
 
-// threads per block of the interior kernel at most
-constexpr int INTERIOR_THREADS = 512;
+// threads per block of the interior kernel, and its blocks per SM: their
+// barriers overlap
+constexpr int INTERIOR_THREADS = 256;
+constexpr int INTERIOR_BLOCKS = 3;
 
 struct Ops {
   double sp_to_fp[MAXNF * MAXN];
@@ -95,37 +97,33 @@ __host__ __device__ __forceinline__ long long n_iface(const Geo& g, int d) {
 }
 
 // ---------------------------------------------------------------------------
-// edge traces of one line along DIR: sp -> fp 0 and fp nf-1
-// (src/sdader_simulator.py:220, src/transforms.py:3-25).  ``at(v, s)`` gives
-// variable v at solution point s.
+// edge traces of one variable on one line along d: sp -> fp 0 and fp nf-1
+// (src/sdader_simulator.py:220, src/transforms.py:3-25).  ``at(s)`` gives the
+// variable at solution point s; LANES2: d is x.
 // ---------------------------------------------------------------------------
 template <int D, int P, bool LANES2, class At>
 __device__ __forceinline__ void trace_line(const Ops& op, const Geo& g, At at, long long c, double* trace, int t_out,
-                                           int d, int j) {
+                                           int d, int j, int v) {
   using k = K<D, P>;
-  // one variable at a time, rolled: the products are inlined (spd_soft.cuh),
-  // and the loop keeps the kernel in the instruction cache
-#pragma unroll 1
-  for (int v = 0; v < k::V; ++v) {
-    Line<k::n> ln;
+  Line<k::n> ln;
 #pragma unroll
-    for (int s = 0; s < k::n; ++s) ln.v[s] = at(v, sp_index<D, P>(d, j, s));
-    line_ready<k::n>(ln, op.soft);
-    double e[2];
-    line_apply<k::n, 2, LANES2>(op.c_sp_to_fp, 0, k::nf - 1, ln, e);
-    trace[(((long long)(0 * k::V + v) * g.T + t_out) * k::NJ + j) * g.Nc + c] = e[0];
-    trace[(((long long)(1 * k::V + v) * g.T + t_out) * k::NJ + j) * g.Nc + c] = e[1];
-  }
+  for (int s = 0; s < k::n; ++s) ln.v[s] = at(sp_index<D, P>(LANES2 ? 0 : d, j, s));
+  line_ready<k::n>(ln, op.soft);
+  double e[2];
+  line_apply<k::n, 2, LANES2>(op.c_sp_to_fp, 0, k::nf - 1, ln, e);
+  trace[(((long long)(0 * k::V + v) * g.T + t_out) * k::NJ + j) * g.Nc + c] = e[0];
+  trace[(((long long)(1 * k::V + v) * g.T + t_out) * k::NJ + j) * g.Nc + c] = e[1];
 }
-// traces of line r = d*NJ + j of time node tu of an iterate U (Tu stored)
+// traces of item r = (d*NJ + j)*V + v of time node tu of an iterate U (Tu
+// stored); D*NJ*V items
 template <int D, int P>
 __device__ __forceinline__ void write_trace(const Ops& op, const Geo& g, const double* __restrict__ U, int Tu, int tu,
                                             long long c, int r, double* t0, double* t1, double* t2, int t_out) {
   using k = K<D, P>;
-  auto at = [&](int v, int s) { return U[(((long long)v * Tu + tu) * k::NS + s) * g.Nc + c]; };
-  const int d = r / k::NJ;
-  if (d == 0) trace_line<D, P, true>(op, g, at, c, t0, t_out, 0, r % k::NJ);
-  else trace_line<D, P, false>(op, g, at, c, d == 1 ? t1 : t2, t_out, d, r % k::NJ);
+  const int v = r % k::V, j = r / k::V % k::NJ, d = r / (k::V * k::NJ);
+  auto at = [&](int s) { return U[(((long long)v * Tu + tu) * k::NS + s) * g.Nc + c]; };
+  if (d == 0) trace_line<D, P, true>(op, g, at, c, t0, t_out, 0, j, v);
+  else trace_line<D, P, false>(op, g, at, c, d == 1 ? t1 : t2, t_out, d, j, v);
 }
 
 // Every kernel of the step is a body ``run(Blk, args...)`` plus a plain
@@ -135,9 +133,9 @@ template <int D, int P>
 struct TracesSp {
   static __device__ __forceinline__ void run(Blk B, const Ops& op, const Geo& g, const double* __restrict__ U_sp,
                                              double* t0, double* t1, double* t2) {
-    // one thread per (cell, line)
+    // one thread per (cell, line, variable)
     const long long tid = B.id * (long long)blockDim.x + threadIdx.x;
-    if (tid >= g.Nc * (D * K<D, P>::NJ)) return;
+    if (tid >= g.Nc * (D * K<D, P>::NJ * K<D, P>::V)) return;
     write_trace<D, P>(op, g, U_sp, 1, 0, tid % g.Nc, (int)(tid / g.Nc), t0, t1, t2, 0);
   }
 };
@@ -151,7 +149,7 @@ template <int D, int P>
 __global__ void k_traces_ader(Ops op, Geo g, const double* __restrict__ U, int Tu, int Teff, double* t0, double* t1,
                               double* t2) {
   const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  constexpr int lines = D * K<D, P>::NJ;
+  constexpr int lines = D * K<D, P>::NJ * K<D, P>::V;
   if (tid >= g.Nc * Teff * lines) return;
   const int r = (int)(tid / g.Nc);
   const int t = r / lines;
@@ -318,23 +316,22 @@ __global__ void k_riemann_sd(Geo g, int d_rt, int Teff, int solver, const double
 // the FV update (:288-298).  mode: 0 = Picard (writes U_ader and the next
 // traces), 1 = SD update of U_sp, 2 = write Ffp.
 //
-// Block = CPB cells x rows of threads; a row takes one (time node, line) of
-// the cells at a time.  Shared memory holds the flux derivative of the cells'
-// nodes, [(v*NS + s)*Tn + t][cell], Tn nodes stored, and per thread the
-// states and then fluxes at its line's interior flux points,
-// [v*(nf-2) + f][thread].  Lines of one direction own their points, so a
-// barrier between directions is all the accumulation needs.  Then each row
-// takes (variable, point) pairs: the T values of the derivative are read
-// once, prepared once and contracted into the T new nodes, which replace
-// them, and the lines of the new nodes give the next traces.
+// Block = CPB cells x rows of threads.  Shared memory holds the flux
+// derivative of the cells' nodes, [(v*NS + s)*Tn + t][cell], Tn nodes stored,
+// and, for a chunk of (node, line) pairs, the states and then the fluxes at
+// their interior flux points, [(line*V + v)*(nf-2) + f][cell].  Per direction
+// and chunk the rows take (line, variable) pairs to interpolate, then (line,
+// flux point) pairs for the fluxes, then (line, variable) pairs for the
+// derivative.  In the end they take (variable, point) pairs: the T values of
+// the derivative are read once, prepared once and contracted into the T new
+// nodes, which replace them, and the lines of the new nodes give the next
+// traces.
 //
-// Bound: the FP64 additions beside the integer pipes (spd_soft.cuh).  Rows
-// are lines, not time nodes, because the tile leaves few cells per SM: 2 KB
-// a cell in 2D at degree 3 and 25 KB in 3D at degree 4, where one block of 8
-// cells x 5 nodes was all an SM held.  The loops over variables and
-// directions are rolled, and the per-thread array is in shared memory so that
-// they can be: with every product inlined the unrolled kernel is over 100 KB
-// of instructions.
+// Bound: the FP64 additions beside the integer pipes (spd_soft.cuh).  A row's
+// work is one variable or one point, not a line of all variables, because
+// small grids leave warps to spare (32^2, p=3: a thread per line was 512
+// warps on 608 schedulers) and because with every product inlined the loop
+// bodies have to be few and small.
 // ---------------------------------------------------------------------------
 // EXT: optional terms, each present when its pointer is not null -- the
 // viscous fluxes G[d] (src/sdader_simulator.py:268, layout of Ffp),
@@ -345,90 +342,125 @@ __global__ void k_riemann_sd(Geo g, int d_rt, int Teff, int solver, const double
 template <int D, int P, bool EXT = false>
 struct Interior {
 using k = K<D, P>;
+static constexpr int ni = k::nf - 2;
 struct Args {
   int mode, Teff, Tu, Tn;
   const double* Uin;
   bool visc, wb, iso;
 };
+// the arrays of one direction
+struct Dir {
+  const double* Fi;
+  double* Ffp;
+  const double *Gv, *meq, *feq;
+};
 
-// lines of direction d: fluxes at the flux points, then their derivative
-// into the tile (added to the lower directions') or the flux-point output
+// states at the interior flux points of lines [l0, l1) along d
 template <bool LANES2>
-static __device__ __forceinline__ void lines(const Ops& op, const Geo& g, const Args& a, int dd, long long c,
-                                             double* tile, double* scr, const double* __restrict__ Fi,
-                                             double* __restrict__ Ffp, const double* __restrict__ Gv,
-                                             const double* __restrict__ meq, const double* __restrict__ feq) {
-  const int d = LANES2 ? 0 : dd;
+static __device__ __forceinline__ void interpolate(const Ops& op, const Geo& g, const Args& a, int d, int l0, int l1,
+                                                   long long c, double* scr) {
+  const int CPB = blockDim.x;
+#pragma unroll 1
+  for (int i = threadIdx.y; i < (l1 - l0) * k::V; i += (int)blockDim.y) {
+    const int v = i % k::V, line = l0 + i / k::V;
+    const int t = line / k::NJ, j = line % k::NJ;
+    const double* u = a.Uin + (((long long)v * a.Tu + (a.Tu == 1 ? 0 : t)) * k::NS) * g.Nc + c;
+    Line<k::n> ln;
+#pragma unroll
+    for (int s = 0; s < k::n; ++s) ln.v[s] = u[sp_index<D, P>(d, j, s) * g.Nc];
+    line_ready<k::n>(ln, op.soft);
+    double m[ni];
+    line_apply<k::n, ni, LANES2>(op.c_sp_to_fp, 1, 1, ln, m);
+#pragma unroll
+    for (int f = 0; f < ni; ++f) scr[(i * ni + f) * CPB] = m[f];
+  }
+}
+
+// their fluxes, in place
+static __device__ __forceinline__ void fluxes(const Geo& g, const Args& a, int d, int l0, int l1, long long c,
+                                              double* scr, const double* __restrict__ meq) {
+  const int CPB = blockDim.x;
+#pragma unroll 1
+  for (int i = threadIdx.y; i < (l1 - l0) * ni; i += (int)blockDim.y) {
+    const int f = i % ni, l = i / ni;
+    double* at = scr + (l * k::V * ni + f) * CPB;
+    double M[k::V];
+#pragma unroll
+    for (int v = 0; v < k::V; ++v) M[v] = at[v * ni * CPB];
+    if (a.wb) {
+      const int j = (l0 + l) % k::NJ;
+#pragma unroll
+      for (int v = 0; v < k::V; ++v) M[v] = M[v] + meq[(((long long)v * k::NJ + j) * k::nf + f + 1) * g.Nc + c];
+    }
+    euler_flux<D>(M, g.gamma, d, a.iso, &g.rgm1, [&](int v, double F) { at[v * ni * CPB] = F; });
+  }
+}
+
+// the derivative of their fluxes into the tile (added to the lower
+// directions'), or the flux-point output
+template <bool LANES2>
+static __device__ __forceinline__ void derive(const Ops& op, const Geo& g, const Args& a, int d, int l0, int l1,
+                                              long long c, double* tile, const double* scr, const Dir& dir) {
+  const int CPB = blockDim.x;
   int cx, cy, cz;
   cell_coords(g, c, cx, cy, cz);
   const long long nI = n_iface(g, d);
   const int cd = (d == 0) ? cx : (d == 1 ? cy : cz);
   const long long il = iface_id(g, d, cx, cy, cz, cd);
   const long long ir = iface_id(g, d, cx, cy, cz, cd + 1);
-  const int CPB = blockDim.x, NT = blockDim.x * blockDim.y;
-  constexpr int ni = k::nf - 2;
-  for (int item = threadIdx.y; item < a.Teff * k::NJ; item += (int)blockDim.y) {
-    const int t = item / k::NJ, j = item % k::NJ;
-    const int tu = (a.Tu == 1) ? 0 : t;
+  const bool pow2 = g.h_pow2[d] != 0;
 #pragma unroll 1
-    for (int v = 0; v < k::V; ++v) {
-      Line<k::n> ln;
+  for (int i = threadIdx.y; i < (l1 - l0) * k::V; i += (int)blockDim.y) {
+    const int v = i % k::V, line = l0 + i / k::V;
+    const int t = line / k::NJ, j = line % k::NJ;
+    const long long vtj = ((long long)v * g.T + t) * k::NJ + j;
+    Line<k::nf> lf;
+    lf.v[0] = dir.Fi[vtj * nI + il];
+    lf.v[k::nf - 1] = dir.Fi[vtj * nI + ir];
 #pragma unroll
-      for (int s = 0; s < k::n; ++s)
-        ln.v[s] = a.Uin[(((long long)v * a.Tu + tu) * k::NS + sp_index<D, P>(d, j, s)) * g.Nc + c];
-      line_ready<k::n>(ln, op.soft);
-      double m[ni];
-      line_apply<k::n, ni, LANES2>(op.c_sp_to_fp, 1, 1, ln, m);
+    for (int f = 0; f < ni; ++f) lf.v[f + 1] = scr[(i * ni + f) * CPB];
+    if (a.wb) {
+      // F -> F' (src/sdader_simulator.py:235-237), before the viscous flux
 #pragma unroll
-      for (int f = 0; f < ni; ++f) scr[(v * ni + f) * NT] = m[f];
+      for (int f = 0; f < k::nf; ++f)
+        lf.v[f] = lf.v[f] - dir.feq[(((long long)v * k::NJ + j) * k::nf + f) * g.Nc + c];
     }
+    if (a.visc) {
 #pragma unroll
-    for (int f = 0; f < ni; ++f) {
-      double M[k::V];
-#pragma unroll
-      for (int v = 0; v < k::V; ++v) M[v] = scr[(v * ni + f) * NT];
-      if (a.wb) {
-#pragma unroll
-        for (int v = 0; v < k::V; ++v) M[v] = M[v] + meq[(((long long)v * k::NJ + j) * k::nf + f + 1) * g.Nc + c];
-      }
-      euler_flux<D>(M, g.gamma, d, a.iso, &g.rgm1, [&](int v, double F) { scr[(v * ni + f) * NT] = F; });
+      for (int f = 0; f < k::nf; ++f) lf.v[f] = lf.v[f] - dir.Gv[(vtj * k::nf + f) * g.Nc + c];
     }
-    const bool pow2 = g.h_pow2[d] != 0;
+    if (a.mode == 2) {
+#pragma unroll
+      for (int f = 0; f < k::nf; ++f) dir.Ffp[(vtj * k::nf + f) * g.Nc + c] = lf.v[f];
+      continue;
+    }
+    line_ready<k::nf>(lf, op.soft, op.dfp_eoff[d]);
+    double val[k::n];
+    line_apply<k::nf, k::n, LANES2>(op.c_dfp, 0, 1, lf, val);
+#pragma unroll
+    for (int so = 0; so < k::n; ++so) {
+      const double x = pow2 ? val[so] : div_by(val[so], g.h[d], g.rh[d]);
+      double* slot = &tile[((v * k::NS + sp_index<D, P>(d, j, so)) * a.Tn + t) * CPB];
+      *slot = LANES2 ? x : *slot + x;
+    }
+  }
+}
+
+template <bool LANES2>
+static __device__ __forceinline__ void direction(const Ops& op, const Geo& g, const Args& a, int dd, int chunk,
+                                                 long long c, bool active, double* tile, double* scr, const Dir& dir) {
+  const int d = LANES2 ? 0 : dd;
+  const int lines = a.Teff * k::NJ;
 #pragma unroll 1
-    for (int v = 0; v < k::V; ++v) {
-      Line<k::nf> lf;
-      const double* fe = Fi + (((long long)v * g.T + t) * k::NJ + j) * nI;
-      lf.v[0] = fe[il];
-      lf.v[k::nf - 1] = fe[ir];
-#pragma unroll
-      for (int f = 0; f < ni; ++f) lf.v[f + 1] = scr[(v * ni + f) * NT];
-      if (a.wb) {
-        // F -> F' (src/sdader_simulator.py:235-237), before the viscous flux
-#pragma unroll
-        for (int f = 0; f < k::nf; ++f)
-          lf.v[f] = lf.v[f] - feq[(((long long)v * k::NJ + j) * k::nf + f) * g.Nc + c];
-      }
-      if (a.visc) {
-#pragma unroll
-        for (int f = 0; f < k::nf; ++f)
-          lf.v[f] = lf.v[f] - Gv[((((long long)v * g.T + t) * k::NJ + j) * k::nf + f) * g.Nc + c];
-      }
-      if (a.mode == 2) {
-#pragma unroll
-        for (int f = 0; f < k::nf; ++f)
-          Ffp[((((long long)v * g.T + t) * k::NJ + j) * k::nf + f) * g.Nc + c] = lf.v[f];
-        continue;
-      }
-      line_ready<k::nf>(lf, op.soft, op.dfp_eoff[d]);
-      double val[k::n];
-      line_apply<k::nf, k::n, LANES2>(op.c_dfp, 0, 1, lf, val);
-#pragma unroll
-      for (int so = 0; so < k::n; ++so) {
-        const double x = pow2 ? val[so] : div_by(val[so], g.h[d], g.rh[d]);
-        double* slot = &tile[((v * k::NS + sp_index<D, P>(d, j, so)) * a.Tn + t) * CPB + threadIdx.x];
-        *slot = LANES2 ? x : *slot + x;
-      }
-    }
+  for (int l0 = 0; l0 < lines; l0 += chunk) {
+    const int l1 = l0 + chunk < lines ? l0 + chunk : lines;
+    // the tile's and the chunk's readers of before are done
+    if (!LANES2 || l0 > 0) __syncthreads();
+    if (active) interpolate<LANES2>(op, g, a, d, l0, l1, c, scr);
+    __syncthreads();
+    if (active) fluxes(g, a, d, l0, l1, c, scr, dir.meq);
+    __syncthreads();
+    if (active) derive<LANES2>(op, g, a, d, l0, l1, c, tile, scr, dir);
   }
 }
 
@@ -461,7 +493,7 @@ static __device__ __forceinline__ void picard(const Ops& op, const Geo& g, doubl
   }
 }
 
-static __device__ __forceinline__ void run(Blk B, const Ops& op, const Geo& g, int mode, int Teff,
+static __device__ __forceinline__ void run(Blk B, const Ops& op, const Geo& g, int mode, int Teff, int chunk,
                                            const double* __restrict__ Uin, int Tu, const double* __restrict__ dt_ptr,
                                            double* __restrict__ U_sp, double* __restrict__ U_ader, const double* Fi0,
                                            const double* Fi1, const double* Fi2, double* tr0, double* tr1,
@@ -481,15 +513,12 @@ static __device__ __forceinline__ void run(Blk B, const Ops& op, const Geo& g, i
   const int cl = threadIdx.x, row = threadIdx.y;
   const long long c = B.id * (long long)CPB + cl;
   const bool active = c < g.Nc;
-  double* scr = dudt_s + (mode == 2 ? 0 : k::V * k::NS * a.Tn * CPB) + row * CPB + cl;
-  if (active) lines<true>(op, g, a, 0, c, dudt_s, scr, Fi0, Ffp0, G0, M0, E0);
+  double* scr = dudt_s + (mode == 2 ? 0 : k::V * k::NS * a.Tn * CPB) + cl;
+  direction<true>(op, g, a, 0, chunk, c, active, dudt_s + cl, scr, Dir{Fi0, Ffp0, G0, M0, E0});
 #pragma unroll 1
-  for (int d = 1; d < D; ++d) {
-    if (mode != 2) __syncthreads();
-    if (active)
-      lines<false>(op, g, a, d, c, dudt_s, scr, d == 1 ? Fi1 : Fi2, d == 1 ? Ffp1 : Ffp2, d == 1 ? G1 : G2,
-                   d == 1 ? M1 : M2, d == 1 ? E1 : E2);
-  }
+  for (int d = 1; d < D; ++d)
+    direction<false>(op, g, a, d, chunk, c, active, dudt_s + cl, scr,
+                     d == 1 ? Dir{Fi1, Ffp1, G1, M1, E1} : Dir{Fi2, Ffp2, G2, M2, E2});
   if (mode == 2) return;
   if (pot) {
     __syncthreads();
@@ -557,26 +586,27 @@ static __device__ __forceinline__ void run(Blk B, const Ops& op, const Geo& g, i
   }
   __syncthreads();
   if (!active) return;
-  for (int item = row; item < g.T * D * k::NJ; item += rows) {
-    const int d = item / (g.T * k::NJ), r = item % (g.T * k::NJ);
-    const int t = r / k::NJ, j = r % k::NJ;
-    auto at = [&](int v, int s) { return dudt_s[((v * k::NS + s) * g.T + t) * CPB + cl]; };
-    if (d == 0) trace_line<D, P, true>(op, g, at, c, tr0, t, 0, j);
-    else trace_line<D, P, false>(op, g, at, c, d == 1 ? tr1 : tr2, t, d, j);
+#pragma unroll 1
+  for (int item = row; item < D * g.T * k::NJ * k::V; item += rows) {
+    const int d = item / (g.T * k::NJ * k::V), r = item % (g.T * k::NJ * k::V);
+    const int v = r % k::V, t = r / (k::V * k::NJ), j = r / k::V % k::NJ;
+    auto at = [&](int s) { return dudt_s[((v * k::NS + s) * g.T + t) * CPB + cl]; };
+    if (d == 0) trace_line<D, P, true>(op, g, at, c, tr0, t, 0, j, v);
+    else trace_line<D, P, false>(op, g, at, c, d == 1 ? tr1 : tr2, t, d, j, v);
   }
 }
 };
 template <int D, int P>
-__global__ void __launch_bounds__(INTERIOR_THREADS) k_interior(Ops op, Geo g, int mode, int Teff, const double* __restrict__ Uin, int Tu,
+__global__ void __launch_bounds__(INTERIOR_THREADS, INTERIOR_BLOCKS) k_interior(Ops op, Geo g, int mode, int Teff, int chunk, const double* __restrict__ Uin, int Tu,
                            const double* __restrict__ dt_ptr, double* __restrict__ U_sp, double* __restrict__ U_ader,
                            const double* Fi0, const double* Fi1, const double* Fi2, double* tr0, double* tr1,
                            double* tr2, double* Ffp0, double* Ffp1, double* Ffp2) {
-  Interior<D, P>::run(hw_blk(), op, g, mode, Teff, Uin, Tu, dt_ptr, U_sp, U_ader, Fi0, Fi1, Fi2, tr0, tr1, tr2, Ffp0,
+  Interior<D, P>::run(hw_blk(), op, g, mode, Teff, chunk, Uin, Tu, dt_ptr, U_sp, U_ader, Fi0, Fi1, Fi2, tr0, tr1, tr2, Ffp0,
                       Ffp1, Ffp2);
 }
 template <int D, int P>
 struct InteriorExt {
-  static __device__ __forceinline__ void run(Blk B, const Ops& op, const Geo& g, int mode, int Teff,
+  static __device__ __forceinline__ void run(Blk B, const Ops& op, const Geo& g, int mode, int Teff, int chunk,
                                              const double* __restrict__ Uin, int Tu, const double* __restrict__ dt_ptr,
                                              double* __restrict__ U_sp, double* __restrict__ U_ader,
                                              const double* Fi0, const double* Fi1, const double* Fi2, double* tr0,
@@ -585,19 +615,19 @@ struct InteriorExt {
                                              const double* gphi, const double* M0, const double* M1,
                                              const double* M2, const double* E0, const double* E1,
                                              const double* E2) {
-    Interior<D, P, true>::run(B, op, g, mode, Teff, Uin, Tu, dt_ptr, U_sp, U_ader, Fi0, Fi1, Fi2, tr0, tr1, tr2, Ffp0,
+    Interior<D, P, true>::run(B, op, g, mode, Teff, chunk, Uin, Tu, dt_ptr, U_sp, U_ader, Fi0, Fi1, Fi2, tr0, tr1, tr2, Ffp0,
                               Ffp1, Ffp2, G0, G1, G2, gphi, M0, M1, M2, E0, E1, E2);
   }
 };
 template <int D, int P>
-__global__ void __launch_bounds__(INTERIOR_THREADS) k_interior_ext(Ops op, Geo g, int mode, int Teff, const double* __restrict__ Uin, int Tu,
+__global__ void __launch_bounds__(INTERIOR_THREADS, INTERIOR_BLOCKS) k_interior_ext(Ops op, Geo g, int mode, int Teff, int chunk, const double* __restrict__ Uin, int Tu,
                                const double* __restrict__ dt_ptr, double* __restrict__ U_sp,
                                double* __restrict__ U_ader, const double* Fi0, const double* Fi1, const double* Fi2,
                                double* tr0, double* tr1, double* tr2, double* Ffp0, double* Ffp1, double* Ffp2,
                                const double* G0, const double* G1, const double* G2, const double* gphi,
                                const double* M0, const double* M1, const double* M2, const double* E0,
                                const double* E1, const double* E2) {
-  InteriorExt<D, P>::run(hw_blk(), op, g, mode, Teff, Uin, Tu, dt_ptr, U_sp, U_ader, Fi0, Fi1, Fi2, tr0, tr1, tr2,
+  InteriorExt<D, P>::run(hw_blk(), op, g, mode, Teff, chunk, Uin, Tu, dt_ptr, U_sp, U_ader, Fi0, Fi1, Fi2, tr0, tr1, tr2,
                          Ffp0, Ffp1, Ffp2, G0, G1, G2, gphi, M0, M1, M2, E0, E1, E2);
 }
 

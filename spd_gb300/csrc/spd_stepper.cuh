@@ -66,50 +66,51 @@ template <int D, int P>
 struct Stepper : StepperBase {
   using k = K<D, P>;
 
-  // Block shape of the interior kernel.  Its shared memory: the tile of
-  // (variable, point, node) values per cell and the flux points of each
-  // thread's line (mode 2 writes those out and has no tile).
-  static constexpr size_t SMEM_MAX = 227 * 1024;
+  // Block shape of the interior kernel: ``cells`` x rows, up to
+  // INTERIOR_THREADS threads.  Its shared memory per cell is the tile of
+  // (variable, point, node) values (mode 2 has none) and the flux points of a
+  // chunk of its (node, line) pairs.
+  static constexpr size_t SMEM_MAX = 227 * 1024, SMEM_SM = 228 * 1024, SMEM_BLOCK = 1024;
   static size_t tile_bytes(int nodes) { return (size_t)k::V * k::NS * nodes * sizeof(double); }
   static constexpr size_t line_bytes() { return (size_t)k::V * (k::nf - 2) * sizeof(double); }
-  // thread rows: the (node, line) pairs of a cell in as few equal rounds as
-  // fit into ``threads`` per block and the shared memory
-  static int rows_for(int cells, int T, int threads) {
-    const int items = T * k::NJ;
-    int most = std::max(1, threads / cells);
-    const size_t tile = tile_bytes(T) * cells;
-    if (tile < SMEM_MAX) most = std::min<int>(most, (int)((SMEM_MAX - tile) / (line_bytes() * cells)));
-    if (tile >= SMEM_MAX || most < 1) return 0;
-    const int rounds = (items + most - 1) / most;
-    return (items + rounds - 1) / rounds;
-  }
-  static size_t interior_smem(int cells, int rows, int nodes) {
-    return (tile_bytes(nodes) + line_bytes() * rows) * cells;
-  }
-  // 256 threads where two such blocks fit an SM, else 512 (two blocks of 256
-  // overlap each other's barriers; a tile too large for that still gets its
-  // threads)
-  static int interior_rows(int cells, int T) {
-    const int r = rows_for(cells, T, 256);
-    if (r > 0 && 2 * interior_smem(cells, r, T) <= SMEM_MAX) return r;
-    return rows_for(cells, T, INTERIOR_THREADS);
+  struct Shape {
+    int cells = 0, rows = 0, chunk = 0, blocks = 0;  // chunk 0: does not fit
+  };
+  static size_t interior_smem(const Shape& s, int nodes) { return (tile_bytes(nodes) + line_bytes() * s.chunk) * s.cells; }
+  // the largest chunk, in equal parts of all lines, that leaves room for
+  // INTERIOR_BLOCKS blocks per SM, or for as many as fit with the smallest
+  static Shape interior_shape(int cells, int T) {
+    Shape best;
+    const int lines = T * k::NJ;
+    for (int parts = 1; parts <= lines; ++parts) {
+      Shape s;
+      s.cells = cells;
+      s.chunk = (lines + parts - 1) / parts;
+      const size_t b = interior_smem(s, T);
+      if (b > SMEM_MAX) continue;
+      s.blocks = std::min<int>(INTERIOR_BLOCKS, (int)(SMEM_SM / (b + SMEM_BLOCK)));
+      s.rows = std::max(1, std::min(INTERIOR_THREADS / cells, s.chunk * k::V));
+      if (s.blocks > best.blocks) best = s;
+      if (best.blocks == INTERIOR_BLOCKS) break;
+    }
+    return best;
   }
 
   int configure(spd_ctx* C) override {
     max_cpb = 64;
-    while (max_cpb > 1 && interior_rows(max_cpb, C->T) < 1) max_cpb /= 2;
-    if (interior_rows(max_cpb, C->T) < 1) return fail(C, SPD_ERR_ARG, "the step's tile exceeds the shared memory");
-    // the widest block that keeps the most threads resident
+    while (max_cpb > 1 && interior_shape(max_cpb, C->T).chunk == 0) max_cpb /= 2;
+    if (interior_shape(max_cpb, C->T).chunk == 0)
+      return fail(C, SPD_ERR_ARG, "the step's tile exceeds the shared memory");
+    // the widest block that keeps the most threads resident, 16 cells (128
+    // bytes of a row) at most
     int best = -1;
-    for (int cells = std::min(32, max_cpb); cells >= 4 || cells == max_cpb; cells /= 2) {
-      const int r = interior_rows(cells, C->T);
-      const int blocks = std::max(1, (int)(SMEM_MAX / interior_smem(cells, r, C->T)));
-      const int resident = std::min(512, blocks * r * cells);
-      if (resident > best) {
-        best = resident;
+    cpb = 1;
+    for (int cells = std::min(16, max_cpb); cells >= std::min(4, max_cpb); cells /= 2) {
+      const Shape s = interior_shape(cells, C->T);
+      if (s.blocks * s.rows * cells > best) {
+        best = s.blocks * s.rows * cells;
         cpb = cells;
       }
-      if (cells == 1) break;
     }
     CK(cudaFuncSetAttribute(k_interior<D, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
     CK(cudaFuncSetAttribute(k_interior_ext<D, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
@@ -172,7 +173,7 @@ struct Stepper : StepperBase {
                          C->stream));
     {
       ProfScope ps_(C, "k_traces_sp");
-      launch<TracesSp<D, P>>(C, "k_traces_sp", k_traces_sp<D, P>, blocks_for(g.Nc * (D * k::NJ), 128), 128, 0, C->ops, g, C->U_sp,
+      launch<TracesSp<D, P>>(C, "k_traces_sp", k_traces_sp<D, P>, blocks_for(g.Nc * (D * k::NJ * k::V), 128), 128, 0, C->ops, g, C->U_sp,
                              C->trace[0], C->trace[1], C->trace[2]);
     }
     CKL();
@@ -221,12 +222,13 @@ struct Stepper : StepperBase {
         CKL();
       }
       const int cells = interior_cells(C);
-      const dim3 block(cells, interior_rows(cells, C->T));
-      const size_t sm = interior_smem(cells, block.y, mode == 2 ? 0 : (mode == 0 ? C->T : Teff));
+      const Shape shape = interior_shape(cells, C->T);
+      const dim3 block(cells, shape.rows);
+      const size_t sm = interior_smem(shape, mode == 2 ? 0 : (mode == 0 ? C->T : Teff));
       if (visc || C->gphi_sp || C->Ueq_sp || C->cfg.isothermal) {
         ProfScope ps_(C, "k_interior");
         launch<InteriorExt<D, P>>(C, "k_interior", k_interior_ext<D, P>, blocks_for(g.Nc, cells), block, sm, C->ops,
-                                  g, mode, Teff, Uin, Tu, C->dt, C->U_sp, C->U_ader, C->Fi[0], C->Fi[1], C->Fi[2],
+                                  g, mode, Teff, shape.chunk, Uin, Tu, C->dt, C->U_sp, C->U_ader, C->Fi[0], C->Fi[1], C->Fi[2],
                                   C->trace[0], C->trace[1], C->trace[2], C->Ffp[0], C->Ffp[1], C->Ffp[2],
                                   visc ? C->Gv[0] : nullptr, C->Gv[1], C->Gv[2], (const double*)C->gphi_sp,
                                   (const double*)C->Meq_fp[0], (const double*)C->Meq_fp[1],
@@ -235,7 +237,7 @@ struct Stepper : StepperBase {
       } else {
         ProfScope ps_(C, "k_interior");
         launch<Interior<D, P>>(C, "k_interior", k_interior<D, P>, blocks_for(g.Nc, cells), block, sm, C->ops, g, mode,
-                               Teff, Uin, Tu, C->dt, C->U_sp, C->U_ader, C->Fi[0], C->Fi[1], C->Fi[2], C->trace[0],
+                               Teff, shape.chunk, Uin, Tu, C->dt, C->U_sp, C->U_ader, C->Fi[0], C->Fi[1], C->Fi[2], C->trace[0],
                                C->trace[1], C->trace[2], C->Ffp[0], C->Ffp[1], C->Ffp[2]);
       }
       CKL();
