@@ -161,18 +161,12 @@ SPD_FN double div_rcp(double a, double b, double rb) {
 // c ? a : b by value
 template <class S>
 SPD_FN S sel(bool c, const S& a, const S& b) { return c ? a : b; }
-#ifndef SPD_FUSED
 SPD_FN Num sel(bool c, const Num& a, const Num& b) { return Num(c ? a.v : b.v, c ? a.ok : b.ok); }
-#endif
 SPD_FN double half(double x) { return 0.5 * x; }
 template <int N> SPD_FN Dual<N> half(const Dual<N>& x) { return 0.5 * x; }
 SPD_FN double sval(double x) { return x; }
 template <int N> SPD_FN double sval(const Dual<N>& x) { return x.v; }
-#ifdef SPD_FUSED
-SPD_FN double ad_sqrt(double x) { return sqrt(x); }
-#else
 SPD_FN double ad_sqrt(double x) { return sqrt_soft(x); }
-#endif
 template <int N>
 SPD_FN Dual<N> ad_sqrt(const Dual<N>& x) {
   Dual<N> r; r.v = sqrt(x.v);
@@ -197,17 +191,12 @@ SPD_FN Dual<N> ad_abs(const Dual<N>& x) {
   return Dual<N>(fabs(x.v));
 }
 
-// a / b with b's reciprocal prepared by recip_of (double: div_soft, or in the
-// build with fused multiply-adds Markstein's correction; dual numbers: plain
-// division, the reciprocal unused)
+// a / b with b's reciprocal prepared by recip_of (double: div_soft; dual
+// numbers: plain division, the reciprocal unused)
 template <class S>
 struct RecipOf {
   using T = S;
 };
-#ifdef SPD_FUSED
-SPD_FN double div_by(double a, double b, double rb) { return div_rcp(a, b, rb); }
-SPD_FN double recip_of(double b) { return 1.0 / b; }
-#else
 template <>
 struct RecipOf<double> {
   using T = Recip;
@@ -218,7 +207,6 @@ struct RecipOf<Num> {
 };
 SPD_FN double div_by(double a, double b, const Recip& rb) { return div_soft(a, b, rb); }
 SPD_FN Recip recip_of(double b) { return recip_soft(b); }
-#endif
 // a prepared reciprocal of a double
 using Rcp = typename RecipOf<double>::T;
 // a / b
@@ -280,13 +268,11 @@ SPD_FN bool fge(double a, double b) {
   return a >= b;
 #endif
 }
-#ifndef SPD_FUSED
 SPD_FN bool fgt(const Num& a, const Num& b) { return fgt(a.v, b.v); }
 SPD_FN bool fgt(const Num& a, double b) { return fgt(a.v, b); }
 SPD_FN bool fgt(double a, const Num& b) { return fgt(a, b.v); }
 SPD_FN Num np_max(const Num& a, const Num& b) { return Num(np_max(a.v, b.v), a.ok & b.ok); }
 SPD_FN Num np_min(const Num& a, const Num& b) { return Num(np_min(a.v, b.v), a.ok & b.ok); }
-#endif
 template <int N> SPD_FN bool fgt(const Dual<N>& a, const Dual<N>& b) { return a.v > b.v; }
 template <int N> SPD_FN bool fgt(const Dual<N>& a, double b) { return a.v > b; }
 template <int N> SPD_FN bool fgt(double a, const Dual<N>& b) { return a > b.v; }

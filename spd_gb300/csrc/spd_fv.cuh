@@ -114,48 +114,54 @@ __device__ __forceinline__ void flux_divergence(const Geo& g, const FvGeo& fg, i
   out = acc;
 }
 
-// Ghost layers written by the active subcells they mirror.
-//
-// The reference fills them direction by direction (src/fv_simulator.py:
-// 224-273), each fill reading the ghosts of the directions before it, so a
-// ghost subcell's value follows from one active subcell: along every ghost
-// direction the periodic or the nearest-edge image (whose layers are not
-// mirrored), the normal velocity negated at a reflective side, and at a side
-// with a fixed state the stored layer.  Writing it from that subcell saves
-// the fills: at 32^2 a substep launched six of them, 4 us each.
-//
-// for_ghosts calls f(e, choice) for every ghost position e (extended
-// coordinates) of the active subcell a; choice[d] is -1 (not a ghost along
-// d) or the side.
-template <int D, class F>
-__device__ __forceinline__ void for_ghosts(const Geo& g, const int* a, F f) {
-  int pos[3][2];  // image at either side, or -1
-  bool any = false;
+// Ghost layers.  The reference fills them direction by direction
+// (src/fv_simulator.py:224-273), each fill reading the ghosts of the
+// directions before it, so a ghost subcell's value follows from one active
+// subcell: along every ghost direction the periodic or the nearest-edge image
+// (whose layers are not mirrored), the normal velocity negated at a
+// reflective side, and at a side with a fixed state the stored layer.  They
+// are gathered so, all directions at once, by blocks of the kernels that run
+// before their readers (six fills of 4 us each per substep at 32^2; written
+// by the subcells they mirror instead, the few ghost owners in every warp
+// slowed k_fv_candidate from 1.2 to 2.2 ms at 48^3).
+struct GhostPos {
+  int e[3];       // extended coordinates
+  int a[3];       // extended coordinates of the active subcell it mirrors
+  int side[3];    // side along d, or -1: not a ghost along d
+};
+template <int D>
+__host__ __device__ __forceinline__ long long n_ghosts(const Geo& g) { return g.Nqe - g.Nq; }
+// the idx-th ghost position: per direction d the layers along d over all
+// positions of the directions before and the active ones of those after
+template <int D>
+__device__ __forceinline__ GhostPos ghost_pos(const Geo& g, long long idx) {
+  GhostPos p;
+  int d = 0;
 #pragma unroll
-  for (int d = 0; d < D; ++d) {
-    const int X = g.X[d], i = a[d];
-    const bool lo = i < NGH, hi = i >= X - NGH;
-    pos[d][0] = (g.bc[d][0] == BC_PERIODIC) ? (hi ? i - (X - NGH) : -1) : (lo ? i : -1);
-    pos[d][1] = (g.bc[d][1] == BC_PERIODIC) ? (lo ? X + NGH + i : -1) : (hi ? i + 2 * NGH : -1);
-    any = any || lo || hi;
-  }
-  if (!any) return;
-  constexpr int combos = (D == 1) ? 3 : (D == 2 ? 9 : 27);
-#pragma unroll 1
-  for (int m = 1; m < combos; ++m) {
-    int e[3] = {0, 0, 0}, choice[3] = {-1, -1, -1};
-    bool ok = true;
-    int r = m;
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      choice[d] = r % 3 - 1;
-      r /= 3;
-      const int p = (choice[d] < 0) ? a[d] + NGH : (choice[d] == 0 ? pos[d][0] : pos[d][1]);
-      ok = ok && p >= 0;
-      e[d] = p;
+  for (int q = D - 1; q > 0; --q) {
+    long long n = 2 * NGH;
+    for (int r = 0; r < D; ++r) n *= (r < q) ? g.Xe[r] : (r > q ? g.X[r] : 1);
+    if (d == 0) {
+      if (idx < n) d = q;
+      else idx -= n;
     }
-    if (ok) f(e, choice);
   }
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    p.e[r] = p.a[r] = 0;
+    p.side[r] = -1;
+    if (r >= D) continue;
+    const int n = (r < d) ? g.Xe[r] : (r > d ? g.X[r] : 2 * NGH);
+    const int k = (int)(idx % n);
+    idx /= n;
+    p.e[r] = (r < d) ? k : (r > d ? k + NGH : (k < NGH ? k : g.X[r] + k));
+    const int X = g.X[r];
+    p.side[r] = p.e[r] < NGH ? 0 : (p.e[r] >= X + NGH ? 1 : -1);
+    p.a[r] = p.e[r];
+    if (p.side[r] == 0) p.a[r] = p.e[r] + (g.bc[r][0] == BC_PERIODIC ? X : NGH);
+    if (p.side[r] == 1) p.a[r] = p.e[r] - (g.bc[r][1] == BC_PERIODIC ? X : NGH);
+  }
+  return p;
 }
 __device__ __forceinline__ long long ext_at(const Geo& g, const int* e) {
   return e[0] + (long long)g.Xe[0] * (e[1] + (long long)g.Xe[1] * e[2]);
@@ -171,48 +177,30 @@ __device__ __forceinline__ long long bc_entry(const Geo& g, int d, int side, int
 struct BcBufs {
   double* b[3];
 };
-// whether an active subcell owns any ghost
+__device__ __forceinline__ bool fixed_bc(int kind) { return kind == BC_IC || kind == BC_PRESSURE; }
+// variable v of the ghost position p from the active values of ext
 template <int D>
-__device__ __forceinline__ bool near_side(const Geo& g, int ix, int iy, int iz) {
-  bool any = ix < NGH || ix >= g.X[0] - NGH;
-  if (D > 1) any = any || iy < NGH || iy >= g.X[1] - NGH;
-  if (D > 2) any = any || iz < NGH || iz >= g.X[2] - NGH;
-  return any;
-}
-// the primitives W of an active subcell into the ghosts it owns; out of line,
-// because few subcells own any
-template <int D>
-__device__ __noinline__ void write_ghosts(const Geo& g, const BcBufs& bc, int ix, int iy, int iz, const double* W,
-                                          double* __restrict__ ext) {
-  constexpr int V = D + 2;
-  const int a[3] = {ix, iy, iz};
-  for_ghosts<D>(g, a, [&](const int* e, const int* choice) {
-    double w[V];
+__device__ __forceinline__ double ghost_value(const Geo& g, const BcBufs& bc, const GhostPos& p, int v,
+                                              const double* __restrict__ ext) {
+  double w = ext[(long long)v * g.Nqe + ext_at(g, p.a)];
 #pragma unroll
-    for (int v = 0; v < V; ++v) w[v] = W[v];
+  for (int d = 0; d < D; ++d) {
+    if (p.side[d] < 0) continue;
+    const int kind = g.bc[d][p.side[d]];
+    if (kind == BC_REFLECTIVE) {
+      if (v == d + 1) w = w * -1.0;
+    } else if (kind == BC_EQ) {
+      w = 0.0;
+    } else if (fixed_bc(kind)) {
+      // the stored layer, at this ghost along the directions before d and at
+      // the mirrored subcell along those after
+      int at[3] = {0, 0, 0};
 #pragma unroll
-    for (int d = 0; d < D; ++d) {
-      if (choice[d] < 0) continue;
-      const int kind = g.bc[d][choice[d]];
-      if (kind == BC_REFLECTIVE) {
-        w[d + 1] = w[d + 1] * -1.0;
-      } else if (kind == BC_EQ) {
-#pragma unroll
-        for (int v = 0; v < V; ++v) w[v] = 0.0;
-      } else if (kind != BC_PERIODIC && kind != BC_GRADFREE) {
-        // the stored layer, at this ghost along the directions before d and
-        // at the active position along those after
-        int at[3] = {0, 0, 0};
-#pragma unroll
-        for (int q = 0; q < D; ++q) at[q] = (q <= d) ? e[q] : a[q] + NGH;
-#pragma unroll
-        for (int v = 0; v < V; ++v) w[v] = bc.b[d][bc_entry(g, d, choice[d], V, v, at)];
-      }
+      for (int q = 0; q < D; ++q) at[q] = (q <= d) ? p.e[q] : p.a[q];
+      w = bc.b[d][bc_entry(g, d, p.side[d], D + 2, v, at)];
     }
-    const long long x = ext_at(g, e);
-#pragma unroll
-    for (int v = 0; v < V; ++v) ext[(long long)v * g.Nqe + x] = w[v];
-  });
+  }
+  return w;
 }
 
 // counters that a substep accumulates, zeroed by its first kernel
@@ -236,8 +224,7 @@ struct FvCandidate {
 static __device__ __forceinline__ void run(Blk B, const Geo& g, const FvGeo& fg, const double* __restrict__ dt_ptr,
                                            double w_i, const double* F0, const double* F1, const double* F2,
                                            const double* __restrict__ U_cv, double* __restrict__ U_new,
-                                           double* ext_old, double* ext_new, int write_ext, const BcBufs& bc,
-                                           const Counters& ct, double* __restrict__ W_cv,
+                                           double* ext_old, double* ext_new, int write_ext, const Counters& ct, double* __restrict__ W_cv,
                                            const double* __restrict__ gphi, const double* __restrict__ Ueq,
                                            const double* __restrict__ Weq) {
   constexpr int V = D + 2;
@@ -274,22 +261,9 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, const FvGeo& fg,
     }
 #pragma unroll
     for (int v = 0; v < V; ++v) ext_old[(long long)v * g.Nqe + e] = W[v];
-    const bool side = near_side<D>(g, ix, iy, iz);
-    if (side) {
-      double w[V];
-#pragma unroll
-      for (int v = 0; v < V; ++v) w[v] = W[v];
-      write_ghosts<D>(g, bc, ix, iy, iz, w, ext_old);
-    }
     prims_cv<D>(g, un, W, Ueq, Weq, q);
 #pragma unroll
     for (int v = 0; v < V; ++v) ext_new[(long long)v * g.Nqe + e] = W[v];
-    if (side) {
-      double w[V];
-#pragma unroll
-      for (int v = 0; v < V; ++v) w[v] = W[v];
-      write_ghosts<D>(g, bc, ix, iy, iz, w, ext_new);
-    }
     if (W_cv != nullptr) {
 #pragma unroll
       for (int v = 0; v < V; ++v) W_cv[(long long)v * g.Nq + q] = W[v];
@@ -298,13 +272,13 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, const FvGeo& fg,
 }
 };
 template <int D>
-__global__ void k_fv_candidate(const __grid_constant__ Geo g, FvGeo fg, const double* __restrict__ dt_ptr, double w_i,
+__global__ void k_fv_candidate(Geo g, FvGeo fg, const double* __restrict__ dt_ptr, double w_i,
                                const double* F0, const double* F1, const double* F2,
                                const double* __restrict__ U_cv, double* __restrict__ U_new, double* ext_old,
-                               double* ext_new, int write_ext, const __grid_constant__ BcBufs bc, Counters ct,
+                               double* ext_new, int write_ext, Counters ct,
                                double* __restrict__ W_cv, const double* __restrict__ gphi, const double* __restrict__ Ueq,
                                const double* __restrict__ Weq) {
-  FvCandidate<D>::run(hw_blk(), g, fg, dt_ptr, w_i, F0, F1, F2, U_cv, U_new, ext_old, ext_new, write_ext, bc, ct, W_cv,
+  FvCandidate<D>::run(hw_blk(), g, fg, dt_ptr, w_i, F0, F1, F2, U_cv, U_new, ext_old, ext_new, write_ext, ct, W_cv,
                       gphi, Ueq, Weq);
 }
 
@@ -312,7 +286,7 @@ __global__ void k_fv_candidate(const __grid_constant__ Geo g, FvGeo fg, const do
 // boundary buffer when the reference does, then copy it into the ghost
 // layers.  bcbuf layout [side][v][g][other], other = the extended index of
 // the remaining directions (lower direction fastest).  The adjoint rebuilds a
-// substep's primitives with it; the step writes its ghosts with write_ghosts.
+// substep's primitives with it; the step gathers its ghosts (ghost_value).
 template <int D>
 struct Ghost {
 static __device__ __forceinline__ void run(Blk B, const Geo& g, int d, int nv, double* ext, double* bcbuf) {
@@ -366,38 +340,100 @@ __global__ void k_ghost(Geo g, int d, int nv, double* ext, double* bcbuf) {
 
 // NAD: relaxed discrete maximum principle over the cross stencil
 // (src/trouble_detection.py:14-38).  mask bit v = possible trouble of var v.
+//
+// Bound by the integer pipes.  A variable is first tried on the upper words
+// of the values' order-preserving keys: one unit there is at least 2^-21 of
+// the value and at most 2^-20 (of the larger value, where a power of two lies
+// between), so a new value within ``slack`` units of the stencil's extrema
+// lies within a relative distance of (slack + 1) 2^-20 of them, and only the
+// others take the exact bounds.  slack < 0: no such test (a zero or
+// differential tolerance).
+//
+// The grid's blocks after the first ``nb_main`` fill the ghosts of ext_old and
+// ext_new; the stencil reads its own images of active subcells instead.
+__device__ __forceinline__ int key_hi(double x) {
+  const int h = (int)hi_word(x);
+  return h ^ ((h >> 31) & 0x7fffffff);
+}
 template <int D>
 struct Nad {
+// the stencil neighbour of an active subcell at a domain side
+static __device__ __noinline__ double outside(const Geo& g, const BcBufs& bc, const double* __restrict__ ext_old, int v,
+                                              int ix, int iy, int iz, int d, int step) {
+  GhostPos p;
+  const int c[3] = {ix, iy, iz};
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    p.e[r] = p.a[r] = (r < D) ? c[r] + NGH + (r == d ? step : 0) : 0;
+    p.side[r] = (r != d) ? -1 : (step < 0 ? 0 : 1);
+    if (r == d) p.a[r] = p.e[r] - step * (g.bc[d][p.side[r]] == BC_PERIODIC ? g.X[d] : NGH);
+  }
+  return ghost_value<D>(g, bc, p, v, ext_old);
+}
 // With sed_list non-null, the flagged (subcell, density / pressure) pairs
 // are also appended to sed_list (item 2*q + is_pressure) for k_sed.
-static __device__ __forceinline__ void run(Blk B, const Geo& g, double tol, int delta, int relax,
-                                           const double* __restrict__ ext_old, const double* __restrict__ ext_new,
-                                           unsigned char* __restrict__ mask, int* any_flag,
-                                           long long* __restrict__ sed_list, unsigned long long* __restrict__ sed_count) {
+static __device__ __forceinline__ void run(Blk B, const Geo& g, unsigned nb_main, const BcBufs& bc, double tol,
+                                           int slack, int delta, int relax, double* __restrict__ ext_old,
+                                           double* __restrict__ ext_new, unsigned char* __restrict__ mask,
+                                           int* any_flag, long long* __restrict__ sed_list,
+                                           unsigned long long* __restrict__ sed_count) {
   constexpr int V = D + 2;
+  if (B.id >= nb_main) {
+    const long long n = n_ghosts<D>(g);
+    const long long i = (B.id - nb_main) * (long long)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const GhostPos p = ghost_pos<D>(g, i);
+    const long long e = ext_at(g, p.e);
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      ext_old[(long long)v * g.Nqe + e] = ghost_value<D>(g, bc, p, v, ext_old);
+      ext_new[(long long)v * g.Nqe + e] = ghost_value<D>(g, bc, p, v, ext_new);
+    }
+    return;
+  }
   const long long q = B.id * (long long)blockDim.x + threadIdx.x;
   unsigned int m = 0;
   if (q < g.Nq) {
     int ix, iy, iz;
     q_coords(g, q, ix, iy, iz);
+    const int ii[3] = {ix, iy, iz};
     const long long e = ext_of<D>(g, ix, iy, iz);
 #pragma unroll
     for (int v = 0; v < V; ++v) {
       const double* W = ext_old + (long long)v * g.Nqe;
-      // maximum / minimum of the cross stencil on order-preserving integer
-      // keys (integer pipes; the FP64 pipe is the step's bottleneck).  A NaN
-      // anywhere makes NumPy's maximum/minimum NaN and the point troubled.
       const double c0 = W[e];
-      bool nan = is_nan_bits(c0);
-      long long kmx = order_key(c0), kmn = kmx;
+      double nb[2 * D];
 #pragma unroll
       for (int d = 0; d < D; ++d) {
         const long long st = ext_stride(g, d);
-        const double a = W[e - st], b = W[e + st];
-        nan = nan || is_nan_bits(a) || is_nan_bits(b);
-        const long long ka = order_key(a), kb = order_key(b);
-        kmx = max(kmx, max(ka, kb));
-        kmn = min(kmn, min(ka, kb));
+        nb[2 * d] = (ii[d] > 0) ? W[e - st] : outside(g, bc, ext_old, v, ix, iy, iz, d, -1);
+        nb[2 * d + 1] = (ii[d] < g.X[d] - 1) ? W[e + st] : outside(g, bc, ext_old, v, ix, iy, iz, d, 1);
+      }
+      const double wn = ext_new[(long long)v * g.Nqe + e];
+      int hmx = key_hi(c0), hmn = hmx;
+#pragma unroll
+      for (int k = 0; k < 2 * D; ++k) {
+        const int h = key_hi(nb[k]);
+        hmx = max(hmx, h);
+        hmn = min(hmn, h);
+      }
+      const int hw = key_hi(wn);
+      // all finite, infinities' and NaN's keys out of reach, and both extrema
+      // normal numbers
+      const bool normal = hmx < 0x7fe00000 && hmn > (int)0x801fffff && (hmx >= 0x00100000 || hmx <= (int)0xffefffff) &&
+                          (hmn >= 0x00100000 || hmn <= (int)0xffefffff);
+      if (slack >= 0 && normal && hw >= hmn - slack && hw <= hmx + slack) continue;
+      // maximum / minimum of the cross stencil on order-preserving integer
+      // keys (integer pipes; the FP64 pipe is the step's bottleneck).  A NaN
+      // anywhere makes NumPy's maximum/minimum NaN and the point troubled.
+      bool nan = is_nan_bits(c0);
+      long long kmx = order_key(c0), kmn = kmx;
+#pragma unroll
+      for (int k = 0; k < 2 * D; ++k) {
+        nan = nan || is_nan_bits(nb[k]);
+        const long long kk = order_key(nb[k]);
+        kmx = max(kmx, kk);
+        kmn = min(kmn, kk);
       }
       double mx = from_order_key(kmx), mn = from_order_key(kmn);
       if (relax) {
@@ -410,7 +446,6 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, double tol, int 
           mx = mx + abs_bits(mx) * tol;
         }
       }
-      const double wn = ext_new[(long long)v * g.Nqe + e];
       // !(wn >= mn) || !(wn <= mx) on the integer keys: true when any of the
       // three is NaN, else the ordered comparison (the keys equate -0, +0)
       const long long kw = order_key(wn);
@@ -439,10 +474,11 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, double tol, int 
 }
 };
 template <int D>
-__global__ void k_nad(Geo g, double tol, int delta, int relax, const double* __restrict__ ext_old,
-                      const double* __restrict__ ext_new, unsigned char* __restrict__ mask, int* any_flag,
-                      long long* __restrict__ sed_list, unsigned long long* __restrict__ sed_count) {
-  Nad<D>::run(hw_blk(), g, tol, delta, relax, ext_old, ext_new, mask, any_flag, sed_list, sed_count);
+__global__ void k_nad(const __grid_constant__ Geo g, unsigned nb_main, const __grid_constant__ BcBufs bc, double tol,
+                      int slack, int delta, int relax, double* __restrict__ ext_old, double* __restrict__ ext_new,
+                      unsigned char* __restrict__ mask, int* any_flag, long long* __restrict__ sed_list,
+                      unsigned long long* __restrict__ sed_count) {
+  Nad<D>::run(hw_blk(), g, nb_main, bc, tol, slack, delta, relax, ext_old, ext_new, mask, any_flag, sed_list, sed_count);
 }
 
 // smooth-extrema relaxation factor of one variable along direction d at
@@ -548,20 +584,15 @@ __global__ void k_sed(Geo g, FvGeo fg, const long long* __restrict__ list, const
 // flagged (and the smoothness relaxation ran), else of W_old
 // (src/fv_simulator.py:224-273, src/trouble_detection.py:40-72).  The buffers
 // themselves are kept as the fills leave them.
+// The grid's blocks after the first ``nb_main`` do the ghosts, a periodic
+// image's flag computed again from its subcell's.
 template <int D>
 struct Troubles {
-static __device__ __forceinline__ void run(Blk B, const Geo& g, int pad, double min_rho, double max_rho, double min_P,
-                                           const unsigned char* __restrict__ mask, const int* __restrict__ flags,
-                                           int sed, const double* __restrict__ ext_old,
-                                           const double* __restrict__ ext_new, const BcBufs& bc,
-                                           double* __restrict__ theta_src, double* __restrict__ troubles,
-                                           const double* __restrict__ Weq) {
-  constexpr int V = D + 2, P_ = D + 1;
-  const long long q = B.id * (long long)blockDim.x + threadIdx.x;
-  if (q >= g.Nq) return;
-  int ix, iy, iz;
-  q_coords(g, q, ix, iy, iz);
-  const long long e = ext_of<D>(g, ix, iy, iz);
+static __device__ __forceinline__ double flag(const Geo& g, int pad, double min_rho, double max_rho, double min_P,
+                                              const unsigned char* __restrict__ mask,
+                                              const double* __restrict__ ext_new, const double* __restrict__ Weq,
+                                              long long q, long long e) {
+  constexpr int P_ = D + 1;
   const unsigned m = mask[q];
   const int pt0 = m & 1u, ptP = (m >> P_) & 1u;
   // max(pt0, ptP) as a double: constants, no conversion on the FP64 pipe
@@ -579,38 +610,64 @@ static __device__ __forceinline__ void run(Blk B, const Geo& g, int pad, double 
     t = fge(max_rho, r) ? t : 1.0;
     t = fge(P, min_P) ? t : 1.0;
   }
-  theta_src[e] = t;
-  troubles[q] = t;
-  const int a[3] = {ix, iy, iz};
-  for_ghosts<D>(g, a, [&](const int* x, const int* choice) {
+  return t;
+}
+static __device__ __forceinline__ void run(Blk B, const Geo& g, unsigned nb_main, int pad, double min_rho,
+                                           double max_rho, double min_P, const unsigned char* __restrict__ mask,
+                                           const int* __restrict__ flags, int sed, const double* __restrict__ ext_old,
+                                           const double* __restrict__ ext_new, const BcBufs& bc,
+                                           double* __restrict__ theta_src, double* __restrict__ troubles,
+                                           const double* __restrict__ Weq) {
+  constexpr int V = D + 2;
+  if (B.id >= nb_main) {
+    const long long i = (B.id - nb_main) * (long long)blockDim.x + threadIdx.x;
+    if (i >= n_ghosts<D>(g)) return;
+    const GhostPos p = ghost_pos<D>(g, i);
     const double* W = (sed && *flags != 0) ? ext_new : ext_old;
-    const long long xe = ext_at(g, x);
-    double th = t;
+    const long long xe = ext_at(g, p.e);
+    bool image = true;
     int last = 0;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      if (choice[d] < 0) continue;
-      if (g.bc[d][choice[d]] != BC_PERIODIC) th = W[xe];
+      if (p.side[d] < 0) continue;
+      image = image && g.bc[d][p.side[d]] == BC_PERIODIC;
       last = d;
     }
+    double th;
+    if (image) {
+      const long long q = (p.a[0] - NGH) + (long long)g.X[0] * ((D > 1 ? p.a[1] - NGH : 0) +
+                                                              (long long)g.X[1] * (D > 2 ? p.a[2] - NGH : 0));
+      th = flag(g, pad, min_rho, max_rho, min_P, mask, ext_new, Weq, q, ext_at(g, p.a));
+    } else {
+      th = W[xe];
+    }
     theta_src[xe] = th;
-    const int side = choice[last], kind = g.bc[last][side];
-    if (kind != BC_PERIODIC && kind != BC_REFLECTIVE && kind != BC_GRADFREE && kind != BC_EQ) return;
+    const int side = p.side[last], kind = g.bc[last][side];
+    if (fixed_bc(kind)) return;
     double* b = last == 0 ? bc.b[0] : (last == 1 ? bc.b[1] : bc.b[2]);
 #pragma unroll
     for (int v = 0; v < V; ++v)
-      b[bc_entry(g, last, side, V, v, x)] = (v == 0 && kind == BC_PERIODIC) ? th : W[(long long)v * g.Nqe + xe];
-  });
+      b[bc_entry(g, last, side, V, v, p.e)] = (v == 0 && kind == BC_PERIODIC) ? th : W[(long long)v * g.Nqe + xe];
+    return;
+  }
+  const long long q = B.id * (long long)blockDim.x + threadIdx.x;
+  if (q >= g.Nq) return;
+  int ix, iy, iz;
+  q_coords(g, q, ix, iy, iz);
+  const long long e = ext_of<D>(g, ix, iy, iz);
+  const double t = flag(g, pad, min_rho, max_rho, min_P, mask, ext_new, Weq, q, e);
+  theta_src[e] = t;
+  troubles[q] = t;
 }
 };
 template <int D>
-__global__ void k_troubles(Geo g, int pad, double min_rho, double max_rho, double min_P,
+__global__ void k_troubles(Geo g, unsigned nb_main, int pad, double min_rho, double max_rho, double min_P,
                            const unsigned char* __restrict__ mask, const int* __restrict__ flags, int sed,
                            const double* __restrict__ ext_old, const double* __restrict__ ext_new, BcBufs bc,
                            double* __restrict__ theta_src, double* __restrict__ troubles,
                            const double* __restrict__ Weq) {
-  Troubles<D>::run(hw_blk(), g, pad, min_rho, max_rho, min_P, mask, flags, sed, ext_old, ext_new, bc, theta_src,
-                   troubles, Weq);
+  Troubles<D>::run(hw_blk(), g, nb_main, pad, min_rho, max_rho, min_P, mask, flags, sed, ext_old, ext_new, bc,
+                   theta_src, troubles, Weq);
 }
 
 // extended-grid coordinates

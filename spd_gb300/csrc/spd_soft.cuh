@@ -14,8 +14,8 @@
 // nonzero and far from underflow and overflow (tested per line of values,
 // see Line), every other operand is multiplied by the FP64 unit.
 //
-// The build with fused multiply-adds keeps a*b + c as one FP64 instruction
-// and uses none of this.
+// The build with fused multiply-adds keeps a*b + c as one FP64 instruction;
+// it uses the quotients and roots only.
 #pragma once
 #include <cmath>
 #include <cstdint>
@@ -139,6 +139,7 @@ SPD_FN double coef_value(const Coef& c, uint32_t) { return c.a; }
 SPD_FN double coef_value(const Coef& c, uint32_t eoff) {
   return from_words(c.hi + eoff, (c.ml >> 10) | (c.mh << 22));
 }
+#endif
 // The product of the scaled significands of a coefficient-like operand
 // (mh:ml in [2^62, 2^63)) and an Opnd, in [2^115, 2^117): words 3:2 hold the
 // 53-bit result when bit 116 is set and one bit less otherwise; then the
@@ -210,9 +211,11 @@ SPD_FN double soft_round(Prod o, uint32_t keep) {
 #endif
   return from_words(o.w3 & keep, o.w2);
 }
+#ifndef SPD_FUSED
 SPD_FN double soft_prod(const Coef& c, const Opnd& x) {
   return soft_round(soft_words(c.ml, c.mh, c.e + x.e, x), x.keep);
 }
+#endif
 
 // A divisor b prepared for several quotients: 2^63 over its significand,
 // rounded down to within 4 units (so in [2^62, 2^63)), the quotient's
@@ -398,6 +401,5 @@ SPD_FN Num half(const Num& a) {
 SPD_FN Num ad_sqrt(const Num& a) { return Num(sqrt_soft(a.v), a.ok); }
 SPD_FN Num ad_abs(const Num& a) { return Num(from_words(hi_word(a.v) & 0x7fffffffu, lo_word(a.v)), a.ok); }
 SPD_FN double sval(const Num& a) { return a.v; }
-#endif  // SPD_FUSED
 
 }  // namespace spd

@@ -299,6 +299,12 @@ struct Stepper : StepperBase {
     return C->tape_aff + ((size_t)C->tape_step * C->T + i) * hist_aff_stride(C);
   }
 
+  // units of a key's upper word that lie within the relative tolerance (Nad)
+  static int nad_slack(const spd_config& cf) {
+    if (cf.NAD_delta || !(cf.tolerance * 0x1p20 > 2.0)) return -1;
+    return (int)std::ceil(std::min(cf.tolerance * 0x1p20, 1024.0)) - 2;
+  }
+
   int fv_update(spd_ctx* C) {
     const Geo& g = C->geo;
     const spd_config& cf = C->cfg;
@@ -315,6 +321,7 @@ struct Stepper : StepperBase {
     for (int d = 0; d < D; ++d) nface[d] = n_faces(g, d);
     const BcBufs bc{{C->bcbuf[0], C->bcbuf[1], C->bcbuf[2]}};
     const Counters counters{C->flags, C->counts};
+    const unsigned nb_q = blocks_for(g.Nq, BS), nb_ghost = blocks_for(n_ghosts<D>(g), BS);
     for (int i = 0; i < C->T; ++i) {
       const double w_i = C->ops.w_tp[i];
       if (C->recording)
@@ -326,7 +333,7 @@ struct Stepper : StepperBase {
         ProfScope ps_(C, "k_fv_candidate");
         launch<FvCandidate<D>>(C, "k_fv_candidate", k_fv_candidate<D>, blocks_for(g.Nq, BS), BS, 0, g, C->fvg, C->dt,
                                w_i, FH[0], FH[1], FH[2], C->U_cv, C->U_new, C->ext_old, C->ext_new,
-                               cf.FB ? (i == 0 ? 1 : 2) : 0, bc, counters, i == C->T - 1 ? C->W_cv : nullptr,
+                               cf.FB ? (i == 0 ? 1 : 2) : 0, counters, i == C->T - 1 ? C->W_cv : nullptr,
                                (const double*)C->gphi_fv, (const double*)C->Ueq_cv,
                                (const double*)C->Weq_cv);
       }
@@ -339,14 +346,19 @@ struct Stepper : StepperBase {
                              C->stream));
           off += (size_t)nface[d];
         }
+        // no detection, only the ghosts
+        launch<Nad<D>>(C, "k_nad", k_nad<D>, nb_ghost, BS, 0, g, 0u, bc, cf.tolerance, -1, cf.NAD_delta, 1, C->ext_old,
+                       C->ext_new, C->mask, C->flags, (long long*)nullptr, C->counts + 3);
+        CKL();
       } else if (cf.FB) {
         // detect_troubles (src/trouble_detection.py:5-87)
         const int sed = (P > 1 && cf.SED) ? 1 : 0;
         {
           ProfScope ps_(C, "k_nad");
           long long* sed_list = sed ? C->list_sed : nullptr;
-          launch<Nad<D>>(C, "k_nad", k_nad<D>, blocks_for(g.Nq, BS), BS, 0, g, cf.tolerance, cf.NAD_delta,
-                         P > 0 ? 1 : 0, C->ext_old, C->ext_new, C->mask, C->flags, sed_list, C->counts + 3);
+          launch<Nad<D>>(C, "k_nad", k_nad<D>, nb_q + nb_ghost, BS, 0, g, nb_q, bc, cf.tolerance, nad_slack(cf),
+                         cf.NAD_delta, P > 0 ? 1 : 0, C->ext_old, C->ext_new, C->mask, C->flags, sed_list,
+                         C->counts + 3);
         }
         CKL();
         if (sed) {
@@ -358,8 +370,8 @@ struct Stepper : StepperBase {
         }
         {
           ProfScope ps_(C, "k_troubles");
-          launch<Troubles<D>>(C, "k_troubles", k_troubles<D>, blocks_for(g.Nq, BS), BS, 0, g, cf.PAD, cf.min_rho,
-                              cf.max_rho, cf.min_P, C->mask, (const int*)C->flags, sed, (const double*)C->ext_old,
+          launch<Troubles<D>>(C, "k_troubles", k_troubles<D>, nb_q + nb_ghost, BS, 0, g, nb_q, cf.PAD,
+                              cf.min_rho, cf.max_rho, cf.min_P, C->mask, (const int*)C->flags, sed, (const double*)C->ext_old,
                               C->ext_new, bc, C->theta_src, C->troubles, (const double*)C->Weq_cv);
         }
         CKL();
