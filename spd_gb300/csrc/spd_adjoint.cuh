@@ -17,32 +17,13 @@ namespace spd {
 // ---------------------------------------------------------------------------
 // predictor
 // ---------------------------------------------------------------------------
-// Adjoint of one fused interior kernel launch (k_interior), one thread per
-// (cell c, time node t, direction d, transverse line j).  Input: the
-// adjoint of dudt (mode 0/1) or of the flux points (mode 2).  Output: the
-// line's share of the adjoint of this iteration's input U[t] (Upart[d],
-// written; each point of a cell lies on exactly one line per direction)
-// and the edge adjoints Ea of the line.
-template <int D, int P>
-__global__ void k_adj_interior(Ops op, Geo g, int mode, int Teff, const double* __restrict__ Uin, int Tu,
-                               const double* __restrict__ dudt_a, const double* Ffa0, const double* Ffa1,
-                               const double* Ffa2, double* Up0, double* Up1, double* Up2, double* Ea0, double* Ea1,
-                               double* Ea2) {
+template <int D, int P, int d>
+__device__ __forceinline__ void adj_interior_line(const Ops& op, const Geo& g, int mode, int Teff,
+                                                  const double* __restrict__ Uin, int Tu,
+                                                  const double* __restrict__ dudt_a, const double* __restrict__ Ffa,
+                                                  double* __restrict__ Up, double* __restrict__ Ea, unsigned nc,
+                                                  unsigned c, int j, int t, int tu) {
   using k = K<D, P>;
-  const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const unsigned nc = (unsigned)g.Nc;
-  if (tid >= (long long)nc * Teff * D * k::NJ) return;
-  const unsigned ut = (unsigned)tid;
-  const unsigned c = ut % nc;
-  unsigned rest = ut / nc;
-  const int j = (int)(rest % k::NJ);
-  rest /= k::NJ;
-  const int d = (int)(rest % D);
-  const int t = (int)(rest / D);
-  const int tu = (Tu == 1) ? 0 : t;
-  const double* Ffa = (d == 0) ? Ffa0 : (d == 1 ? Ffa1 : Ffa2);
-  double* Up = (d == 0) ? Up0 : (d == 1 ? Up1 : Up2);
-  double* Ea = (d == 0) ? Ea0 : (d == 1 ? Ea1 : Ea2);
   double Fla[k::V][k::nf];
   if (mode == 2) {
 #pragma unroll
@@ -62,7 +43,7 @@ __global__ void k_adj_interior(Ops op, Geo g, int mode, int Teff, const double* 
         const int s = sp_index<D, P>(d, j, so);
         const double da = dudt_a[(((long long)v * g.T + t) * k::NS + s) * nc + c] * rh;
 #pragma unroll
-        for (int f = 0; f < k::nf; ++f) Fla[v][f] += op.dfp_to_sp[so * k::nf + f] * da;
+        for (int f = 0; f < k::nf; ++f) Fla[v][f] = fma(op.dfp_to_sp[so * k::nf + f], da, Fla[v][f]);
       }
     }
   }
@@ -86,7 +67,9 @@ __global__ void k_adj_interior(Ops op, Geo g, int mode, int Teff, const double* 
     double M[k::V], W[k::V], Wa[k::V], Ma[k::V];
 #pragma unroll
     for (int v = 0; v < k::V; ++v) {
-      M[v] = dot_dir<k::n>(op.sp_to_fp + f * k::n, u[v], d);
+      M[v] = op.sp_to_fp[f * k::n] * u[v][0];
+#pragma unroll
+      for (int s = 1; s < k::n; ++s) M[v] = fma(op.sp_to_fp[f * k::n + s], u[v][s], M[v]);
       Wa[v] = 0.0;
       Ma[v] = 0.0;
     }
@@ -99,7 +82,7 @@ __global__ void k_adj_interior(Ops op, Geo g, int mode, int Teff, const double* 
 #pragma unroll
     for (int v = 0; v < k::V; ++v)
 #pragma unroll
-      for (int s = 0; s < k::n; ++s) acc[v][s] += op.sp_to_fp[f * k::n + s] * Ma[v];
+      for (int s = 0; s < k::n; ++s) acc[v][s] = fma(op.sp_to_fp[f * k::n + s], Ma[v], acc[v][s]);
   }
 #pragma unroll
   for (int v = 0; v < k::V; ++v)
@@ -108,11 +91,44 @@ __global__ void k_adj_interior(Ops op, Geo g, int mode, int Teff, const double* 
       Up[(((long long)v * Teff + t) * k::NS + sp_index<D, P>(d, j, s)) * nc + c] = acc[v][s];
 }
 
+// Adjoint of one fused interior kernel launch (k_interior), one thread per
+// (cell c, time node t, direction d, transverse line j).  Input: the
+// adjoint of dudt (mode 0/1) or of the flux points (mode 2).  Output: the
+// line's share of the adjoint of this iteration's input U[t] (Upart[d],
+// written; each point of a cell lies on exactly one line per direction)
+// and the edge adjoints Ea of the line.
+template <int D, int P>
+__global__ void k_adj_interior(Ops op, Geo g, int mode, int Teff, const double* __restrict__ Uin, int Tu,
+                               const double* __restrict__ dudt_a, const double* Ffa0, const double* Ffa1,
+                               const double* Ffa2, double* Up0, double* Up1, double* Up2, double* Ea0, double* Ea1,
+                               double* Ea2) {
+  using k = K<D, P>;
+  const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const unsigned nc = (unsigned)g.Nc;
+  if (tid >= (long long)nc * Teff * D * k::NJ) return;
+  const unsigned ut = (unsigned)tid;
+  const unsigned c = ut % nc;
+  unsigned rest = ut / nc;
+  const int j = (int)(rest % k::NJ);
+  rest /= k::NJ;
+  const int d = (int)(rest % D);
+  const int t = (int)(rest / D);
+  const int tu = (Tu == 1) ? 0 : t;
+  // the direction as a template argument: the rotated velocity indices are
+  // constants, not indices into local memory
+  if (d == 0)
+    adj_interior_line<D, P, 0>(op, g, mode, Teff, Uin, Tu, dudt_a, Ffa0, Up0, Ea0, nc, c, j, t, tu);
+  else if (D > 1 && d == 1)
+    adj_interior_line<D, P, (D > 1 ? 1 : 0)>(op, g, mode, Teff, Uin, Tu, dudt_a, Ffa1, Up1, Ea1, nc, c, j, t, tu);
+  else if (D > 2)
+    adj_interior_line<D, P, (D > 2 ? 2 : 0)>(op, g, mode, Teff, Uin, Tu, dudt_a, Ffa2, Up2, Ea2, nc, c, j, t, tu);
+}
+
 // Adjoint of the element-interface Riemann fluxes of direction d: the
 // interface adjoint is the sum of the edge adjoints of the cells that use
 // the flux; (ML, MR) adjoints go (atomically) to the traces they came from.
-template <int D, int P>
-__global__ void k_adj_riemann(Geo g, int d, int Teff, int solver, const double* __restrict__ trace,
+template <int D, int P, int d>
+__global__ void k_adj_riemann(Geo g, int Teff, int solver, const double* __restrict__ trace,
                               const double* __restrict__ bcfix, const double* __restrict__ Ea,
                               double* __restrict__ Tra) {
   using k = K<D, P>;
@@ -250,7 +266,7 @@ __global__ void k_adj_traces(Ops op, Geo g, int Teff, const double* __restrict__
       const int j = (d == 0) ? (ky + k::n * kz) : (d == 1 ? (kx + k::n * kz) : (kx + k::n * ky));
       const double l = Tra[d][(((long long)(0 * k::V + v) * g.T + t) * k::NJ + j) * nc + c];
       const double r = Tra[d][(((long long)(1 * k::V + v) * g.T + t) * k::NJ + j) * nc + c];
-      a += op.sp_to_fp[kd] * l + op.sp_to_fp[(k::nf - 1) * k::n + kd] * r;
+      a = fma(op.sp_to_fp[kd], l, fma(op.sp_to_fp[(k::nf - 1) * k::n + kd], r, a));
     }
     Ua[ui] = a;
   }
@@ -276,7 +292,8 @@ __global__ void k_adj_picard(Ops op, Geo g, const double* __restrict__ dt_ptr, c
   double tot = 0.0;
   for (int p = 0; p < g.T; ++p) {
     double a = 0.0;
-    for (int t = 0; t < g.T; ++t) a += op.invader[t * g.T + p] * Ua[(((long long)v * g.T + t) * k::NS + s) * g.Nc + c];
+    for (int t = 0; t < g.T; ++t)
+      a = fma(op.invader[t * g.T + p], Ua[(((long long)v * g.T + t) * k::NS + s) * g.Nc + c], a);
     a = -dt * a;
     if (collapse) tot += a;
     else dudt_a[(((long long)v * g.T + p) * k::NS + s) * g.Nc + c] = a;
@@ -336,7 +353,7 @@ __global__ void k_adj_cv_to_sp(Geo g, const double* __restrict__ Kfull, const do
   for (int in = 0; in < k::NS; ++in) {
     double s = 0.0;
 #pragma unroll
-    for (int o = 0; o < k::NS; ++o) s += Kfull[(long long)o * k::NS + in] * a[o];
+    for (int o = 0; o < k::NS; ++o) s = fma(Kfull[(long long)o * k::NS + in], a[o], s);
     const int kx = in % k::n, ky = (in / k::n) % k::n, kz = in / (k::n * k::n);
     const long long q = (cx * k::n + kx) + (long long)g.X[0] * ((D >= 2 ? cy * k::n + ky : 0) +
                                                                (long long)g.X[1] * (D >= 3 ? cz * k::n + kz : 0));
@@ -366,7 +383,7 @@ __global__ void k_adj_sp_to_cv(Geo g, const double* __restrict__ Kfull, const do
   for (int in = 0; in < k::NS; ++in) {
     double s = 0.0;
 #pragma unroll
-    for (int o = 0; o < k::NS; ++o) s += Kfull[(long long)o * k::NS + in] * a[o];
+    for (int o = 0; o < k::NS; ++o) s = fma(Kfull[(long long)o * k::NS + in], a[o], s);
     Usp_a[((long long)v * k::NS + in) * g.Nc + c] += s;
   }
 }
@@ -419,7 +436,7 @@ __global__ void k_adj_integrate_faces(Ops op, Geo g, int d, const double* __rest
           for (int b = 0; b < k::n; ++b) {
             double s = 0.0;
 #pragma unroll
-            for (int bo = 0; bo < k::n; ++bo) s += op.sp_to_cv[bo * k::n + b] * G[a + k::n * bo];
+            for (int bo = 0; bo < k::n; ++bo) s = fma(op.sp_to_cv[bo * k::n + b], G[a + k::n * bo], s);
             G1[a + k::n * b] = s;
           }
 #pragma unroll
@@ -433,7 +450,7 @@ __global__ void k_adj_integrate_faces(Ops op, Geo g, int d, const double* __rest
           for (int a = 0; a < k::n; ++a) {
             double s = 0.0;
 #pragma unroll
-            for (int ao = 0; ao < k::n; ++ao) s += op.sp_to_cv[ao * k::n + a] * G[ao + k::n * b];
+            for (int ao = 0; ao < k::n; ++ao) s = fma(op.sp_to_cv[ao * k::n + a], G[ao + k::n * b], s);
             G0[a + k::n * b] = s;
           }
 #pragma unroll
@@ -501,7 +518,7 @@ __device__ __forceinline__ void limiter_vjp(int limiter, double SL, double SR, d
   SLa = 0.0;
   SRa = 0.0;
   if (limiter == LIM_MINMOD) {
-    const double ratio = SR / SL;
+    const double ratio = quot(SR, SL);
     if (ratio < 1.0) {
       if (ratio > 0.0) SRa = a;  // ratio * SL = SR
     } else {
@@ -510,8 +527,9 @@ __device__ __forceinline__ void limiter_vjp(int limiter, double SL, double SR, d
     return;
   }
   if (!(SL * SR >= 0.0)) return;
-  const double dUC = (hl * SL + hr * SR) / (hl + hr);
-  const double q1 = 2.0 * SL * hl / hm, q2 = 2.0 * SR * hr / hm;
+  const Rcp rs = recip_of(hl + hr), rm = recip_of(hm);
+  const double dUC = div_by(hl * SL + hr * SR, hl + hr, rs);
+  const double q1 = div_by(2.0 * SL * hl, hm, rm), q2 = div_by(2.0 * SR * hr, hm, rm);
   const double c1 = fabs(q1), c2 = fabs(q2), c3 = fabs(dUC);
   const double sg = sign0(dUC);
   // slope = sg * min(min(c1, c2), c3): the derivative weight of each
@@ -525,10 +543,10 @@ __device__ __forceinline__ void limiter_vjp(int limiter, double SL, double SR, d
   if (c1 == c2) { w1 = 0.5 * wm; w2 = 0.5 * wm; }
   else if (c1 < c2 || c1 != c1) { w1 = wm; w2 = 0.0; }
   else { w1 = 0.0; w2 = wm; }
-  const double dq1 = sign0(q1) * 2.0 * hl / hm, dq2 = sign0(q2) * 2.0 * hr / hm;
+  const double dq1 = div_by(sign0(q1) * 2.0 * hl, hm, rm), dq2 = div_by(sign0(q2) * 2.0 * hr, hm, rm);
   const double s3 = sign0(dUC);
-  SLa = sg * (w1 * dq1 + w3 * s3 * hl / (hl + hr)) * a;
-  SRa = sg * (w2 * dq2 + w3 * s3 * hr / (hl + hr)) * a;
+  SLa = sg * (w1 * dq1 + div_by(w3 * s3 * hl, hl + hr, rs)) * a;
+  SRa = sg * (w2 * dq2 + div_by(w3 * s3 * hr, hl + hr, rs)) * a;
 }
 
 // Limited gradients of extended cell e in every direction (the forward's
@@ -570,7 +588,7 @@ SPD_FN void predictor_vjp(const double* W, const double (*dMh)[D + 2], double dt
     dta[v] = 0.5 * dti * pra[v];
   }
   dta[P_] = 0.0;
-  const double rw0 = 1.0 / W[0];
+  const double rw0 = quot(1.0, W[0]);
   for (int dd = 0; dd < D; ++dd) {
     const int vel = dd + 1;
     double* dma = in_a + V + dd * V;
@@ -643,8 +661,8 @@ __device__ __forceinline__ void adj_muscl_riemann_face(const Geo& g, int d, int 
   }
 }
 
-template <int D>
-__global__ void k_adj_muscl_riemann(Geo g, int d, int solver, const long long* __restrict__ list,
+template <int D, int d>
+__global__ void k_adj_muscl_riemann(Geo g, int solver, const long long* __restrict__ list,
                                     const unsigned long long* __restrict__ count, const double* __restrict__ Mpred,
                                     const double* __restrict__ S, const double* __restrict__ Fba,
                                     double* __restrict__ FA) {

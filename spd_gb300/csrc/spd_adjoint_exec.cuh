@@ -38,8 +38,10 @@ int adj_iteration(spd_ctx* C, int mode, const double* Uin, int Tu, int Teff) {
     CK(cudaMemsetAsync(C->Tra[d], 0, sizeof(double) * 2 * k::V * g.T * k::NJ * g.Nc, C->stream));
     const long long tot = (long long)Teff * k::NJ * n_iface(g, d);
     ProfScope ps_(C, "k_adj_riemann");
-    k_adj_riemann<D, P><<<blocks_for(tot, 64), 64, 0, C->stream>>>(g, d, Teff, C->cfg.riemann_solver_sd,
-                                                                  C->trace[d], C->bcfix[d], C->Ea[d], C->Tra[d]);
+    auto kern = d == 0 ? k_adj_riemann<D, P, 0>
+                       : (d == 1 ? k_adj_riemann<D, P, (D > 1 ? 1 : 0)> : k_adj_riemann<D, P, (D > 2 ? 2 : 0)>);
+    kern<<<blocks_for(tot, 64), 64, 0, C->stream>>>(g, Teff, C->cfg.riemann_solver_sd, C->trace[d], C->bcfix[d],
+                                                    C->Ea[d], C->Tra[d]);
     CKL();
   }
   {
@@ -139,9 +141,11 @@ int adjoint_vjp(spd_ctx* C) {
           ProfScope ps_(C, "k_adj_muscl_riemann");
           const double* mp = C->hist_mpred + (size_t)i * (1 + D) * k::V * g.Nqe;
           const unsigned nb = (unsigned)std::min<long long>(PERSIST_BLOCKS, blocks_for(nface[d], 64));
-          k_adj_muscl_riemann<D><<<nb, 64, 0, C->stream>>>(g, d, cf.riemann_solver_fv, C->list_face[d],
-                                                           C->counts + 4 + d, mp, mp + (size_t)k::V * g.Nqe,
-                                                           C->Fba[d], C->FA[d]);
+          auto kern = d == 0 ? k_adj_muscl_riemann<D, 0>
+                             : (d == 1 ? k_adj_muscl_riemann<D, (D > 1 ? 1 : 0)>
+                                       : k_adj_muscl_riemann<D, (D > 2 ? 2 : 0)>);
+          kern<<<nb, 64, 0, C->stream>>>(g, cf.riemann_solver_fv, C->list_face[d], C->counts + 4 + d, mp,
+                                         mp + (size_t)k::V * g.Nqe, C->Fba[d], C->FA[d]);
           CKL();
         }
         // W_a and LA are zero on the cells that border no used face

@@ -514,6 +514,53 @@ SPD_FN void hllc(const S* WL, const S* WR, const S* UL, const S* UR, S* F, doubl
   if (iso) F[P_] = F[P_] * 0.0;
 }
 
+// U -> W (plain velocity order) and the Euler flux along direction d in the
+// rotated frame, in 1D and 2D with their products on the integer pipes as
+// above: k_interior 11.2 -> 10.6 ms and k_fv_candidate 1.22 -> 1.14 ms at
+// 512^2, p=3.  In 3D the integer pipes are the busier ones already (48^3,
+// p=2: 7.45 -> 7.87 and 1.2 -> 1.31 ms), so their products stay FP64.
+template <int D>
+struct NumEuler {
+#if defined(__CUDA_ARCH__) && !defined(SPD_FUSED)
+  static constexpr bool value = D <= 2;
+#else
+  static constexpr bool value = false;
+#endif
+};
+#if defined(__CUDA_ARCH__)
+template <int D>
+__device__ __noinline__ void prim_slow(const double* U, double* W, double gamma, int idim_order, bool iso) {
+  prim<D>(U, W, gamma, idim_order, nullptr, iso);
+}
+#endif
+template <int D>
+SPD_FN void prim_num(const double* U, double* W, double gamma, int idim_order, Recip* r0, bool iso) {
+  constexpr int V = D + 2;
+  Num u[V], w[V];
+  uint32_t ok = 0x40000000u;
+#pragma unroll
+  for (int v = 0; v < V; ++v) u[v] = Num(U[v]);
+  prim<D>(u, w, gamma, idim_order, r0, iso);
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    ok &= w[v].ok;
+    W[v] = w[v].v;
+  }
+#if defined(__CUDA_ARCH__)
+  if (ok != 0u) return;
+  double us[V], ws[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) us[v] = U[v];
+  prim_slow<D>(us, ws, gamma, idim_order, iso);
+#pragma unroll
+  for (int v = 0; v < V; ++v) W[v] = ws[v];
+#endif
+}
+template <int D>
+SPD_FN void prims(const double* U, double* W, double gamma, bool iso) {
+  if constexpr (NumEuler<D>::value) prim_num<D>(U, W, gamma, 0, nullptr, iso);
+  else prim<D>(U, W, gamma, 0, nullptr, iso);
+}
 // the solver of a kernel instantiated for SV
 template <int SV>
 SPD_FN int solver_of(int solver) {
@@ -553,8 +600,19 @@ SPD_FN void riemann(int solver, const S* ML, const S* MR, S* F, double gamma, do
   } else {
 #pragma unroll
     for (int v = 0; v < V; ++v) { UL[v] = ML[v]; UR[v] = MR[v]; }
-    prim<D>(UL, WL, gamma, idim, &rL, iso);
-    prim<D>(UR, WR, gamma, idim, &rR, iso);
+    bool done = false;
+    if constexpr (BM == 0 && std::is_same<S, double>::value && NumEuler<D>::value) {
+      if (solver != RS_LLF) {
+        // the conversions' products on the integer pipes, HLLC's own not
+        prim_num<D>(UL, WL, gamma, idim, &rL, iso);
+        prim_num<D>(UR, WR, gamma, idim, &rR, iso);
+        done = true;
+      }
+    }
+    if (!done) {
+      prim<D>(UL, WL, gamma, idim, &rL, iso);
+      prim<D>(UR, WR, gamma, idim, &rR, iso);
+    }
     prL = &rL;
     prR = &rR;
   }
@@ -602,20 +660,7 @@ SPD_FN void riemann(int solver, const S* ML, const S* MR, S* F, double gamma, do
   else hllc<D, S, BM>(WL, WR, UL, UR, F, gamma, min_c2, idim, solver == RS_LHLLC, br, prL, prR, iso);
 }
 
-// U -> W (plain velocity order) and the Euler flux along direction d in the
-// rotated frame, in 1D and 2D with their products on the integer pipes as
-// above: k_interior 11.2 -> 10.6 ms and k_fv_candidate 1.22 -> 1.14 ms at
-// 512^2, p=3.  In 3D the integer pipes are the busier ones already (48^3,
-// p=2: 7.45 -> 7.87 and 1.2 -> 1.31 ms), so their products stay FP64.
-template <int D>
-constexpr bool num_euler() {
-#if defined(__CUDA_ARCH__) && !defined(SPD_FUSED)
-  return D <= 2;
-#else
-  return false;
-#endif
-}
-#if defined(__CUDA_ARCH__) && !defined(SPD_FUSED)
+#if defined(__CUDA_ARCH__)
 template <int D>
 __device__ __noinline__ void euler_slow(const double* U, double* W, double* F, double gamma, int d, bool iso) {
   prim<D>(U, W, gamma, 0, nullptr, iso);
@@ -632,42 +677,11 @@ __device__ __noinline__ void euler_slow(const double* U, double* W, double* F, d
   for (int q = 0; q < D; ++q) F[rvel<D>(d, q)] = Fr[1 + q];
 }
 #endif
-template <int D>
-SPD_FN void prims(const double* U, double* W, double gamma, bool iso) {
-  constexpr int V = D + 2;
-#if defined(__CUDA_ARCH__) && !defined(SPD_FUSED)
-  if constexpr (num_euler<D>()) {
-    Num u[V], w[V];
-    uint32_t ok = 0x40000000u;
-#pragma unroll
-    for (int v = 0; v < V; ++v) u[v] = Num(U[v]);
-    prim<D>(u, w, gamma, 0, nullptr, iso);
-#pragma unroll
-    for (int v = 0; v < V; ++v) {
-      ok &= w[v].ok;
-      W[v] = w[v].v;
-    }
-    if (ok != 0u) return;
-    double us[V], ws[V];
-#pragma unroll
-    for (int v = 0; v < V; ++v) us[v] = U[v];
-    euler_slow<D>(us, ws, nullptr, gamma, 0, iso);
-#pragma unroll
-    for (int v = 0; v < V; ++v) W[v] = ws[v];
-    return;
-  }
-#endif
-  prim<D>(U, W, gamma, 0, nullptr, iso);
-}
 // flux of the conservative state U; store(v, F_v) takes its components
 template <int D, class Store>
 SPD_FN void euler_flux(const double* U, double gamma, int d, bool iso, const Rcp* rg, Store store) {
   constexpr int V = D + 2;
-#if defined(__CUDA_ARCH__) && !defined(SPD_FUSED)
-  using S = typename std::conditional<num_euler<D>(), Num, double>::type;
-#else
-  using S = double;
-#endif
+  using S = typename std::conditional<NumEuler<D>::value, Num, double>::type;
   // the velocities in the rotated order of direction d, as flux's own order
   // for direction 0
   S u[V], w[V], wr[V], f[V];
@@ -684,8 +698,8 @@ SPD_FN void euler_flux(const double* U, double gamma, int d, bool iso, const Rcp
     wr[1 + q] = x;
   }
   flux<D>(wr, f, gamma, 0, iso, rg);
-#if defined(__CUDA_ARCH__) && !defined(SPD_FUSED)
-  if constexpr (num_euler<D>()) {
+#if defined(__CUDA_ARCH__)
+  if constexpr (NumEuler<D>::value) {
     uint32_t ok = 0x40000000u;
 #pragma unroll
     for (int v = 0; v < V; ++v) ok &= f[v].ok;

@@ -20,6 +20,9 @@ namespace spd {
 // barriers overlap
 constexpr int INTERIOR_THREADS = 256;
 constexpr int INTERIOR_BLOCKS = 3;
+// the tile of 3D at degree 4 leaves room for two, and 128 registers
+template <int D, int P>
+constexpr int interior_blocks = (D == 3 && P == 4) ? 2 : INTERIOR_BLOCKS;
 
 struct Ops {
   double sp_to_fp[MAXNF * MAXN];
@@ -597,7 +600,7 @@ static __device__ __forceinline__ void run(Blk B, const Ops& op, const Geo& g, i
 }
 };
 template <int D, int P>
-__global__ void __launch_bounds__(INTERIOR_THREADS, INTERIOR_BLOCKS) k_interior(Ops op, Geo g, int mode, int Teff, int chunk, const double* __restrict__ Uin, int Tu,
+__global__ void __launch_bounds__(INTERIOR_THREADS, (interior_blocks<D, P>)) k_interior(Ops op, Geo g, int mode, int Teff, int chunk, const double* __restrict__ Uin, int Tu,
                            const double* __restrict__ dt_ptr, double* __restrict__ U_sp, double* __restrict__ U_ader,
                            const double* Fi0, const double* Fi1, const double* Fi2, double* tr0, double* tr1,
                            double* tr2, double* Ffp0, double* Ffp1, double* Ffp2) {
@@ -620,7 +623,7 @@ struct InteriorExt {
   }
 };
 template <int D, int P>
-__global__ void __launch_bounds__(INTERIOR_THREADS, INTERIOR_BLOCKS) k_interior_ext(Ops op, Geo g, int mode, int Teff, int chunk, const double* __restrict__ Uin, int Tu,
+__global__ void __launch_bounds__(INTERIOR_THREADS, (interior_blocks<D, P>)) k_interior_ext(Ops op, Geo g, int mode, int Teff, int chunk, const double* __restrict__ Uin, int Tu,
                                const double* __restrict__ dt_ptr, double* __restrict__ U_sp,
                                double* __restrict__ U_ader, const double* Fi0, const double* Fi1, const double* Fi2,
                                double* tr0, double* tr1, double* tr2, double* Ffp0, double* Ffp1, double* Ffp2,

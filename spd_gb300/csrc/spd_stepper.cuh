@@ -485,32 +485,34 @@ struct Stepper : StepperBase {
 
   void k_muscl_cells_grid(spd_ctx* C, double w_i, int i) {
     const Geo& g = C->geo;
-    const long long nb = std::min<long long>(PERSIST_BLOCKS, blocks_for(g.Nqe, 128));
+    const long long nb = std::min<long long>(2 * PERSIST_BLOCKS, blocks_for(g.Nqe, LIST_CELLS));
+    const dim3 block(LIST_CELLS, k::V);
     ProfScope ps_(C, "k_muscl_cells");
     if (C->tape_mode == 0) {
       unsigned char* no_tape = nullptr;
-      launch<MusclCells<D>>(C, "k_muscl_cells", k_muscl_cells<D>, (unsigned)nb, 128, 0, g, C->fvg,
+      launch<MusclCells<D>>(C, "k_muscl_cells", k_muscl_cells<D>, (unsigned)nb, block, 0, g, C->fvg,
                             C->cfg.slope_limiter, C->dt, w_i, C->list_cell, C->counts, C->ext_old, C->Mpred, C->S,
                             no_tape, (const double*)C->Meq_fv, (const double*)C->gphi_fv);
       return;
     }
     unsigned char* lt = C->tape_lim + ((size_t)C->tape_step * C->T + i) * D * k::V * g.Nqe;
     if (C->tape_mode == 1)
-      k_muscl_cells<D, 1><<<(unsigned)nb, 128, 0, C->stream>>>(g, C->fvg, C->cfg.slope_limiter, C->dt, w_i,
+      k_muscl_cells<D, 1><<<(unsigned)nb, block, 0, C->stream>>>(g, C->fvg, C->cfg.slope_limiter, C->dt, w_i,
                                                                C->list_cell, C->counts, C->ext_old, C->Mpred, C->S, lt,
                                                                nullptr, nullptr);
     else
-      k_muscl_cells<D, 2><<<(unsigned)nb, 128, 0, C->stream>>>(g, C->fvg, C->cfg.slope_limiter, C->dt, w_i,
+      k_muscl_cells<D, 2><<<(unsigned)nb, block, 0, C->stream>>>(g, C->fvg, C->cfg.slope_limiter, C->dt, w_i,
                                                                C->list_cell, C->counts, C->ext_old, C->Mpred, C->S, lt,
                                                                nullptr, nullptr);
   }
 
   void k_fv_correct_grid(spd_ctx* C, double w_i, const double* const* FH, double* W_cv) {
     const Geo& g = C->geo;
-    const long long nb = std::min<long long>(PERSIST_BLOCKS, blocks_for(g.Nq, 128));
+    const long long nb = std::min<long long>(2 * PERSIST_BLOCKS, blocks_for(g.Nq, LIST_CELLS));
+    const dim3 block(LIST_CELLS, k::V);
     {
       ProfScope ps_(C, "k_fv_correct");
-      launch<FvCorrect<D>>(C, "k_fv_correct", k_fv_correct<D>, (unsigned)nb, 128, 0, g, C->fvg, C->dt, w_i,
+      launch<FvCorrect<D>>(C, "k_fv_correct", k_fv_correct<D>, (unsigned)nb, block, 0, g, C->fvg, C->dt, w_i,
                            C->cfg.godunov, C->list_q, C->counts + 1, FH[0], FH[1], FH[2], C->F_FB[0], C->F_FB[1],
                            C->F_FB[2], C->aff[0], C->aff[1], C->aff[2], C->U_cv, C->U_new, C->ext_new, W_cv,
                            (const double*)C->gphi_fv, (const double*)C->Ueq_cv, (const double*)C->Weq_cv);

@@ -21,23 +21,23 @@ template <int D>
 SPD_FN void prim_vjp_add(const double* U, const double* Wa, double* Ua, double gamma) {
   constexpr int P_ = D + 1;
   const double r = U[0];
-  const double rr = 1.0 / r;
+  const double rr = quot(1.0, r);
   double w[D + 2], ks = 0.0;
 #pragma unroll
   for (int v = 1; v <= D; ++v) {
     w[v] = U[v] * rr;
-    ks += w[v] * w[v];
+    ks = fma(w[v], w[v], ks);
   }
   const double Pa = Wa[P_];
-  Ua[P_] += (gamma - 1.0) * Pa;
   const double Ka = -(gamma - 1.0) * Pa;
-  const double ksa = Ka * 0.5 * r;
-  double ra = Wa[0] + Ka * 0.5 * ks;
+  Ua[P_] -= Ka;
+  const double ksa = 0.5 * Ka * r;
+  double ra = fma(0.5 * Ka, ks, Wa[0]);
 #pragma unroll
   for (int v = 1; v <= D; ++v) {
-    const double wa = (Wa[v] + 2.0 * w[v] * ksa) * rr;
+    const double wa = fma(2.0 * w[v], ksa, Wa[v]) * rr;
     Ua[v] += wa;
-    ra -= wa * w[v];
+    ra = fma(-wa, w[v], ra);
   }
   Ua[0] += ra;
 }
@@ -49,14 +49,15 @@ SPD_FN void cons_vjp_add(const double* W, const double* Ua, double* Wa, double g
   const double r = W[0];
   double ks = 0.0;
 #pragma unroll
-  for (int v = 1; v <= D; ++v) ks += W[v] * W[v];
-  Wa[P_] += Ua[P_] * (1.0 / (gamma - 1.0));
-  const double ksa = Ua[P_] * 0.5 * r;
-  double ra = Ua[0] + Ua[P_] * 0.5 * ks;
+  for (int v = 1; v <= D; ++v) ks = fma(W[v], W[v], ks);
+  Wa[P_] = fma(Ua[P_], quot(1.0, gamma - 1.0), Wa[P_]);
+  const double ha = 0.5 * Ua[P_];
+  const double ksa = ha * r;
+  double ra = fma(ha, ks, Ua[0]);
 #pragma unroll
   for (int v = 1; v <= D; ++v) {
-    Wa[v] += 2.0 * W[v] * ksa + Ua[v] * r;
-    ra += Ua[v] * W[v];
+    Wa[v] += fma(2.0 * W[v], ksa, Ua[v] * r);
+    ra = fma(Ua[v], W[v], ra);
   }
   Wa[0] += ra;
 }
@@ -69,38 +70,39 @@ SPD_FN void flux_vjp_add(const double* W, const double* Fa, double* Wa, double g
   const double r = W[0], u = W[v1], P = W[P_];
   double ks = 0.0;
 #pragma unroll
-  for (int v = 1; v <= D; ++v) ks += W[v] * W[v];
-  const double rg = 1.0 / (gamma - 1.0);
-  const double E = P * rg + 0.5 * r * ks;
-  double ra = Fa[0] * u + Fa[v1] * u * u;
-  double ua = Fa[0] * r + Fa[v1] * 2.0 * r * u + Fa[P_] * (E + P);
-  double Pa = Fa[v1] + Fa[P_] * u;
+  for (int v = 1; v <= D; ++v) ks = fma(W[v], W[v], ks);
+  const double rg = quot(1.0, gamma - 1.0);
+  const double hk = 0.5 * ks;
+  const double E = fma(P, rg, r * hk);
   const double Ea = Fa[P_] * u;
+  const double m1 = Fa[v1] * u;
+  double ra = fma(Ea, hk, fma(m1, u, Fa[0] * u));
+  double ua = fma(Fa[P_], E + P, fma(2.0 * r, m1, Fa[0] * r));
+  const double Ear = Ea * r;
 #pragma unroll
   for (int k = 1; k < D; ++k) {
     const int vt = rvel<D>(idim, k);
-    ra += Fa[vt] * W[vt] * u;
-    ua += Fa[vt] * r * W[vt];
-    Wa[vt] += Fa[vt] * r * u;
+    const double a = Fa[vt] * W[vt], b = Fa[vt] * r;
+    ra = fma(a, u, ra);
+    ua = fma(a, r, ua);
+    Wa[vt] = fma(b, u, Wa[vt]);
   }
-  Pa += Ea * rg;
-  ra += Ea * 0.5 * ks;
 #pragma unroll
-  for (int v = 1; v <= D; ++v) Wa[v] += Ea * r * W[v];
+  for (int v = 1; v <= D; ++v) Wa[v] = fma(Ear, W[v], Wa[v]);
   Wa[0] += ra;
   Wa[v1] += ua;
-  Wa[P_] += Pa;
+  Wa[P_] += fma(Ea, rg, fma(Fa[P_], u, Fa[v1]));
 }
 
 // c = sound_speed(P, rho) (floored): adds dc/dP * ca, dc/drho * ca
 SPD_FN void sound_speed_vjp_add(double P, double rho, double gamma, double min_c2, double ca, double& Pa,
                                 double& ra) {
-  const double rr = 1.0 / rho;
-  const double c2 = div_rcp(gamma * P, rho, rr);  // the forward's quotient (decides the floor)
-  if (!(c2 > min_c2)) return;
-  const double c2a = ca * (0.5 / sqrt(c2));
-  Pa += c2a * gamma * rr;
-  ra -= c2a * c2 * rr;
+  const Rcp q = recip_of(rho);
+  const double c2 = div_by(gamma * P, rho, q);  // the forward's quotient (decides the floor)
+  if (!fgt(c2, min_c2)) return;
+  const double x = ca * quot(0.5, ad_sqrt(c2)) * div_by(1.0, rho, q);
+  Pa = fma(x, gamma, Pa);
+  ra = fma(-x, c2, ra);
 }
 
 // LLF / HLLC flux F(ML, MR): (MLa, MRa) = J^T Fa (written).  prims: the
@@ -127,7 +129,7 @@ SPD_FN void riemann_vjp_rev(int solver, const double* ML, const double* MR, cons
   for (int v = 0; v < V; ++v) { WLa[v] = 0.0; WRa[v] = 0.0; ULa[v] = 0.0; URa[v] = 0.0; }
   const double cL = sound_speed(WL[P_], WL[0], gamma, min_c2) + fabs(WL[v1]);
   const double cR = sound_speed(WR[P_], WR[0], gamma, min_c2) + fabs(WR[v1]);
-  const bool Lmax = cL > cR;
+  const bool Lmax = fgt(cL, cR);
   const double cmax = Lmax ? cL : cR;
   double cmax_a = 0.0;
   if (solver == RS_LLF) {
@@ -146,52 +148,54 @@ SPD_FN void riemann_vjp_rev(int solver, const double* ML, const double* MR, cons
   } else {
     const bool low_mach = solver == RS_LHLLC;
     const double vL = WL[v1], vR = WR[v1];
-    const bool minL = vL < vR, maxL = vL > vR;
+    const bool minL = fgt(vR, vL), maxL = fgt(vL, vR);
     const double sL = (minL ? vL : vR) - cmax;
     const double sR = (maxL ? vL : vR) + cmax;
     const double rcL = WL[0] * (vL - sL);
     const double rcR = WR[0] * (sR - vR);
     const double den = rcR + rcL;
-    const double rden = 1.0 / den;
-    const double vstar = div_rcp(rcR * vR + rcL * vL + (WL[P_] - WR[P_]), den, rden);
+    const Rcp qden = recip_of(den);
+    const double rden = div_by(1.0, den, qden);
+    const double vstar = div_by(rcR * vR + rcL * vL + (WL[P_] - WR[P_]), den, qden);
     double phi = 1.0, Mach = 0.0, mx = 0.0;
     if (low_mach) {
-      mx = np_max(fabs(vL), fabs(vR)) / cmax;
+      mx = quot(np_max(fabs(vL), fabs(vR)), cmax);
       Mach = np_min(1.0, mx);
       phi = Mach * (2.0 - Mach);
     }
-    const double Pstar = low_mach ? div_rcp(rcR * WL[P_] + rcL * WR[P_] + phi * rcL * rcR * (vL - vR), den, rden)
-                                  : div_rcp(rcR * WL[P_] + rcL * WR[P_] + rcL * rcR * (vL - vR), den, rden);
+    const double Pstar = low_mach ? div_by(rcR * WL[P_] + rcL * WR[P_] + phi * rcL * rcR * (vL - vR), den, qden)
+                                  : div_by(rcR * WL[P_] + rcL * WR[P_] + rcL * rcR * (vL - vR), den, qden);
     int region;
     double r, vg, Pg, e, dd = 1.0, rdd = 1.0;
-    if (sL > 0.0) {
+    if (fgt(sL, 0.0)) {
       region = 0; r = WL[0]; vg = vL; Pg = WL[P_]; e = UL[P_];
-    } else if (vstar > 0.0 || sR > 0.0) {
+    } else if (fgt(vstar, 0.0) || fgt(sR, 0.0)) {
       // left (region 1) and right (region 2) star states: one path with
       // per-lane operands (both sides of a warp evaluate it once)
-      const bool lft = vstar > 0.0;
+      const bool lft = fgt(vstar, 0.0);
       region = lft ? 1 : 2;
       const double s = lft ? sL : sR, v = lft ? vL : vR;
       const double w0 = lft ? WL[0] : WR[0], wP = lft ? WL[P_] : WR[P_], uP = lft ? UL[P_] : UR[P_];
       dd = s - vstar;
-      rdd = 1.0 / dd;
-      r = div_rcp(w0 * (s - v), dd, rdd);
-      e = div_rcp((s - v) * uP - wP * v + Pstar * vstar, dd, rdd);
+      const Rcp qd = recip_of(dd);
+      rdd = div_by(1.0, dd, qd);
+      r = div_by(w0 * (s - v), dd, qd);
+      e = div_by((s - v) * uP - wP * v + Pstar * vstar, dd, qd);
       vg = vstar; Pg = Pstar;
     } else {
       region = 3; r = WR[0]; vg = vR; Pg = WR[P_]; e = UR[P_];
     }
     const double F0 = r * vg;
-    const bool left = vstar > 0.0;
+    const bool left = fgt(vstar, 0.0);
     // reverse of the flux assembly
     double F0a = Fa[0] + Fa[v1] * vg;
 #pragma unroll
     for (int k = 1; k < D; ++k) {
       const int vt = rvel<D>(idim, k);
       const double wv = left ? WL[vt] : WR[vt];
-      F0a += Fa[vt] * wv;
-      if (left) WLa[vt] += Fa[vt] * F0;
-      else WRa[vt] += Fa[vt] * F0;
+      F0a = fma(Fa[vt], wv, F0a);
+      if (left) WLa[vt] = fma(Fa[vt], F0, WLa[vt]);
+      else WRa[vt] = fma(Fa[vt], F0, WRa[vt]);
     }
     const double ra = F0a * vg;
     const double vga = F0a * r + Fa[v1] * F0 + Fa[P_] * (e + Pg);
@@ -223,7 +227,7 @@ SPD_FN void riemann_vjp_rev(int solver, const double* ML, const double* MR, cons
       vK_a += -na * EK - na * PK;
       const double EK_a = na * (sK - vK);
       const double PK_a = -na * vK;
-      Pstar_a += na * vstar;
+      Pstar_a = fma(na, vstar, Pstar_a);
       if (isL) {
         WLa[0] += rho_a; vL_a += vK_a; sL_a += sK_a; ULa[P_] += EK_a; WLa[P_] += PK_a;
       } else {
@@ -234,11 +238,11 @@ SPD_FN void riemann_vjp_rev(int solver, const double* ML, const double* MR, cons
     double rcL_a = 0.0, rcR_a = 0.0, den_a = 0.0;
     {
       const double na = Pstar_a * rden;
-      den_a -= na * Pstar;
+      den_a = fma(-na, Pstar, den_a);
       rcR_a += na * WL[P_] + na * phi * rcL * (vL - vR);
       rcL_a += na * WR[P_] + na * phi * rcR * (vL - vR);
-      WLa[P_] += na * rcR;
-      WRa[P_] += na * rcL;
+      WLa[P_] = fma(na, rcR, WLa[P_]);
+      WRa[P_] = fma(na, rcL, WRa[P_]);
       vL_a += na * phi * rcL * rcR;
       vR_a -= na * phi * rcL * rcR;
       if (low_mach) {
@@ -248,9 +252,9 @@ SPD_FN void riemann_vjp_rev(int solver, const double* ML, const double* MR, cons
         const double wmx = (mx == 1.0) ? 0.5 : ((1.0 <= mx || mx != mx) ? 0.0 : 1.0);
         const double mx_a = Mach_a * wmx;
         // mx = np_max(|vL|, |vR|) / cmax
-        cmax_a -= mx_a * mx / cmax;
+        cmax_a -= quot(mx_a * mx, cmax);
         const double aL = fabs(vL), aR = fabs(vR);
-        const double m_a = mx_a / cmax;
+        const double m_a = quot(mx_a, cmax);
         double wL, wR;
         if (aL == aR) { wL = 0.5; wR = 0.5; }
         else if (aL >= aR || aL != aL) { wL = 1.0; wR = 0.0; }
@@ -262,11 +266,11 @@ SPD_FN void riemann_vjp_rev(int solver, const double* ML, const double* MR, cons
     // vstar = (rcR vR + rcL vL + (PL - PR)) / den
     {
       const double na = vstar_a * rden;
-      den_a -= na * vstar;
-      rcR_a += na * vR;
-      rcL_a += na * vL;
-      vR_a += na * rcR;
-      vL_a += na * rcL;
+      den_a = fma(-na, vstar, den_a);
+      rcR_a = fma(na, vR, rcR_a);
+      rcL_a = fma(na, vL, rcL_a);
+      vR_a = fma(na, rcR, vR_a);
+      vL_a = fma(na, rcL, vL_a);
       WLa[P_] += na;
       WRa[P_] -= na;
     }
@@ -274,11 +278,11 @@ SPD_FN void riemann_vjp_rev(int solver, const double* ML, const double* MR, cons
     rcL_a += den_a;
     // rcL = rhoL (vL - sL); rcR = rhoR (sR - vR)
     WLa[0] += rcL_a * (vL - sL);
-    vL_a += rcL_a * WL[0];
-    sL_a -= rcL_a * WL[0];
+    vL_a = fma(rcL_a, WL[0], vL_a);
+    sL_a = fma(-rcL_a, WL[0], sL_a);
     WRa[0] += rcR_a * (sR - vR);
-    sR_a += rcR_a * WR[0];
-    vR_a -= rcR_a * WR[0];
+    sR_a = fma(rcR_a, WR[0], sR_a);
+    vR_a = fma(-rcR_a, WR[0], vR_a);
     // sL = min-select(vL, vR) - cmax; sR = max-select(vL, vR) + cmax
     if (minL) vL_a += sL_a; else vR_a += sL_a;
     cmax_a -= sL_a;
