@@ -339,8 +339,9 @@ int spd_create(const spd_config* cfg, const spd_operators* ops, spd_ctx** out) {
   if (int r = dalloc(C, &C->dt, 1)) return r;
   if (int r = dalloc(C, &C->flags, 4)) return r;
   if (int r = dalloc(C, &C->counts, 8)) return r;
-  CK(cudaMemset(C->flags, 0, 4 * sizeof(int)));
-  CK(cudaMemset(C->counts, 0, 8 * sizeof(unsigned long long)));
+  // on the context's stream: the first CFL reduction accumulates into them
+  CK(cudaMemsetAsync(C->flags, 0, 4 * sizeof(int), C->stream));
+  CK(cudaMemsetAsync(C->counts, 0, 8 * sizeof(unsigned long long), C->stream));
   for (int d = 0; d < D; ++d) {
     const long long nI = Nc / g.N[d] * (g.N[d] + 1);
     if (int r = dalloc(C, &C->trace[d], (size_t)2 * V * T * NJ * Nc)) return r;
