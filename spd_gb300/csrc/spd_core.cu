@@ -381,9 +381,9 @@ int spd_create(const spd_config* cfg, const spd_operators* ops, spd_ctx** out) {
     CK(cudaMemset(C->gphi_fv, 0, sizeof(double) * D * Nq));
   }
   if (cfg->viscosity) {
-    if (int r = dalloc(C, &C->dWsp, (size_t)D * V * T * NS * Nc)) return r;
+    if (int r = dalloc(C, &C->dWsp, (size_t)D * D * T * NS * Nc)) return r;
     for (int d = 0; d < D; ++d) {
-      if (int r = dalloc(C, &C->Wfp[d], (size_t)V * T * NJ * nf * Nc)) return r;
+      if (int r = dalloc(C, &C->Wfp[d], (size_t)(D + 1) * T * NJ * nf * Nc)) return r;
       if (int r = dalloc(C, &C->Gv[d], (size_t)V * T * NJ * nf * Nc)) return r;
     }
   }

@@ -96,8 +96,9 @@ struct spd_ctx {
   double* Fi[3] = {nullptr, nullptr, nullptr};
   double* Ffp[3] = {nullptr, nullptr, nullptr};
   double* bcfix[3] = {nullptr, nullptr, nullptr};
-  // viscosity scratch: primitives at the flux points (left interface
-  // states), their gradients at the solution points, viscous fluxes
+  // viscosity scratch: density and velocities at the flux points (left
+  // interface states), velocity gradients at the solution points, viscous
+  // fluxes
   double* Wfp[3] = {nullptr, nullptr, nullptr};
   double* dWsp = nullptr;
   double* Gv[3] = {nullptr, nullptr, nullptr};

@@ -3,14 +3,18 @@
 // every Picard iteration and subtracted from the flux at every flux point by
 // the interior kernel.  Bit-identical to the reference's NumPy path:
 //
-//  * ViscGrad: the primitives W at the nf flux points of every direction d
-//    (interpolation of the iterate, then U -> W in the plain velocity
-//    order), with both edge points replaced by the LEFT state of their
+//  * ViscGrad: density and velocities at the nf flux points of every
+//    direction d (interpolation of the iterate, then the quotients of
+//    U -> W), with both edge points replaced by the LEFT state of their
 //    element interface (ML: the right-edge state of the cell on the left,
 //    or the domain-boundary state of src/sd_boundary.py:32-68), stored as
-//    Wfp[d]; their derivative along d at the solution points, divided by h_d,
-//    stored as dWsp[d];
-//  * ViscFlux: for every flux direction d and gradient direction e, dWsp[e]
+//    Wfp[d]; the velocities' derivative along d at the solution points,
+//    divided by h_d, stored as dWsp[d].  The viscous flux reads no other
+//    variable, so neither the energy's line nor the pressure is formed
+//    (128^2, p = 3, 8 launches: 1.15 -> 0.66 ms);
+//  * ViscFlux: for every flux direction d and gradient direction e, the
+//    velocities' dWsp[e] that the flux reads (all for e = d, those along d
+//    and e otherwise: 7 of 15 derivatives in 3D; 1.66 -> 1.07 ms)
 //    interpolated to the flux points of d, with both edge points replaced by
 //    the RIGHT state of their interface (MR: the left-edge value of the cell
 //    on the right, or the boundary state); the viscous flux from Wfp[d] and
@@ -30,7 +34,7 @@
 
 namespace spd {
 
-// threads per block: the flux points of a line, 720 bytes a thread in 3D at
+// threads per block: the flux points of a line, 432 bytes a thread in 3D at
 // degree 4, in 48 KB of shared memory
 constexpr int VISC_THREADS = 64;
 
@@ -43,9 +47,17 @@ struct ViscGrad {
                                              double* W2, double* __restrict__ dWsp, const double* mq0,
                                              const double* mq1, const double* mq2) {
     using k = K<D, P>;
-    // primitives at the flux points of the thread's line (shared memory, so
+    // density and velocities, the variables 0..D
+    constexpr int NV = D + 1;
+    // their values at the flux points of the thread's line (shared memory, so
     // that the loops over variables can stay rolled)
-    __shared__ double scr[k::V * k::nf * VISC_THREADS];
+    __shared__ double scr[NV * k::nf * VISC_THREADS];
+    auto velocities = [](const double* M, double* W) {
+      const Rcp r0 = recip_of(M[0]);
+      W[0] = M[0];
+#pragma unroll
+      for (int v = 1; v < NV; ++v) W[v] = div_by(M[v], M[0], r0);
+    };
     auto Wf = [&](int v, int f) -> double& { return scr[(v * k::nf + f) * VISC_THREADS + threadIdx.x]; };
     // well-balanced mode: the conservative equilibrium at the flux points is
     // part of the state whose primitives are taken (src/sdader_simulator.py:221-223)
@@ -81,7 +93,7 @@ struct ViscGrad {
           return bcfix[d][(((long long)side * k::V + v) * k::NJ + j) * ntrans + ct];
         };
 #pragma unroll 1
-        for (int v = 0; v < k::V; ++v) {
+        for (int v = 0; v < NV; ++v) {
           Line<k::n> ln;
 #pragma unroll
           for (int s = 0; s < k::n; ++s)
@@ -94,65 +106,66 @@ struct ViscGrad {
         }
 #pragma unroll
         for (int f = 1; f < k::nf - 1; ++f) {
-          double M[k::V], W[k::V];
+          double M[NV], W[NV];
 #pragma unroll
-          for (int v = 0; v < k::V; ++v) {
+          for (int v = 0; v < NV; ++v) {
             M[v] = Wf(v, f);
             if (meq[0]) M[v] = M[v] + meq[d][(((long long)v * k::NJ + j) * k::nf + f) * g.Nc + c];
           }
-          prims<D>(M, W, g.gamma, g.iso != 0);
+          velocities(M, W);
 #pragma unroll
-          for (int v = 0; v < k::V; ++v) Wf(v, f) = W[v];
+          for (int v = 0; v < NV; ++v) Wf(v, f) = W[v];
         }
         // right edge: the cell's own right-edge state (its trace), or the
         // stored state on a "pressure" side
         {
-          double M[k::V], W[k::V];
+          double M[NV], W[NV];
           if (cd == Nd - 1 && b1 == BC_PRESSURE) {
 #pragma unroll
-            for (int v = 0; v < k::V; ++v) W[v] = fix(1, v);
+            for (int v = 0; v < NV; ++v) W[v] = fix(1, v);
           } else {
 #pragma unroll
-            for (int v = 0; v < k::V; ++v) M[v] = tr(1, v, c);
-            prims<D>(M, W, g.gamma, g.iso != 0);
+            for (int v = 0; v < NV; ++v) M[v] = tr(1, v, c);
+            velocities(M, W);
           }
 #pragma unroll
-          for (int v = 0; v < k::V; ++v) Wf(v, k::nf - 1) = W[v];
+          for (int v = 0; v < NV; ++v) Wf(v, k::nf - 1) = W[v];
         }
         // left edge: the right-edge state of the cell on the left, or the
         // boundary state
         {
-          double M[k::V], W[k::V];
+          double M[NV], W[NV];
           if (cd > 0 || b0 == BC_PERIODIC || b0 == BC_REFLECTIVE || b0 == BC_GRADFREE) {
             const long long src = (cd > 0) ? c - step : (b0 == BC_PERIODIC ? c + (Nd - 1) * step : c);
             const int side = (cd > 0 || b0 == BC_PERIODIC) ? 1 : 0;
 #pragma unroll
-            for (int v = 0; v < k::V; ++v) M[v] = tr(side, v, src);
-            prims<D>(M, W, g.gamma, g.iso != 0);
+            for (int v = 0; v < NV; ++v) M[v] = tr(side, v, src);
+            velocities(M, W);
             if (cd == 0 && b0 == BC_REFLECTIVE) W[d + 1] = W[d + 1] * -1.0;
           } else {
 #pragma unroll
-            for (int v = 0; v < k::V; ++v) W[v] = fix(0, v);
+            for (int v = 0; v < NV; ++v) W[v] = fix(0, v);
           }
 #pragma unroll
-          for (int v = 0; v < k::V; ++v) Wf(v, 0) = W[v];
+          for (int v = 0; v < NV; ++v) Wf(v, 0) = W[v];
         }
         const bool pow2 = g.h_pow2[d] != 0;
 #pragma unroll 1
-        for (int v = 0; v < k::V; ++v) {
+        for (int v = 0; v < NV; ++v) {
           Line<k::nf> lf;
 #pragma unroll
           for (int f = 0; f < k::nf; ++f) {
             lf.v[f] = Wf(v, f);
             Wfp[d][((((long long)v * g.T + t) * k::NJ + j) * k::nf + f) * g.Nc + c] = lf.v[f];
           }
+          if (v == 0) continue;
           line_ready<k::nf>(lf, op.soft, op.dfp_eoff[d]);
           double dv[k::n];
           line_apply<k::nf, k::n, d == 0>(op.c_dfp, 0, 1, lf, dv);
 #pragma unroll
           for (int so = 0; so < k::n; ++so) {
             const double val = pow2 ? dv[so] : div_by(dv[so], g.h[d], g.rh[d]);
-            dWsp[((((long long)d * k::V + v) * g.T + t) * k::NS + sp_index<D, P>(d, j, so)) * g.Nc + c] = val;
+            dWsp[((((long long)d * D + v - 1) * g.T + t) * k::NS + sp_index<D, P>(d, j, so)) * g.Nc + c] = val;
           }
         }
       }
@@ -179,10 +192,10 @@ struct ViscFlux {
                                              double* G2) {
     using k = K<D, P>;
     constexpr int P_ = D + 1;
-    // gradients at the flux points of the thread's line
-    __shared__ double scr[D * k::V * k::nf * VISC_THREADS];
+    // velocity gradients at the flux points of the thread's line
+    __shared__ double scr[D * D * k::nf * VISC_THREADS];
     auto gf = [&](int e, int v, int f) -> double& {
-      return scr[((e * k::V + v) * k::nf + f) * VISC_THREADS + threadIdx.x];
+      return scr[((e * D + v - 1) * k::nf + f) * VISC_THREADS + threadIdx.x];
     };
     const long long tid = B.id * (long long)blockDim.x + threadIdx.x;
     // one thread per (cell, direction, node, line)
@@ -210,37 +223,38 @@ struct ViscFlux {
           return bcfix[d][(((long long)side * k::V + v) * k::NJ + j) * ntrans + ct];
         };
         auto sp_val = [&](int e, int v, int s, long long cell) -> double {
-          return dWsp[((((long long)e * k::V + v) * g.T + t) * k::NS + sp_index<D, P>(d, j, s)) * g.Nc + cell];
+          return dWsp[((((long long)e * D + v - 1) * g.T + t) * k::NS + sp_index<D, P>(d, j, s)) * g.Nc + cell];
         };
         // gradients along every direction e at the flux points of d
         {
 #pragma unroll 1
-          for (int ev = 0; ev < D * k::V; ++ev) {
-            const int e = ev / k::V, v = ev % k::V;
+          for (int ev = 0; ev < D * D; ++ev) {
+            const int e = ev / D, v = ev % D + 1;
+            if (e != d && v != e + 1 && v != d + 1) continue;
             Line<k::n> ln;
 #pragma unroll
             for (int s = 0; s < k::n; ++s) ln.v[s] = sp_val(e, v, s, c);
             line_ready<k::n>(ln, op.soft);
             double gl[k::nf];
-            line_apply<k::n, k::nf, d == 0>(op.c_sp_to_fp, 0, 1, ln, gl);
+            line_apply<k::n, k::nf - 1, d == 0>(op.c_sp_to_fp, 0, 1, ln, gl);
             // left edge: the cell's own left-edge value (MR of its left
             // interface) unless a "pressure" side overwrote it
             if (cd == 0 && b0 == BC_PRESSURE) gl[0] = fix(0, v);
             // right edge: the left-edge value of the cell on the right, or
-            // the boundary state
-            double r;
-            if (cd < Nd - 1 || b1 == BC_PERIODIC) {
-              const long long nb = (cd < Nd - 1) ? c + step : c - (Nd - 1) * step;
-              Line<k::n> ls;
+            // the boundary state (from the cell's own right-edge value)
+            const bool inner = cd < Nd - 1 || b1 == BC_PERIODIC;
+            const long long nb = !inner ? c : ((cd < Nd - 1) ? c + step : c - (Nd - 1) * step);
 #pragma unroll
-              for (int s = 0; s < k::n; ++s) ls.v[s] = sp_val(e, v, s, nb);
-              line_ready<k::n>(ls, op.soft);
-              line_apply<k::n, 1, d == 0>(op.c_sp_to_fp, 0, 1, ls, &r);
-            } else if (b1 == BC_REFLECTIVE || b1 == BC_GRADFREE) {
-              r = gl[k::nf - 1];
-              if (b1 == BC_REFLECTIVE && v == d + 1) r = r * -1.0;
-            } else {
-              r = fix(1, v);
+            for (int s = 0; s < k::n; ++s) ln.v[s] = sp_val(e, v, s, nb);
+            line_ready<k::n>(ln, op.soft);
+            double r;
+            line_apply<k::n, 1, d == 0>(op.c_sp_to_fp, inner ? 0 : k::nf - 1, 1, ln, &r);
+            if (!inner) {
+              if (b1 == BC_REFLECTIVE) {
+                if (v == d + 1) r = r * -1.0;
+              } else if (b1 != BC_GRADFREE) {
+                r = fix(1, v);
+              }
             }
             gl[k::nf - 1] = r;
 #pragma unroll
