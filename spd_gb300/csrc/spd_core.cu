@@ -240,7 +240,12 @@ int spd_create(const spd_config* cfg, const spd_operators* ops, spd_ctx** out) {
     prepare(C->ops.invader, T * T, C->ops.c_invader);
     prepare(C->ops.w_tp, T, C->ops.c_w_tp);
     C->ops.soft = in ? 1 : 0;
-    // an operator out of their range is also not scaled by 1/h
+    // an operator out of their range is also not scaled by 1/h; nor is the
+    // fused build's, whose entries carry no exponent of their own (a quotient
+    // by a power of two gives the scaled sum's bits)
+#ifdef SPD_FUSED
+    in = false;
+#endif
     for (int d = 0; d < 3; ++d) g.h_pow2[d] = in ? g.h_pow2[d] : 0;
     for (int d = 0; d < 3; ++d) C->ops.dfp_eoff[d] = g.h_pow2[d] ? (unsigned)-std::ilogb(g.h[d]) << 20 : 0u;
   }

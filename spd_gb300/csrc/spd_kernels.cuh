@@ -41,7 +41,7 @@ struct Ops {
   // 1/h_d as a power of two, k << 20, for directions whose h_d is one
   // (Geo::h_pow2), else 0: scaling every product and partial sum of the
   // derivative by 2^k is exact (away from underflow and overflow), so
-  // sum(dfp*F)*(1/h) == sum((dfp/h)*F)
+  // sum(dfp*F)*(1/h) == sum((dfp/h)*F).  0 in the fused build.
   unsigned dfp_eoff[3];
 };
 
