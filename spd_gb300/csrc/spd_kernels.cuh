@@ -771,7 +771,7 @@ struct Full {
         double p[O];
 #ifdef SPD_FUSED
 #pragma unroll
-        for (int o = 0; o < O; ++o) p[o] = K[o].a * x;
+        for (int o = 0; o < O; ++o) p[o] = coef_value(K[o], 0u) * x;
 #else
         uint32_t ok = soft ? 0x40000000u : 0u;
         const Opnd xo = opnd_of(x, ok);

@@ -15,7 +15,8 @@
 // see Line), every other operand is multiplied by the FP64 unit.
 //
 // The build with fused multiply-adds keeps a*b + c as one FP64 instruction;
-// it uses the quotients and roots only.
+// it takes quotients, roots and the first product of each sum from here (that
+// one has nothing to fuse with).
 #pragma once
 #include <cmath>
 #include <cstdint>
@@ -72,12 +73,6 @@ SPD_FN bool gt0_w(double x) {
 // An operator entry (made on the host, coef_of).  For soft_prod: the
 // significand scaled to [2^62, 2^63), and sign and exponent less the bias in
 // the upper 12 bits; the double's own high word gives the value back.
-#ifdef SPD_FUSED
-struct Coef {
-  double a;
-};
-inline Coef coef_of(double a) { return Coef{a}; }
-#else
 struct alignas(16) Coef {
   uint32_t ml, mh, e, hi;
 };
@@ -88,7 +83,6 @@ inline Coef coef_of(double a) {
   const uint32_t hi = (uint32_t)(b >> 32);
   return Coef{(uint32_t)m, (uint32_t)(m >> 32), (hi & 0xfff00000u) - (1023u << 20), hi};
 }
-#endif
 // Magnitudes for which an operator takes part, all of its entries within
 // [2^-256, 2^256] (so none zero): with the other operand's exponent window
 // (Line) no product can then leave the normal range.
@@ -132,14 +126,10 @@ SPD_FN Opnd opnd_of(double x, uint32_t& ok) {
   return Opnd{l << 1, funnel_l1(l, m), zero ? h | (1023u << 20) : h & 0xfff00000u, zero ? 0x80000000u : 0xffffffffu};
 }
 
-#ifdef SPD_FUSED
-SPD_FN double coef_value(const Coef& c, uint32_t) { return c.a; }
-#else
 // the entry, times 2^k with ``eoff`` = k << 20
 SPD_FN double coef_value(const Coef& c, uint32_t eoff) {
   return from_words(c.hi + eoff, (c.ml >> 10) | (c.mh << 22));
 }
-#endif
 // The product of the scaled significands of a coefficient-like operand
 // (mh:ml in [2^62, 2^63)) and an Opnd, in [2^115, 2^117): words 3:2 hold the
 // 53-bit result when bit 116 is set and one bit less otherwise; then the
@@ -211,11 +201,9 @@ SPD_FN double soft_round(Prod o, uint32_t keep) {
 #endif
   return from_words(o.w3 & keep, o.w2);
 }
-#ifndef SPD_FUSED
 SPD_FN double soft_prod(const Coef& c, const Opnd& x) {
   return soft_round(soft_words(c.ml, c.mh, c.e + x.e, x), x.keep);
 }
-#endif
 
 // A divisor b prepared for several quotients: 2^63 over its significand,
 // rounded down to within 4 units (so in [2^62, 2^63)), the quotient's
