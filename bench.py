@@ -196,11 +196,11 @@ def compulsory_bytes_per_cell_step(D, p):
 # `python bench.py --lean --cells 256 --steps 1 --warmup 1 [--build fma]`,
 # divided by the 65,536 cells (both scale with the cell count, and h = 1/256
 # is a power of two as at 512^2, so the derivative takes the same
-# prescaled form; the full 512^2 workload is not captured with more than
+# form; the full 512^2 workload is not captured with more than
 # one pass).  Keyed by (D, p, update, build).
 NCU_K_INTERIOR = {
-    (2, 3, "FV", "ieee"): {"cells_captured": 256 * 256, "dram_bytes": 12085.9 + 14239.4, "fp64_inst": 42043.0},
-    (2, 3, "FV", "fma"): {"cells_captured": 256 * 256, "dram_bytes": 12122.4 + 14251.4, "fp64_inst": 28651.0},
+    (2, 3, "FV", "ieee"): {"cells_captured": 256 * 256, "dram_bytes": 11034.0 + 13929.7, "fp64_inst": 17256.0},
+    (2, 3, "FV", "fma"): {"cells_captured": 256 * 256, "dram_bytes": 11031.3 + 14132.8, "fp64_inst": 18952.0},
 }
 
 

@@ -489,7 +489,7 @@ __global__ void k_adj_faces(Geo g, FvGeo fg, int d, const double* __restrict__ d
     double Fa = 0.0;
     int q[3] = {f[0], f[1], f[2]};
     // quotients by the subcell widths from their correctly rounded
-    // reciprocals (div_rcp: the IEEE quotient's bits in 3 FP64 operations)
+    // reciprocals (div_soft: the IEEE quotient's bits on the integer pipes)
     if (f[d] >= 1) {  // right face of subcell f-1
       q[d] = f[d] - 1;
       const long long qi = q[0] + (long long)g.X[0] * (q[1] + (long long)g.X[1] * q[2]);

@@ -504,7 +504,7 @@ __device__ __forceinline__ double sed_alpha_dir(const double* W, long long e0, l
                                                 const double* c2, const Rcp* rc2, const double* hfp) {
   // line accessors in extended coordinates j along d; c2[j] = cen[j+1] -
   // cen[j-1] and rc2[j] its correctly rounded reciprocal (the quotients
-  // below are the IEEE ones, div_rcp)
+  // below are the IEEE ones, div_soft)
   auto U = [&](int j) { return W[e0 + (long long)j * st]; };
   const int k = i + NGH;
   const int lo = (i == 0) ? k - 1 : k - 2;
