@@ -116,15 +116,15 @@ SPD_FN uint32_t funnel_l1(uint32_t lo, uint32_t hi) {
   return (hi << 1) | (lo >> 31);
 #endif
 }
-// ``ok`` keeps bit 30 when x is a zero or its biased exponent lies in
-// [512, 1535] (the two upper exponent bits differ: |x| in [2^-511, 2^513)).
-SPD_FN Opnd opnd_of(double x, uint32_t& ok) {
+// ``ok`` keeps bit 30 when x is a zero (``zero``) or its biased exponent lies
+// in [512, 1535] (the two upper exponent bits differ: |x| in [2^-511, 2^513)).
+SPD_FN Opnd opnd_words(double x, bool zero, uint32_t& ok) {
   const uint32_t h = hi_word(x), l = lo_word(x), h2 = h << 1;
-  const bool zero = (h2 | l) == 0u;
   const uint32_t m = zero ? 0u : (h & 0xfffffu) | 0x100000u;
   ok &= zero ? 0x40000000u : h ^ h2;
   return Opnd{l << 1, funnel_l1(l, m), zero ? h | (1023u << 20) : h & 0xfff00000u, zero ? 0x80000000u : 0xffffffffu};
 }
+SPD_FN Opnd opnd_of(double x, uint32_t& ok) { return opnd_words(x, ((hi_word(x) << 1) | lo_word(x)) == 0u, ok); }
 
 // the entry, times 2^k with ``eoff`` = k << 20
 SPD_FN double coef_value(const Coef& c, uint32_t eoff) {
@@ -351,9 +351,11 @@ SPD_FN double sqrt_soft(double x) {
 // on the integer pipes (sums stay on the FP64 pipe).  ``ok`` (bit 30): the
 // value and every value it came from are zeros or within opnd_of's window.
 // A product of two such values is at least 2^-1022; one above the largest
-// double carries into the sign bit and leaves an exponent field below 8, so
-// it fails the window itself.  A result without ``ok`` is computed again in
-// plain FP64 arithmetic.  Unused preparations are dead code.
+// double leaves the exponent field 2047, or 0 with a carry into the sign bit,
+// and fails the window itself.  Its words can be those of a zero (a product
+// that rounds to 2^1025), so whether a product is a zero is taken from its
+// factors.  A result without ``ok`` is computed again in plain FP64
+// arithmetic.  Unused preparations are dead code.
 struct Num {
   double v;
   Opnd o;
@@ -369,8 +371,12 @@ SPD_FN Num operator-(const Num& a, const Num& b) { return Num(a.v - b.v, a.ok & 
 SPD_FN Num operator-(const Num& a) { return Num(from_words(hi_word(a.v) ^ 0x80000000u, lo_word(a.v)), a.ok); }
 SPD_FN Num operator*(const Num& a, const Num& b) {
   const uint32_t ch = (a.o.mh << 9) | (a.o.ml >> 23);
-  return Num(soft_round(soft_words(a.o.ml << 9, ch, a.o.e + b.o.e - (1023u << 20), b.o), a.o.keep & b.o.keep),
-             a.ok & b.ok);
+  const uint32_t keep = a.o.keep & b.o.keep;
+  Num r;
+  r.v = soft_round(soft_words(a.o.ml << 9, ch, a.o.e + b.o.e - (1023u << 20), b.o), keep);
+  r.ok = a.ok & b.ok;
+  r.o = opnd_words(r.v, keep != 0xffffffffu, r.ok);
+  return r;
 }
 SPD_FN Num operator+(const Num& a, double b) { return a + Num(b); }
 SPD_FN Num operator-(const Num& a, double b) { return a - Num(b); }
