@@ -161,7 +161,13 @@ SPD_FN double div_rcp(double a, double b, double rb) {
 // c ? a : b by value
 template <class S>
 SPD_FN S sel(bool c, const S& a, const S& b) { return c ? a : b; }
-SPD_FN Num sel(bool c, const Num& a, const Num& b) { return Num(c ? a.v : b.v, c ? a.ok : b.ok); }
+// A Num out of range may have any value, so a choice made by comparing two of
+// them stands only if both are in range; a bound (always exact) counts only
+// where it is taken.
+SPD_FN Num sel(bool c, const Num& a, const Num& b) { return Num(c ? a.v : b.v, a.ok & b.ok); }
+template <class S>
+SPD_FN S bounded(bool c, const S& a, double bound) { return c ? a : S(bound); }
+SPD_FN Num bounded(bool c, const Num& a, double bound) { return Num(c ? a.v : bound, a.ok); }
 SPD_FN double half(double x) { return 0.5 * x; }
 template <int N> SPD_FN Dual<N> half(const Dual<N>& x) { return 0.5 * x; }
 SPD_FN double sval(double x) { return x; }
@@ -405,7 +411,7 @@ SPD_FN S sound_speed(const S& P, const S& rho, double gamma, double min_c2,
                                          Br<BM>* br = nullptr,
                                          const typename RecipOf<S>::T* rrho = nullptr) {
   S c2 = div_by(gamma * P, rho, rrho ? *rrho : recip_of(rho));
-  c2 = sel(pick(br, fgt(c2, min_c2)), c2, S(min_c2));
+  c2 = bounded(pick(br, fgt(c2, min_c2)), c2, min_c2);
   return ad_sqrt(c2);
 }
 
@@ -434,6 +440,9 @@ template <int D, class S, int BM = 0>
 SPD_FN void hllc(const S* WL, const S* WR, const S* UL, const S* UR, S* F, double gamma,
                                      double min_c2, int idim, bool low_mach, Br<BM>* br = nullptr,
                                      const typename RecipOf<S>::T* rL = nullptr, const typename RecipOf<S>::T* rR = nullptr, bool iso = false) {
+  // vstar and sR decide between states that do not hang on them, and their
+  // range flags would be lost there
+  static_assert(!std::is_same<S, Num>::value, "HLLC's choices carry no range flag");
   constexpr int P_ = D + 1;
   const int v1 = rvel<D>(idim, 0);
   const S cL = sound_speed(WL[P_], WL[0], gamma, min_c2, br, rL) + abs_br(WL[v1], br);
