@@ -263,9 +263,9 @@ struct ViscFlux {
         }
 #pragma unroll
         for (int f = 0; f < k::nf; ++f) {
-          double W[k::V];
+          double W[D + 1];  // density and velocities, all that Wfp holds
 #pragma unroll
-          for (int v = 0; v < k::V; ++v)
+          for (int v = 0; v <= D; ++v)
             W[v] = Wfp[d][((((long long)v * g.T + t) * k::NJ + j) * k::nf + f) * g.Nc + c];
           double F[k::V];
           F[v1] = 2.0 * gf(d, v1, f) - beta * gf(d, v1, f);
