@@ -472,8 +472,10 @@ template <int TT>
 static __device__ __forceinline__ void picard(const Ops& op, const Geo& g, double* slot, int CPB, int Teff, double dt,
                                               double usp, double* __restrict__ out, long long stride) {
   double acc[TT];
+  // Teff == 1: one derivative for all nodes
+#ifndef SPD_FUSED
   if (Teff == 1) {
-    // one derivative for all nodes: one operand, TT x TT products
+    // one operand, TT x TT products
     Line<1> one;
     one.v[0] = slot[0];
     line_ready<1>(one, op.soft);
@@ -481,10 +483,14 @@ static __device__ __forceinline__ void picard(const Ops& op, const Geo& g, doubl
     line_apply<1, TT * TT, false>(op.c_invader, 0, 1, one, p);
 #pragma unroll
     for (int t = 0; t < TT; ++t) acc[t] = sum_terms<TT, false>(p + t * TT);
-  } else {
+  } else
+#endif
+  {
+    // (also the fused build's form for one value: its terms after the first
+    // are one rounding each, not a product and a sum)
     Line<TT> ln;
 #pragma unroll
-    for (int p = 0; p < TT; ++p) ln.v[p] = slot[p * CPB];
+    for (int p = 0; p < TT; ++p) ln.v[p] = slot[Teff == 1 ? 0 : p * CPB];
     line_ready<TT>(ln, op.soft);
     line_apply<TT, TT, false>(op.c_invader, 0, 1, ln, acc);
   }
