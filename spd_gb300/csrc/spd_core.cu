@@ -294,30 +294,28 @@ int spd_create(const spd_config* cfg, const spd_operators* ops, spd_ctx** out) {
   {
     std::vector<double> buf;
     std::vector<Rcp> rcp;
-    size_t off[3][6], roff[3][3];
+    size_t off[3][5], roff[3][3];
     for (int d = 0; d < D; ++d) {
       const int Xd = g.X[d], Xe = g.Xe[d];
       const double* fp = ops->faces[d];
       off[d][0] = buf.size();
       for (int k2 = 0; k2 < Xd; ++k2) buf.push_back(fp[NGH + 1 + k2] - fp[NGH + k2]);
-      off[d][1] = buf.size();
       std::vector<double> cen(Xe);
       for (int e = 0; e < Xe; ++e) cen[e] = 0.5 * (fp[e + 1] + fp[e]);
-      buf.insert(buf.end(), cen.begin(), cen.end());
-      off[d][2] = buf.size();
+      off[d][1] = buf.size();
       for (int e = 0; e < Xe; ++e) buf.push_back(fp[e + 1] - fp[e]);
-      off[d][3] = buf.size();
+      off[d][2] = buf.size();
       for (int e = 0; e + 1 < Xe; ++e) buf.push_back(cen[e + 1] - cen[e]);
-      off[d][4] = buf.size();
+      off[d][3] = buf.size();
       for (int e = 0; e < Xe; ++e) buf.push_back((e >= 1 && e + 1 < Xe) ? cen[e + 1] - cen[e - 1] : 1.0);
-      off[d][5] = buf.size();
-      for (int e = 0; e + 1 < Xe; ++e) buf.push_back(1.0 / buf[off[d][3] + e]);
+      off[d][4] = buf.size();
+      for (int e = 0; e + 1 < Xe; ++e) buf.push_back(1.0 / buf[off[d][2] + e]);
       roff[d][0] = rcp.size();
       for (int k2 = 0; k2 < Xd; ++k2) rcp.push_back(recip_of(buf[off[d][0] + k2]));
       roff[d][1] = rcp.size();
-      for (int e = 0; e + 1 < Xe; ++e) rcp.push_back(recip_of(buf[off[d][3] + e]));
+      for (int e = 0; e + 1 < Xe; ++e) rcp.push_back(recip_of(buf[off[d][2] + e]));
       roff[d][2] = rcp.size();
-      for (int e = 0; e < Xe; ++e) rcp.push_back(recip_of(buf[off[d][4] + e]));
+      for (int e = 0; e < Xe; ++e) rcp.push_back(recip_of(buf[off[d][3] + e]));
     }
     if (int r = dalloc(C, &C->geo_arrays, buf.size())) return r;
     CK(cudaMemcpy(C->geo_arrays, buf.data(), buf.size() * sizeof(double), cudaMemcpyHostToDevice));
@@ -325,11 +323,10 @@ int spd_create(const spd_config* cfg, const spd_operators* ops, spd_ctx** out) {
     CK(cudaMemcpy(C->geo_rcp, rcp.data(), rcp.size() * sizeof(Rcp), cudaMemcpyHostToDevice));
     for (int d = 0; d < D; ++d) {
       C->fvg.dx[d] = C->geo_arrays + off[d][0];
-      C->fvg.centers[d] = C->geo_arrays + off[d][1];
-      C->fvg.hfp[d] = C->geo_arrays + off[d][2];
-      C->fvg.hcv[d] = C->geo_arrays + off[d][3];
-      C->fvg.c2[d] = C->geo_arrays + off[d][4];
-      C->fvg.ihcv[d] = C->geo_arrays + off[d][5];
+      C->fvg.hfp[d] = C->geo_arrays + off[d][1];
+      C->fvg.hcv[d] = C->geo_arrays + off[d][2];
+      C->fvg.c2[d] = C->geo_arrays + off[d][3];
+      C->fvg.ihcv[d] = C->geo_arrays + off[d][4];
       C->fvg.rdx[d] = C->geo_rcp + roff[d][0];
       C->fvg.rhcv[d] = C->geo_rcp + roff[d][1];
       C->fvg.rc2[d] = C->geo_rcp + roff[d][2];

@@ -197,16 +197,6 @@ void launch(spd_ctx* C, const char* name, void (*kern)(P...), dim3 grid, dim3 bl
   spd_batch::launch_step(C->stream, kern, grid, block, smem, std::forward<A>(a)...);
 }
 
-// zero-fill of device bytes on the context's stream (recorded while a batch
-// recorder is attached)
-inline cudaError_t zero_fill(spd_ctx* C, void* p, size_t bytes) {
-  if (C->brec) {
-    C->brec->add_zero(p, bytes);
-    return cudaSuccess;
-  }
-  return cudaMemsetAsync(p, 0, bytes, C->stream);
-}
-
 inline cudaEvent_t get_event(spd_ctx* C) {
   if (!C->pool.empty()) {
     cudaEvent_t e = C->pool.back();

@@ -739,10 +739,9 @@ SPD_FN void euler_flux(const double* U, double gamma, int d, bool iso, const Rcp
   for (int q = 0; q < D; ++q) store(rvel<D>(d, q), sval(f[1 + q]));
 }
 
-// One output of a 1D operator contraction: sum_s A[s] * x[s].  ``lanes2``
-// is the order of an einsum over the contiguous x axis (even and odd terms
-// accumulated separately, then added); otherwise a left-to-right sum
-// (src/transforms.py:3-25).
+// One output of a 1D operator contraction: sum_s A[s] * x[s], left to right,
+// or (dot_lanes2) in the order of an einsum over the contiguous x axis, even
+// and odd terms accumulated separately and then added (src/transforms.py:3-25).
 template <int L>
 SPD_FN double dot_seq(const double* A, const double* x) {
   double acc = A[0] * x[0];
@@ -761,10 +760,6 @@ SPD_FN double dot_lanes2(const double* A, const double* x) {
     else o = o + A[s] * x[s];
   }
   return e + o;
-}
-template <int L>
-SPD_FN double dot_dir(const double* A, const double* x, int idim) {
-  return idim == 0 ? dot_lanes2<L>(A, x) : dot_seq<L>(A, x);
 }
 
 // Limiters (src/muscl.py:12-59); NaN semantics follow the np.where forms.

@@ -10,7 +10,6 @@ namespace spd {
 
 struct FvGeo {
   const double* dx[3];       // active subcell widths, X_d values
-  const double* centers[3];  // extended subcell centres, Xe_d values
   const double* hfp[3];      // extended subcell widths, Xe_d values
   const double* hcv[3];      // extended centre distances, Xe_d - 1 values
   const Rcp* rdx[3];      // reciprocals of dx
