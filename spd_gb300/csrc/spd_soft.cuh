@@ -116,15 +116,22 @@ SPD_FN uint32_t funnel_l1(uint32_t lo, uint32_t hi) {
   return (hi << 1) | (lo >> 31);
 #endif
 }
-// ``ok`` keeps bit 30 when x is a zero (``zero``) or its biased exponent lies
-// in [512, 1535] (the two upper exponent bits differ: |x| in [2^-511, 2^513)).
-SPD_FN Opnd opnd_words(double x, bool zero, uint32_t& ok) {
+// ``ok`` keeps bit 30 when x is a zero or its biased exponent lies in
+// [512, 1535] (the two upper exponent bits differ: |x| in [2^-511, 2^513)).
+SPD_FN Opnd opnd_of(double x, uint32_t& ok) {
   const uint32_t h = hi_word(x), l = lo_word(x), h2 = h << 1;
+  const bool zero = (h2 | l) == 0u;
   const uint32_t m = zero ? 0u : (h & 0xfffffu) | 0x100000u;
   ok &= zero ? 0x40000000u : h ^ h2;
   return Opnd{l << 1, funnel_l1(l, m), zero ? h | (1023u << 20) : h & 0xfff00000u, zero ? 0x80000000u : 0xffffffffu};
 }
-SPD_FN Opnd opnd_of(double x, uint32_t& ok) { return opnd_words(x, ((hi_word(x) << 1) | lo_word(x)) == 0u, ok); }
+// The same of a product, whose mask ``keep`` says whether a factor is a zero:
+// the fields by the mask's bits instead of a choice each.
+SPD_FN Opnd opnd_of_product(double x, uint32_t keep, uint32_t& ok) {
+  const uint32_t h = hi_word(x), l = lo_word(x);
+  ok &= (h ^ (h << 1)) | ~keep;
+  return Opnd{l << 1, funnel_l1(l, ((h & 0xfffffu) | 0x100000u) & keep), (h & 0xfff00000u) | (~keep & (1023u << 20)), keep};
+}
 
 // the entry, times 2^k with ``eoff`` = k << 20
 SPD_FN double coef_value(const Coef& c, uint32_t eoff) {
@@ -375,7 +382,7 @@ SPD_FN Num operator*(const Num& a, const Num& b) {
   Num r;
   r.v = soft_round(soft_words(a.o.ml << 9, ch, a.o.e + b.o.e - (1023u << 20), b.o), keep);
   r.ok = a.ok & b.ok;
-  r.o = opnd_words(r.v, keep != 0xffffffffu, r.ok);
+  r.o = opnd_of_product(r.v, keep, r.ok);
   return r;
 }
 SPD_FN Num operator+(const Num& a, double b) { return a + Num(b); }
