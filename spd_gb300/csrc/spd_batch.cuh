@@ -175,7 +175,8 @@ struct Site : SiteBase {
   }
   cudaError_t launch(cudaStream_t s) override {
     if (boff.back() == 0) return cudaSuccess;
-    return launch_step(s, k_batched<Body, A...>, dim3(boff.back()), block, smem, d_packs, d_boff, count());
+    launch_step(s, k_batched<Body, A...>, dim3(boff.back()), block, smem, d_packs, d_boff, count());
+    return cudaGetLastError();  // the launch's error, not left for the next check
   }
 };
 
@@ -194,7 +195,8 @@ struct ZeroSite : SiteBase {
   }
   cudaError_t launch(cudaStream_t s) override {
     if (boff.back() == 0) return cudaSuccess;
-    return launch_step(s, k_zero_ranges, dim3(boff.back()), block, 0, d_ranges, d_boff, count());
+    launch_step(s, k_zero_ranges, dim3(boff.back()), block, 0, d_ranges, d_boff, count());
+    return cudaGetLastError();
   }
 };
 #endif
