@@ -133,6 +133,19 @@ cudaError_t launch_step(cudaStream_t s, void (*kern)(P...), dim3 grid, dim3 bloc
 
 constexpr unsigned MAX_GRID = 0x7fffffffu;
 
+#ifdef __CUDACC__
+// Lets a kernel have all the shared memory of a block.  The limit belongs to
+// the kernel, which several launches of a step and several ensembles share, so
+// it is never one launch's own need.
+inline cudaError_t allow_dynamic_smem(const void* kern) {
+  cudaFuncAttributes a{};
+  const cudaError_t e = cudaFuncGetAttributes(&a, kern);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              227 * 1024 - (int)a.sharedSizeBytes);
+}
+#endif
+
 struct SiteBase {
   const char* name = "";
   dim3 block{1, 1, 1};
@@ -169,8 +182,7 @@ struct Site : SiteBase {
     if (e != cudaSuccess) return e;
     e = cudaMemcpy(d_packs, packs.data(), sizeof(Pack<A...>) * packs.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return e;
-    if (smem > 48 * 1024)
-      e = cudaFuncSetAttribute(k_batched<Body, A...>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) e = allow_dynamic_smem(reinterpret_cast<const void*>(k_batched<Body, A...>));
     return e;
   }
   cudaError_t launch(cudaStream_t s) override {
