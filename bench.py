@@ -799,7 +799,7 @@ def ensemble_arm(args):
     if sims:
         if args.ensemble_form == "auto":
             ens = SDADER_Ensemble(sims)
-            tuning = ens.autotune(streams=(1, 4, 16), cpbs=(32, 64), probe_launches=1)
+            tuning = ens.autotune(streams=(1, 4, 16), cpbs=(16, 32), probe_launches=1)
         else:
             ens = SDADER_Ensemble(sims, nstreams=16, packed=args.ensemble_form == "packed")
             tuning = {"form": args.ensemble_form, "streams": None if args.ensemble_form == "packed" else 16,
