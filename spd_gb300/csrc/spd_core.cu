@@ -241,8 +241,8 @@ int spd_create(const spd_config* cfg, const spd_operators* ops, spd_ctx** out) {
     prepare(C->ops.w_tp, T, C->ops.c_w_tp);
     C->ops.soft = in ? 1 : 0;
     // an operator out of their range is also not scaled by 1/h; nor is the
-    // fused build's, whose entries carry no exponent of their own (a quotient
-    // by a power of two gives the scaled sum's bits)
+    // fused build's, which divides by every h alike (a quotient by a power of
+    // two gives the scaled sum's bits, for one integer quotient per value)
 #ifdef SPD_FUSED
     in = false;
 #endif

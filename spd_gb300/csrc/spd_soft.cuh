@@ -1,14 +1,14 @@
 // Correctly rounded FP64 products on the integer pipes.
 //
-// Why: GB300 issues 1.6 FP64 lane-operations per clock and SM (a dependent
-// DADD, DMUL or DFMA chain: 80 issue cycles of an SM sub-partition per warp
-// instruction, measured), against 64 integer lanes.  The step's contractions
-// are a rounded product and a rounded sum per term, so half of the FP64
-// instructions that bound them are products with a constant operator entry.
-// The product of two 53-bit significands is four 32x32 -> 64-bit multiplies
-// and a carry chain; rounded to nearest-even in integer registers it takes 46
-// issue cycles and runs beside the FP64 additions (product + DADD: 80
-// cycles, DMUL + DADD: 160, measured).
+// Why: GB300 issues about 1.7 FP64 lane-operations per clock and SM (DADD and
+// DMUL chains: 76 issue cycles of an SM sub-partition per warp instruction),
+// against 64 integer lanes.  The step's contractions are a rounded product and
+// a rounded sum per term, so half of the FP64 instructions that bound them are
+// products with a constant operator entry.  The product of two 53-bit
+// significands is four 32x32 -> 64-bit multiplies and a carry chain; rounded
+// to nearest-even in integer registers, its operand's preparation included, it
+// takes 49 issue cycles and runs beside the FP64 additions (product + DADD: 76
+// cycles, DMUL + DADD: 152).  Measured by profiles/integer_pipe_rates.cu.
 //
 // The result is the IEEE 754 product bit for bit: the operands are finite,
 // nonzero and far from underflow and overflow (tested per line of values,
@@ -224,8 +224,8 @@ struct alignas(16) Recip {
 // Muller et al., Handbook of Floating-Point Arithmetic, 2nd ed., 4.7):
 // relative error 2^-22, then 2^-43.9, then the rounding of the last step.
 // Each step rounds down, and one unit is taken off at the end, so the result
-// is below the exact value.  About 35 integer instructions, where the FP64
-// reciprocal is seven instructions of 80 cycles.
+// is below the exact value.  62 issue cycles, 344 for the FP64 1 / x (a whole
+// quotient 135 against 572; profiles/integer_pipe_rates.cu).
 SPD_FN Recip recip_soft(double b) {
   const uint32_t h = hi_word(b), l = lo_word(b);
   const uint32_t bh = (((h & 0xfffffu) | 0x100000u) << 11) | (l >> 21), bl = l << 11;  // [2^63, 2^64)
@@ -302,7 +302,8 @@ SPD_FN double div_soft(double a, double b, const Recip& rb) {
 // to 2^-43, then s += (m - s^2) y / 2 to the last place of scale 2^60, taken
 // down by 4 units so that its 53-bit floor q is at most one below the
 // root's; the exact m - q^2 against q decides the last place (a root of a
-// 53-bit number is never a tie).  About 50 integer instructions.
+// 53-bit number is never a tie).  125 issue cycles, 574 for the FP64 root
+// (profiles/integer_pipe_rates.cu).
 SPD_FN double sqrt_soft(double x) {
   const uint32_t h = hi_word(x), l = lo_word(x);
   if (((h ^ (h << 1)) & 0x40000000u) == 0u || (h >> 31) != 0u) return sqrt(x);
